@@ -32,7 +32,7 @@ from pageflow_b200 import datagen, paged, serve, tqpkernels
 from pageflow_b200.aggregation_slab import DenseAggregationSlab
 from pageflow_b200.batch import BatchJoinAggregate, Instance
 from pageflow_b200.gather import index_select_many
-from pageflow_b200.join_aggregate import JoinAggregate, join_group_aggregate
+from pageflow_b200.join_aggregate import JoinAggregate
 from pageflow_b200.keyed_aggregate import KeyedPass1
 from pageflow_b200.sorted_run_merge import merge_sorted_unique_runs_inplace
 
@@ -412,9 +412,8 @@ def _paged_run(state):
     stats = parts.read_stats()
     n = stats["rows"]
     # a bucket's rows come in no fixed order: the join's groups are the result
-    keys, sums, counts = join_group_aggregate(
-        key, group, parts.columns["fk"][:n], parts.columns["price"][:n], group_min=0,
-        n_groups=c["groups"], B=64)
+    plan = JoinAggregate(c["n_build"], n, 0, c["groups"], DEVICE, autotune=False)
+    keys, sums, counts = plan.run(key, group, parts.columns["fk"][:n], parts.columns["price"][:n])
     return keys, sums, counts, parts.bucket_offsets, n
 
 
