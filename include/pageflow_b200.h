@@ -396,6 +396,81 @@ int pf_group_hash(const void* const* key_cols, const int* row_bytes, const int64
 int pf_hash_buckets(const int64_t* hash, int64_t n, int B, int32_t* bucket_out,
                     int64_t* counts_out, void* stream);
 
+/*
+ * The hash route in one read of the rows, for chunks whose groups fit a table
+ * in memory (by default about 64 MiB / (8 * (1 + naccs))): the grouping hash as
+ * pf_group_hash's, a place per distinct hash that holds every accumulator of
+ * the group, the groups ascending by hash, their buckets as
+ * pf_hash_buckets's.  pf_keyed_pass1_read queues the reading, into the
+ * workspace; pf_keyed_pass1_emit, with the same rows, accumulators and
+ * workspace, writes the results and waits once.  expect: 0, or how many
+ * groups the table is made for (at most 2^28; the same in every call).
+ * *n_groups gets the groups, or minus an estimate of them when they do not
+ * fit: read again with expect, or take pf_group_hash and pf_unique_reduce.
+ * Accumulators (naccs <= 15), each folding one column of its kind:
+ *   PF_KA_WORD   the largest (as int64) 8-byte word `word` of the column's
+ *                row_bytes-byte rows, zero-padded (a key's representative)
+ *   PF_KA_COUNT  the rows (no column)
+ *   PF_KA_NULLS  the rows whose value is the null -64
+ *   PF_KA_SUM_I  the int64 sum of an integer column (wraps)
+ *   PF_KA_SUM_F  the float64 sum of a float column, in no fixed order
+ *   PF_KA_MIN, PF_KA_MAX  of an integer column
+ * Outputs (nouts <= 40), with room for pf_keyed_pass1_groups(n, naccs, expect)
+ * rows
+ * as hash_out and bucket_out, from accumulators acc, acc2 and acc3:
+ *   PF_KO_WORD      bytes [8 * word, 8 * word + 8) of row_bytes-byte rows
+ *   PF_KO_I64, PF_KO_I32, PF_KO_F64, PF_KO_F32  the accumulator as that type
+ *   PF_KO_I64_MAX0, PF_KO_I32_MAX0  the larger of it and 0
+ *   PF_KO_COUNT     acc - acc2 as int64
+ *   PF_KO_AVG_I, PF_KO_AVG_F  the float64 pair (acc, an integer or a float
+ *                   sum; acc2 - acc3)
+ * B > 1: bucket_out, counts_out (device int64[B]) and host_counts (host
+ * int64[B]).  Hashes crowded into a small part of their range are ordered by
+ * a radix sort: *crowded (0 in the first call) gets the bytes it needs, with
+ * nothing output; call pf_keyed_pass1_emit again with *crowded as it is and a
+ * sort_workspace of that size.
+ */
+#define PF_KA_WORD 0
+#define PF_KA_COUNT 1
+#define PF_KA_NULLS 2
+#define PF_KA_SUM_I 3
+#define PF_KA_SUM_F 4
+#define PF_KA_MIN 5
+#define PF_KA_MAX 6
+#define PF_KK_I64 0
+#define PF_KK_I32 1
+#define PF_KK_F64 2
+#define PF_KK_F32 3
+#define PF_KO_WORD 0
+#define PF_KO_I64 1
+#define PF_KO_I32 2
+#define PF_KO_F64 3
+#define PF_KO_F32 4
+#define PF_KO_I64_MAX0 5
+#define PF_KO_I32_MAX0 6
+#define PF_KO_COUNT 7
+#define PF_KO_AVG_I 8
+#define PF_KO_AVG_F 9
+typedef struct pf_keyed_acc {
+  int op, kind, row_bytes, word;
+  const void* src;
+} pf_keyed_acc;
+typedef struct pf_keyed_out {
+  int op, acc, acc2, acc3, row_bytes, word;
+  void* dst;
+} pf_keyed_out;
+size_t pf_keyed_pass1_workspace(int64_t n, int naccs, int64_t expect);
+int64_t pf_keyed_pass1_groups(int64_t n, int naccs, int64_t expect);
+int pf_keyed_pass1_read(const void* const* key_cols, const int* row_bytes,
+                        const int64_t* const* coeffs, int ncols, int64_t n,
+                        const pf_keyed_acc* accs, int naccs, int64_t expect, void* workspace,
+                        size_t workspace_bytes, void* stream);
+int pf_keyed_pass1_emit(int64_t n, const pf_keyed_acc* accs, int naccs, int64_t expect,
+                        const pf_keyed_out* outs, int nouts, int64_t* hash_out, int B, int32_t* bucket_out,
+                        int64_t* counts_out, int64_t* host_counts, int64_t* n_groups,
+                        int64_t* crowded, void* workspace, size_t workspace_bytes,
+                        void* sort_workspace, size_t sort_workspace_bytes, void* stream);
+
 /* ---- sorted runs of the two-pass aggregation -------------------------------- */
 /*
  * Stable ascending sort of n int64 keys carrying int64 values (vals_in NULL:
@@ -436,6 +511,24 @@ int pf_merge_sorted_runs(const int64_t* run_keys, const void* const* run_vals, i
                          int ncols, const int* kinds, const int* esizes, const int* widths,
                          const int* ops, int64_t* out_keys, void* const* out_vals, int64_t* n_out,
                          void* workspace, size_t workspace_bytes, void* stream);
+/*
+ * The merge in place where it moves nothing: *n_new (host) gets the tick keys
+ * that the run does not hold, and when there is none every tick row is
+ * combined into its run row, op(run value, tick value), and the run is the
+ * merged one.  Else nothing is written (take pf_merge_sorted_runs).  The
+ * workspace is pf_merge_sorted_runs_workspace's; waits once.
+ */
+int pf_fold_sorted_run(const int64_t* run_keys, void* const* run_vals, int64_t n_run,
+                       const int64_t* tick_keys, const void* const* tick_vals, int64_t n_tick,
+                       int ncols, const int* kinds, const int* esizes, const int* widths,
+                       const int* ops, int64_t* n_new, void* workspace, size_t workspace_bytes,
+                       void* stream);
+/*
+ * The first n rows of up to 17 columns copied in one launch (dst[q] from
+ * src[q], row_bytes[q] bytes a row; the two must not overlap).  Queued only.
+ */
+int pf_copy_rows(const void* const* src, void* const* dst, const int* row_bytes, int ncols,
+                 int64_t n, void* stream);
 
 /* ---- compressed pages: decode on arrival, filter, partition ---------------- */
 /*

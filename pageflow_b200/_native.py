@@ -91,6 +91,12 @@ _SIGS = {
                                   _vp]),
     "pf_group_hash": (_int, [_vp, _vp, _vp, _int, _i64, _vp, _vp]),
     "pf_hash_buckets": (_int, [_vp, _i64, _int, _vp, _vp, _vp]),
+    "pf_keyed_pass1_workspace": (_sz, [_i64, _int, _i64]),
+    "pf_keyed_pass1_groups": (_i64, [_i64, _int, _i64]),
+    "pf_keyed_pass1_read": (_int, [_vp, _vp, _vp, _int, _i64, _vp, _int, _i64, _vp, _sz, _vp]),
+    "pf_keyed_pass1_emit": (_int, [_i64, _vp, _int, _i64, _vp, _int, _vp, _int, _vp, _vp, _vp,
+                                   ctypes.POINTER(_i64), ctypes.POINTER(_i64), _vp, _sz, _vp,
+                                   _sz, _vp]),
     "pf_sort_pairs_workspace": (_sz, [_i64]),
     "pf_sort_pairs": (_int, [_vp, _vp, _i64, _vp, _vp, _vp, _sz, _vp]),
     "pf_unique_reduce_workspace": (_sz, [_i64]),
@@ -99,6 +105,9 @@ _SIGS = {
     "pf_merge_sorted_runs_workspace": (_sz, [_i64]),
     "pf_merge_sorted_runs": (_int, [_vp, _vp, _i64, _vp, _vp, _i64, _int, _vp, _vp, _vp, _vp,
                                     _vp, _vp, ctypes.POINTER(_i64), _vp, _sz, _vp]),
+    "pf_fold_sorted_run": (_int, [_vp, _vp, _i64, _vp, _vp, _i64, _int, _vp, _vp, _vp, _vp,
+                                  ctypes.POINTER(_i64), _vp, _sz, _vp]),
+    "pf_copy_rows": (_int, [_vp, _vp, _vp, _int, _i64, _vp]),
     "pf_encode_pages_workspace": (_sz, [_int]),
     "pf_encode_pages": (_int, [_vp, _int, _vp, _int, _vp, _i64, _vp, _vp, _sz, _vp]),
     "pf_page_encode": (_i64, [_vp, _int, _i64, _vp, _i64]),
@@ -121,6 +130,17 @@ _SIGS = {
     "pf_batch_run": (_int, [_vp, _vp, _vp]),
     "pf_batch_slab": (_vp, [_vp, _int]),
 }
+
+
+class KeyedAcc(ctypes.Structure):
+    """pf_keyed_acc (include/pageflow_b200.h)."""
+    _fields_ = [("op", _int), ("kind", _int), ("row_bytes", _int), ("word", _int), ("src", _vp)]
+
+
+class KeyedOut(ctypes.Structure):
+    """pf_keyed_out (include/pageflow_b200.h)."""
+    _fields_ = [("op", _int), ("acc", _int), ("acc2", _int), ("acc3", _int),
+                ("row_bytes", _int), ("word", _int), ("dst", _vp)]
 
 
 class BatchInstance(ctypes.Structure):

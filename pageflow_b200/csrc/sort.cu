@@ -11,6 +11,9 @@
 //   pf_merge_sorted_runs merge_sorted_unique_runs_inplace (:94-174): the union
 //                        of two ascending unique runs, matched keys combined,
 //                        out of place (the caller copies it back)
+//   pf_fold_sorted_run   the same where the run holds every tick key already:
+//                        the values combined in place, nothing moved
+//   pf_copy_rows         the rows of several columns in one launch
 //
 // A radix pass: k_rs_hist counts each 4096-key tile's digits; an exclusive
 // scan over [digit][tile] gives every (digit, tile) run's output start;
@@ -48,7 +51,19 @@ __global__ void __launch_bounds__(RT) k_minmax(const long long* __restrict__ k, 
     lo = min(lo, __shfl_xor_sync(FULL, lo, o));
     hi = max(hi, __shfl_xor_sync(FULL, hi, o));
   }
+  // one atomic pair a block: a pair a warp queued up on two addresses (4M keys:
+  // 31 us, with their reads 6)
+  __shared__ long long red[2][RT / 32];
   if ((threadIdx.x & 31) == 0) {
+    red[0][threadIdx.x >> 5] = lo;
+    red[1][threadIdx.x >> 5] = hi;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < RT / 32; ++w) {
+      lo = min(lo, red[0][w]);
+      hi = max(hi, red[1][w]);
+    }
     atomicMin(&mm[0], lo);
     atomicMax(&mm[1], hi);
   }
@@ -493,16 +508,58 @@ __device__ __forceinline__ void put_rows(const VCols& c, long long dst, long lon
   }
 }
 
-// Per tick key: its rank in the run and whether the run holds it.
+// Per tick key: its rank in the run and whether the run holds it; the keys
+// that it does not hold counted into *news.
 __global__ void k_merge_tick(const long long* __restrict__ run, long long R,
                              const long long* __restrict__ tick, long long T,
-                             long long* __restrict__ lb, long long* __restrict__ isnew) {
+                             long long* __restrict__ lb, long long* __restrict__ isnew,
+                             unsigned long long* __restrict__ news) {
+  unsigned mine = 0;
   for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < T;
        k += (long long)gridDim.x * blockDim.x) {
     const long long p = lower_bound(run, R, tick[k]);
     lb[k] = p;
-    isnew[k] = (p < R && run[p] == tick[k]) ? 0 : 1;
+    const bool fresh = !(p < R && run[p] == tick[k]);
+    isnew[k] = fresh ? 1 : 0;
+    mine += fresh;
   }
+  if (!news) return;
+  for (int o = 16; o; o >>= 1) mine += __shfl_xor_sync(FULL, mine, o);
+  if ((threadIdx.x & 31) == 0 && mine) atomicAdd(news, (unsigned long long)mine);
+}
+
+// A tick whose keys the run holds: each tick row combined into its run row.
+__global__ void k_merge_fold(const long long* __restrict__ lb, long long T, VCols c) {
+  for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < T;
+       k += (long long)gridDim.x * blockDim.x) {
+    const long long p = lb[k];
+    put_rows(c, p, p, k, false);
+  }
+}
+
+struct CopyCols {
+  const unsigned char* src[MAXV + 1];
+  unsigned char* dst[MAXV + 1];
+  long long bytes[MAXV + 1];
+};
+
+// Column blockIdx.y's bytes, 16 at a time where both sides allow it.
+__global__ void __launch_bounds__(256) k_copy_rows(CopyCols c) {
+  const unsigned char* __restrict__ src = c.src[blockIdx.y];
+  unsigned char* __restrict__ dst = c.dst[blockIdx.y];
+  const long long n = c.bytes[blockIdx.y];
+  const long long t = (long long)blockIdx.x * 256 + threadIdx.x, step = (long long)gridDim.x * 256;
+  long long done = 0;
+  if ((((uintptr_t)src | (uintptr_t)dst) & 15) == 0) {
+    for (long long i = t; i < n / 16; i += step)
+      reinterpret_cast<uint4*>(dst)[i] = reinterpret_cast<const uint4*>(src)[i];
+    done = n / 16 * 16;
+  } else if ((((uintptr_t)src | (uintptr_t)dst) & 3) == 0) {
+    for (long long i = t; i < n / 4; i += step)
+      reinterpret_cast<unsigned*>(dst)[i] = reinterpret_cast<const unsigned*>(src)[i];
+    done = n / 4 * 4;
+  }
+  for (long long i = done + t; i < n; i += step) dst[i] = src[i];
 }
 
 // Every run key moves up by the new tick keys below it; a matched key takes
@@ -730,7 +787,7 @@ extern "C" int pf_merge_sorted_runs(const int64_t* run_keys, const void* const* 
       PF_KERNEL("k_merge_tick", st);
       k_merge_tick<<<grid_of(n_tick, 256), 256, 0, st>>>((const long long*)run_keys, n_run,
                                                          (const long long*)tick_keys, n_tick,
-                                                         l.lb, l.isnew);
+                                                         l.lb, l.isnew, nullptr);
     }
     PF_LAUNCH("k_merge_tick");
     if (int rc = scan_i64(l.isnew, l.newex, n_tick, false, l.total, l.scratch, st)) return rc;
@@ -753,5 +810,83 @@ extern "C" int pf_merge_sorted_runs(const int64_t* run_keys, const void* const* 
   }
   PF_LAUNCH("k_merge_place_new");
   *n_out = n_run + num_new;
+  return ok();
+}
+
+extern "C" int pf_fold_sorted_run(const int64_t* run_keys, void* const* run_vals, int64_t n_run,
+                                  const int64_t* tick_keys, const void* const* tick_vals,
+                                  int64_t n_tick, int ncols, const int* kinds, const int* esizes,
+                                  const int* widths, const int* ops, int64_t* n_new,
+                                  void* workspace, size_t workspace_bytes, void* stream) {
+  cudaStream_t st = (cudaStream_t)stream;
+  if (n_run < 0 || n_tick < 0 || !n_new) return fail(PF_EINVAL, "fold_sorted_run: bad sizes");
+  if (int rc = check_cols(ncols, kinds, esizes, widths, ops, "fold_sorted_run")) return rc;
+  *n_new = 0;
+  if (n_tick == 0) return ok();
+  if ((n_run > 0 && !run_keys) || !tick_keys)
+    return fail(PF_EINVAL, "fold_sorted_run: null keys");
+  VCols c{};
+  c.n = ncols;
+  for (int q = 0; q < ncols; ++q) {
+    if ((n_run > 0 && !run_vals[q]) || !tick_vals[q])
+      return fail(PF_EINVAL, "fold_sorted_run: null value column %d", q);
+    c.a[q] = run_vals[q];
+    c.b[q] = tick_vals[q];
+    c.out[q] = run_vals[q];
+    c.kind[q] = kinds[q];
+    c.esize[q] = esizes[q];
+    c.width[q] = widths[q];
+    c.op[q] = ops[q];
+  }
+  Arena a(workspace, workspace_bytes);
+  MergeLayout l = merge_layout(a, n_tick);
+  if (!workspace || !a.fits())
+    return fail(PF_ENOSPACE, "fold_sorted_run: workspace of %zu bytes, %zu needed",
+                workspace_bytes, a.used);
+  PF_CUDA(cudaMemsetAsync(l.total, 0, sizeof(long long), st));
+  {
+    PF_KERNEL("k_merge_tick", st);
+    k_merge_tick<<<grid_of(n_tick, 256), 256, 0, st>>>(
+        (const long long*)run_keys, n_run, (const long long*)tick_keys, n_tick, l.lb, l.isnew,
+        (unsigned long long*)l.total);
+  }
+  PF_LAUNCH("k_merge_tick");
+  long long news = 0;
+  if (int rc = read_words(l.total, 1, &news, st)) return rc;
+  *n_new = news;
+  if (news || ncols == 0) return ok();
+  {
+    PF_KERNEL("k_merge_fold", st);
+    k_merge_fold<<<grid_of(n_tick, 256), 256, 0, st>>>(l.lb, n_tick, c);
+  }
+  PF_LAUNCH("k_merge_fold");
+  return ok();
+}
+
+extern "C" int pf_copy_rows(const void* const* src, void* const* dst, const int* row_bytes,
+                            int ncols, int64_t n, void* stream) {
+  cudaStream_t st = (cudaStream_t)stream;
+  if (ncols < 0 || ncols > MAXV + 1)
+    return fail(PF_EINVAL, "copy_rows: at most %d columns", MAXV + 1);
+  if (n < 0) return fail(PF_EINVAL, "copy_rows: negative rows");
+  if (n == 0 || ncols == 0) return ok();
+  CopyCols c{};
+  long long most = 0;
+  for (int q = 0; q < ncols; ++q) {
+    if (!src[q] || !dst[q] || row_bytes[q] < 1)
+      return fail(PF_EINVAL, "copy_rows: column %d is null or has no bytes", q);
+    c.src[q] = (const unsigned char*)src[q];
+    c.dst[q] = (unsigned char*)dst[q];
+    c.bytes[q] = n * row_bytes[q];
+    most = std::max(most, c.bytes[q]);
+  }
+  const dim3 grid((unsigned)std::max<long long>(
+                      1, std::min<long long>((most + 4095) / 4096, (long long)sm_count() * 8)),
+                  ncols);
+  {
+    PF_KERNEL("k_copy_rows", st);
+    k_copy_rows<<<grid, 256, 0, st>>>(c);
+  }
+  PF_LAUNCH("k_copy_rows");
   return ok();
 }

@@ -14,6 +14,12 @@ One chunk's rows are reduced to one row per group:
   buckets   with B > 1, each group's bucket (``_bucket_ids``) and the groups
             per bucket, on the host and on the device (pf_hash_buckets)
 
+A chunk whose rows share groups (two a group or more) takes hash and groups
+in one read of its rows (pf_keyed_pass1_read, _emit: a place of a hash table
+holds every accumulator of its group); one of mostly single rows, or of
+columns that the table does not hold (floats' min and max, two-dimensional or
+narrow values), the steps above.
+
 Aggregates: ``('sum', col)``, ``('count', None)`` (every row) or
 ``('count', col)`` (the rows whose value is not the null -64), ``('min',
 col)``, ``('max', col)`` (folded from 0, as the reference's partial is) and
@@ -102,6 +108,15 @@ def _unpack_words(words: torch.Tensor, like: torch.Tensor) -> torch.Tensor:
     return raw.view(like.dtype).reshape(n, like.shape[1])
 
 
+# accumulators, column kinds and outputs of pf_keyed_pass1_read and _emit
+_KA_WORD, _KA_COUNT, _KA_NULLS, _KA_SUM_I, _KA_SUM_F, _KA_MIN, _KA_MAX = range(7)
+_KK = {torch.int64: 0, torch.int32: 1, torch.float64: 2, torch.float32: 3}
+(_KO_WORD, _KO_I64, _KO_I32, _KO_F64, _KO_F32, _KO_I64_MAX0, _KO_I32_MAX0, _KO_COUNT, _KO_AVG_I,
+ _KO_AVG_F) = range(10)
+_MAX_ACCS, _MAX_OUTS, _MAX_KEYS, _MAX_B = 15, 40, 8, 4096
+_MAX_EXPECT = 1 << 24
+
+
 class KeyedPass1:
     """Pass 1 of a keyed aggregation over plain columns: ``key_ids`` group
     the rows (``emitted_ids``, default all of them, are carried out as key
@@ -116,6 +131,7 @@ class KeyedPass1:
             if op not in ('sum', 'count', 'min', 'max', 'avg'):
                 raise NotImplementedError(f"KeyedPass1: aggregate {op!r}")
         self._coeffs = None
+        self._laid = None   # (column types and widths, _layout's answer for them)
 
     def pass1(self, columns: Dict[int, torch.Tensor], B: int = 1):
         """``[hash] + keys + values`` of one chunk (hash ascending, unique),
@@ -124,51 +140,217 @@ class KeyedPass1:
         keys = [_as_2d(columns[k]) for k in self.key_ids]
         if self._coeffs is None:
             self._coeffs = make_key_coeffs(keys, keys[0].device)
+        out = self._one_read(columns, keys, B)
+        if out is not None:
+            return out
+        out = self._hash_and_sort(columns, keys)
+        buckets = None
+        if B > 1 and out[0].numel() > 0:
+            buckets = hash_buckets(out[0], B)
+        return out, buckets
+
+    def _layout(self, keys, cols):
+        """What pf_keyed_pass1_read does for columns of these types and widths:
+        its accumulators and outputs without their pointers, which column each
+        accumulator reads, and each result column's dtype and width; None when
+        it does not take them."""
+        accs, source, where = [], [], {}
+
+        def acc(op, cid=None, kind=0, row_bytes=0, word=0):
+            at = where.get((op, cid, word))
+            if at is None:
+                at = where[(op, cid, word)] = len(accs)
+                accs.append(_native.KeyedAcc(op, kind, row_bytes, word, None))
+                source.append(None if cid is None else (op == _KA_WORD, cid))
+            return at
+
+        outs, dest, results = [], [], []
+
+        def out(*fields):
+            outs.append(_native.KeyedOut(*fields, None))
+            dest.append(len(results))
+
+        for e in self.emitted:
+            k = keys[e]
+            rb = k.shape[1] * k.element_size()
+            for w in range(packed_width(k)):
+                out(_KO_WORD, acc(_KA_WORD, e, 0, rb, w), 0, 0, rb, w)
+            results.append((k.dtype, k.shape[1]))
+        for op, cid in self.aggs:
+            v = None if cid is None else cols[cid]
+            fp = v is not None and v.dtype.is_floating_point
+            kind = 0 if v is None else _KK[v.dtype]
+            if op == 'count':
+                c = acc(_KA_COUNT)
+                if v is None:
+                    out(_KO_I64, c, 0, 0, 0, 0)
+                else:
+                    out(_KO_COUNT, c, acc(_KA_NULLS, cid, kind), 0, 0, 0)
+                results.append((torch.int64, 1))
+            elif op == 'avg':
+                s = acc(_KA_SUM_F if fp else _KA_SUM_I, cid, kind)
+                out(_KO_AVG_F if fp else _KO_AVG_I, s, acc(_KA_COUNT), acc(_KA_NULLS, cid, kind),
+                    0, 0)
+                results.append((torch.float64, 2))
+            elif op == 'sum':
+                s = acc(_KA_SUM_F if fp else _KA_SUM_I, cid, kind)
+                out({torch.float64: _KO_F64, torch.float32: _KO_F32}.get(v.dtype, _KO_I64), s, 0,
+                    0, 0, 0)
+                results.append((v.dtype if fp else torch.int64, 1))
+            elif fp:
+                return None
+            else:
+                wide = v.dtype == torch.int64
+                m = acc(_KA_MIN if op == 'min' else _KA_MAX, cid, kind)
+                # MAX folds into a zeroed partial (operator_utils.py:365-369)
+                out((_KO_I64 if wide else _KO_I32) if op == 'min' else
+                    (_KO_I64_MAX0 if wide else _KO_I32_MAX0), m, 0, 0, 0, 0)
+                results.append((v.dtype, 1))
+        if len(accs) > _MAX_ACCS or len(outs) > _MAX_OUTS:
+            return None
+        return (bytes((_native.KeyedAcc * max(1, len(accs)))(*accs)), source,
+                bytes((_native.KeyedOut * max(1, len(outs)))(*outs)), dest, results)
+
+    def _one_read(self, columns, keys, B=1):
+        """pass1 by pf_keyed_pass1_read, or None when a column's type or shape or
+        the number of groups is not its."""
+        n, dev = keys[0].shape[0], keys[0].device
+        if (n == 0 or dev.type != 'cuda' or len(keys) > _MAX_KEYS or not 1 <= B <= _MAX_B
+                or B & (B - 1) or not set(self.emitted) <= set(self.key_ids)
+                or any(k.dim() != 2 or k.shape[0] != n or k.shape[1] == 0 or k.device != dev
+                       for k in keys)):
+            return None
+        cols = {cid: columns[cid] for _, cid in self.aggs if cid is not None}
+        if any(v.dim() != 1 or v.shape[0] != n or v.device != dev or v.dtype not in _KK
+               for v in cols.values()):
+            return None
+        # the layout depends on types and widths alone
+        sig = (tuple((k.dtype, k.shape[1]) for k in keys),
+               tuple(v.dtype for v in cols.values()))
+        if self._laid is None or self._laid[0] != sig:
+            self._laid = (sig, self._layout(dict(zip(self.key_ids, keys)), cols))
+        lay = self._laid[1]
+        if lay is None:
+            return None
+        acc_bytes, source, out_bytes, dest, results = lay
+        L = lib()
+        nk, na, no = len(keys), len(source), len(dest)
+        keys = [k.contiguous() for k in keys]
+        held = {True: dict(zip(self.key_ids, keys)),
+                False: {cid: v.contiguous() for cid, v in cols.items()}}
+        coeffs = [c.contiguous() for c in self._coeffs]
+        accs = (_native.KeyedAcc * max(1, na)).from_buffer_copy(acc_bytes)
+        for a, src in zip(accs, source):
+            if src is not None:
+                a.src = held[src[0]][src[1]].data_ptr()
+        kcols = (ctypes.c_void_p * nk)(*[k.data_ptr() for k in keys])
+        kbytes = (ctypes.c_int * nk)(*[k.shape[1] * k.element_size() for k in keys])
+        kcoeffs = (ctypes.c_void_p * nk)(*[c.data_ptr() for c in coeffs])
+        groups, crowded = ctypes.c_int64(), ctypes.c_int64()
+        expect = 0
+        with torch.cuda.device(dev):
+            st = stream_of(dev)
+            while True:
+                ws_bytes = L.pf_keyed_pass1_workspace(n, na, expect)
+                ws = _native.workspace(ws_bytes, dev)
+                check(L.pf_keyed_pass1_read(kcols, kbytes, kcoeffs, nk, n, accs, na, expect,
+                                            ws.data_ptr(), ws_bytes, st), "keyed_pass1")
+                # the outputs are made while the rows are read
+                room = L.pf_keyed_pass1_groups(n, na, expect)
+                res = [torch.empty((room, w) if w > 1 else room, dtype=dt, device=dev)
+                       for dt, w in results]
+                outs = (_native.KeyedOut * max(1, no)).from_buffer_copy(out_bytes)
+                for o, i in zip(outs, dest):
+                    o.dst = res[i].data_ptr()
+                h = torch.empty(room, dtype=torch.int64, device=dev)
+                bucket = counts = None
+                host_counts = (ctypes.c_int64 * B)()
+                if B > 1:
+                    bucket = torch.empty(room, dtype=torch.int32, device=dev)
+                    counts = torch.empty(B, dtype=torch.int64, device=dev)
+                sort_ws = None
+                while True:
+                    check(L.pf_keyed_pass1_emit(
+                        n, accs, na, expect, outs, no, h.data_ptr(), B, ptr(bucket), ptr(counts),
+                        host_counts, ctypes.byref(groups), ctypes.byref(crowded), ws.data_ptr(),
+                        ws_bytes, ptr(sort_ws), crowded.value, st), "keyed_pass1")
+                    if not crowded.value:
+                        break
+                    sort_ws = _native.workspace(crowded.value, dev)
+                g = groups.value
+                if g >= 0:
+                    break
+                # more groups than the table holds, about -g: once more into
+                # one for them, unless most rows are a group of their own (the
+                # general route is as fast then, at a smaller workspace)
+                if expect or -g > 2 * n // 3 or -g > _MAX_EXPECT:
+                    return None
+                expect = -g
+        buckets = (bucket[:g], list(host_counts), counts) if B > 1 and g > 0 else None
+        return [h[:g]] + [t[:g] for t in res], buckets
+
+    def _hash_and_sort(self, columns, keys):
+        """pass1's columns by the grouping hash of every row, a radix sort
+        and a segmented reduction a column (pf_group_hash, pf_unique_reduce)."""
         h = group_hash(keys, self._coeffs)
-        vals, ops, post = [], [], []
+        vals, ops, post, at = [], [], [], {}
+
+        def column(name, make, op):
+            """The value column `name`'s place, made once: AVG(x)'s sum is
+            SUM(x)'s."""
+            if name not in at:
+                at[name] = len(vals)
+                vals.append(make())
+                ops.append(op)
+            return at[name]
+
         emitted = [_as_2d(columns[k]) for k in self.emitted]
         for e in emitted:
             vals.append(_pack_words(e))
             ops.append('amax')   # every row of a group holds the same key
         n = h.numel()
+
+        def summed(cid):
+            v = columns[cid]
+            # integer sums in int64, as the reference's result
+            return v if v.dtype in (torch.float32, torch.float64) else v.to(torch.int64)
+
+        def non_null(cid):
+            # COUNT(x) counts the rows whose x is not the null value
+            # (operator_utils.py:384-385); COUNT(*) every row
+            return (columns[cid] != NULL).to(torch.int64)
+
+        def ranged(cid):
+            v = columns[cid]
+            return v if v.dtype in (torch.float32, torch.float64, torch.int64, torch.int32) \
+                else v.to(torch.int64)
+
         for op, cid in self.aggs:
             if op == 'count':
-                # COUNT(x) counts the rows whose x is not the null value
-                # (operator_utils.py:384-385); COUNT(*) every row
-                if cid is None:
-                    vals.append(torch.ones(n, dtype=torch.int64, device=h.device))
-                else:
-                    vals.append((columns[cid] != NULL).to(torch.int64))
-                ops.append('sum')
-                post.append(('count', len(vals) - 1))
+                j = (column('rows', lambda: torch.ones(n, dtype=torch.int64, device=h.device),
+                            'sum') if cid is None else
+                     column(('non_null', cid), lambda: non_null(cid), 'sum'))
+                post.append(('count', j, None))
             elif op == 'avg':
                 # the state [SUM(x), COUNT(x)] (aggregate.py:249-250, 323-336):
                 # the sum over every row, the count over the non-null ones
-                v = columns[cid]
-                vals.append(v if v.dtype in (torch.float32, torch.float64) else v.to(torch.int64))
-                ops.append('sum')
-                vals.append((v != NULL).to(torch.int64))
-                ops.append('sum')
-                post.append(('avg', len(vals) - 2))
+                post.append(('avg', column(('sum', cid), lambda: summed(cid), 'sum'),
+                             column(('non_null', cid), lambda: non_null(cid), 'sum')))
+            elif op == 'sum':
+                post.append((op, column(('sum', cid), lambda: summed(cid), 'sum'), None))
             else:
-                v = columns[cid]
-                if v.dtype in (torch.float32, torch.float64):
-                    pass
-                elif op == 'sum' or v.dtype not in (torch.int64, torch.int32):
-                    v = v.to(torch.int64)   # integer sums in int64, as the reference's result
-                vals.append(v)
-                ops.append({'sum': 'sum', 'min': 'amin', 'max': 'amax'}[op])
-                post.append((op, len(vals) - 1))
+                post.append((op, column((op, cid), lambda: ranged(cid),
+                                        {'min': 'amin', 'max': 'amax'}[op]), None))
         u, red = reduce_tick_slice(h, vals, ops)
         key_reps = []
         for i, e in enumerate(emitted):
             rep = _unpack_words(red[i], e)
             key_reps.append(rep.squeeze(1) if rep.shape[1] == 1 else rep)
         agg_vals = []
-        for op, j in post:
+        for op, j, j2 in post:
             if op == 'avg':
                 agg_vals.append(torch.stack([red[j].to(torch.float64),
-                                             red[j + 1].to(torch.float64)], dim=1))
+                                             red[j2].to(torch.float64)], dim=1))
             elif op == 'max':
                 # MAX folds into a zeroed partial (a scatter_reduce into zeros
                 # that includes them, operator_utils.py:365-369), so a group
@@ -176,7 +358,4 @@ class KeyedPass1:
                 agg_vals.append(torch.clamp_min(red[j], 0))
             else:
                 agg_vals.append(red[j])
-        buckets = None
-        if B > 1 and u.numel() > 0:
-            buckets = hash_buckets(u, B)
-        return [u] + key_reps + agg_vals, buckets
+        return [u] + key_reps + agg_vals

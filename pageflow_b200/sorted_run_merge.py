@@ -10,7 +10,10 @@ functions, arguments and results).
   fixed buffers, returning the merged length (pf_merge_sorted_runs: binary
   searches place every key, matched keys combine; the merge is computed out
   of place into a temporary of the merged size and copied back, where the
-  reference shifts in place in chunks: the same result, a larger peak).
+  reference shifts in place in chunks: the same result, a larger peak).  A
+  tick without a new key, the usual one once every group has been met, is
+  combined in place (pf_fold_sorted_run): 250K keys of seven columns into a
+  run of 250K, 33 us of GPU work and 8 copies less a merge.
 """
 from __future__ import annotations
 
@@ -81,6 +84,28 @@ def reduce_tick_slice(keys: torch.Tensor, vals: Sequence[torch.Tensor],
     return out_k[:u], [o[:u] for o in outs]
 
 
+def _copy_rows(dst: Sequence[torch.Tensor], src: Sequence[torch.Tensor], n: int) -> None:
+    """``d[:n] = s[:n]`` for every pair, the plain ones in one launch."""
+    plain = []
+    for d, s in zip(dst, src):
+        if (d.is_cuda and s.is_cuda and d.device == s.device and d.dtype == s.dtype
+                and d.shape[1:] == s.shape[1:] and d.shape[0] >= n and s.shape[0] >= n
+                and d.is_contiguous() and s.is_contiguous() and d[:1].numel() > 0
+                and not d.requires_grad and not s.requires_grad
+                and d.untyped_storage().data_ptr() != s.untyped_storage().data_ptr()):
+            plain.append((d, s))
+        else:
+            d[:n] = s[:n]
+    for i in range(0, len(plain), 16):
+        part = plain[i:i + 16]
+        rb = [d.element_size() * (d.numel() // d.shape[0]) for d, _ in part]
+        with torch.cuda.device(part[0][0].device):
+            check(lib().pf_copy_rows(arr(ctypes.c_void_p, [ptr(s) for _, s in part]),
+                                     arr(ctypes.c_void_p, [ptr(d) for d, _ in part]),
+                                     arr(ctypes.c_int, rb), len(part), n,
+                                     stream_of(part[0][0].device)), "copy_rows")
+
+
 def merge_sorted_unique_runs_inplace(key_buf: torch.Tensor, val_bufs: Sequence[torch.Tensor],
                                      run_len: int, tick_keys: torch.Tensor,
                                      tick_vals: Sequence[torch.Tensor], ops: Sequence[str],
@@ -92,23 +117,33 @@ def merge_sorted_unique_runs_inplace(key_buf: torch.Tensor, val_bufs: Sequence[t
     if T == 0:
         return run_len
     if run_len == 0:
-        key_buf[:T] = tick_keys
-        for vb, tv in zip(val_bufs, tick_vals):
-            vb[:T] = tv
+        _copy_rows([key_buf] + list(val_bufs), [tick_keys] + list(tick_vals), T)
         return T
     R = run_len
     dev = key_buf.device
     kinds, sizes, widths, opc = _describe(list(tick_vals), ops, "merge_sorted_unique_runs")
     tick_keys = tick_keys.contiguous()
     tick_vals = [t.contiguous() for t in tick_vals]
+    ws_bytes = lib().pf_merge_sorted_runs_workspace(T)
+    ws = _native.workspace(ws_bytes, dev)
+    m = ctypes.c_int64()
+    nc = max(1, len(val_bufs))
+    if (key_buf.dtype == torch.int64 and len(val_bufs) == len(tick_vals) and all(
+            b.is_cuda and b.device == t.device and b.is_contiguous() and b.dtype == t.dtype
+            and b.shape[1:] == t.shape[1:] and b.shape[0] >= R and t.shape[0] == T
+            for b, t in zip([key_buf] + list(val_bufs), [tick_keys] + tick_vals))):
+        check(lib().pf_fold_sorted_run(
+            ptr(key_buf), (ctypes.c_void_p * nc)(*[ptr(v) for v in val_bufs]), R,
+            ptr(tick_keys), (ctypes.c_void_p * nc)(*[ptr(v) for v in tick_vals]), T,
+            len(val_bufs), kinds, sizes, widths, opc, ctypes.byref(m), ptr(ws), ws_bytes,
+            stream_of(dev)), "merge_sorted_unique_runs")
+        if m.value == 0:
+            return R
     run_vals = [vb[:R].contiguous() for vb in val_bufs]
     cap = R + T
     out_k = torch.empty(cap, dtype=torch.int64, device=dev)
     outs = [torch.empty((cap,) + tuple(vb.shape[1:]), dtype=vb.dtype, device=dev)
             for vb in val_bufs]
-    ws = _native.workspace(lib().pf_merge_sorted_runs_workspace(T), dev)
-    m = ctypes.c_int64()
-    nc = max(1, len(val_bufs))
     a = (ctypes.c_void_p * nc)(*[ptr(v) for v in run_vals])
     b = (ctypes.c_void_p * nc)(*[ptr(v) for v in tick_vals])
     o = (ctypes.c_void_p * nc)(*[ptr(v) for v in outs])
@@ -121,9 +156,7 @@ def merge_sorted_unique_runs_inplace(key_buf: torch.Tensor, val_bufs: Sequence[t
     assert M <= key_buf.shape[0], (
         f"merge capacity exhausted: M={M} > buf={key_buf.shape[0]} — the buffers must be "
         f"sized to the pass2 total input rows")
-    key_buf[:M] = out_k[:M]
-    for vb, ov in zip(val_bufs, outs):
-        vb[:M] = ov[:M]
+    _copy_rows([key_buf] + list(val_bufs), [out_k] + outs, M)
     return M
 
 
