@@ -318,6 +318,24 @@ int pf_join_aggregate_ex(const int64_t* build_key, const int32_t* build_group, i
                          int64_t* count_out, int64_t* stats_out, const pf_join_knobs* knobs,
                          void* workspace, size_t workspace_bytes, void* stream);
 /*
+ * The same join without a radix pass, for builds whose hash table fits L2
+ * (pf_join_direct_fits: 1 for sizes it takes, about 6.7M build rows and, in
+ * the largest table, half a million groups at most; 0 else): one table over all
+ * build rows, each probe row looked up in it.  Outputs as
+ * pf_join_aggregate's and, with keys_out, the occupied groups as
+ * pf_groups_finish's (*n_out of them, host).  Waits once.  *done (host) is 0
+ * when the build keys' hashes crowd its table: nothing was joined, take
+ * pf_join_aggregate.
+ */
+int pf_join_direct_fits(int64_t n_build, int64_t n_probe, int64_t n_groups);
+size_t pf_join_direct_workspace(int64_t n_build, int64_t n_groups);
+int pf_join_direct(const int64_t* build_key, const int32_t* build_group, int64_t n_build,
+                   const int64_t* probe_fk, const int64_t* probe_price,
+                   const int64_t* probe_disc, int64_t scale, int64_t n_probe, int64_t group_min,
+                   int64_t n_groups, int64_t* sum_out, int64_t* count_out, int64_t* stats_out,
+                   int64_t* keys_out, int64_t* sums_out, int64_t* counts_out, int64_t* n_out,
+                   int* done, void* workspace, size_t workspace_bytes, void* stream);
+/*
  * The fused join + group-by sharded over ranks, in its two rank-local
  * phases (no counterpart in the reference, which runs on one GPU; the
  * exchange between them is the caller's, e.g. NCCL all-to-alls):

@@ -72,6 +72,11 @@ _SIGS = {
     "pf_join_aggregate_workspace_ex": (_sz, [_i64, _i64, _int, _i64, _vp]),
     "pf_join_aggregate_ex": (_int, [_vp, _vp, _i64, _vp, _vp, _vp, _i64, _i64, _int, _i64, _i64,
                                     _vp, _vp, _vp, _vp, _vp, _sz, _vp]),
+    "pf_join_direct_fits": (_int, [_i64, _i64, _i64]),
+    "pf_join_direct_workspace": (_sz, [_i64, _i64]),
+    "pf_join_direct": (_int, [_vp, _vp, _i64, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _vp, _vp,
+                              _vp, _vp, _vp, _vp, ctypes.POINTER(_i64), ctypes.POINTER(_int),
+                              _vp, _sz, _vp]),
     "pf_join_partition_workspace": (_sz, [_i64, _i64, _int]),
     "pf_join_partition": (_int, [_vp, _vp, _i64, _vp, _vp, _vp, _i64, _i64, _int, _vp, _vp, _vp,
                                  _vp, _vp, _sz, _vp]),

@@ -1322,7 +1322,8 @@ struct SJArgs {
   long long S;
   int logS;
   long long group_min, n_groups;
-  unsigned long long* slab;
+  unsigned long long* slab;        // [reps][2 * n_groups]
+  int reps;
   unsigned long long* stats;
   unsigned long long* counter;
   const unsigned long long* ovf;   // nonzero: a region overflowed, nothing to join
@@ -1412,6 +1413,9 @@ __global__ void __launch_bounds__(SJT, PF_SJ_MINB) k_sjoin(SJArgs a) {
     sj_sum_clear(S, t);
     S.cnt[t] = 0;
   }
+  // this block's copy of the groups' sums (slab_reps)
+  unsigned long long* const slab =
+      a.slab + 2ULL * (unsigned)(blockIdx.x % a.reps) * (unsigned long long)a.n_groups;
   unsigned matched = 0;  // rows a thread matched (below 2^32: at most 2^40 / SJT)
   unsigned bad_group = 0;  // below 2^32: a thread flushes at most 2^40 / SJT rows
   // Thread 0 fetches the next sub-partition and its ranges into the other
@@ -1538,8 +1542,8 @@ __global__ void __launch_bounds__(SJT, PF_SJ_MINB) k_sjoin(SJArgs a) {
         const bool gok = g >= 0 && g < a.n_groups;
         bad_group += !gok;
         if (c && gok) {
-          atomicAdd(&a.slab[2 * (unsigned long long)g], sj_sum_get(S, t));
-          atomicAdd(&a.slab[2 * (unsigned long long)g + 1], (unsigned long long)c);
+          atomicAdd(&slab[2 * (unsigned long long)g], sj_sum_get(S, t));
+          atomicAdd(&slab[2 * (unsigned long long)g + 1], (unsigned long long)c);
         }
         S.key[t] = SJ_EMPTY;
         sj_sum_clear(S, t);
@@ -1549,8 +1553,8 @@ __global__ void __launch_bounds__(SJT, PF_SJ_MINB) k_sjoin(SJArgs a) {
         if (S.has_min) {
           bad_group += S.min_goff == SJ_NONE;
           if (S.min_cnt && S.min_goff != SJ_NONE) {
-            atomicAdd(&a.slab[2 * (unsigned long long)S.min_goff], (unsigned long long)S.min_sum);
-            atomicAdd(&a.slab[2 * (unsigned long long)S.min_goff + 1],
+            atomicAdd(&slab[2 * (unsigned long long)S.min_goff], (unsigned long long)S.min_sum);
+            atomicAdd(&slab[2 * (unsigned long long)S.min_goff + 1],
                       (unsigned long long)S.min_cnt);
           }
         }
@@ -1613,6 +1617,8 @@ __global__ void __launch_bounds__(SJF_T, PF_SJF_MINB) k_sjoin_fp(SJArgs a) {
   extern __shared__ __align__(16) unsigned char sjf_smem[];
   SJFSmem& S = *reinterpret_cast<SJFSmem*>(sjf_smem);
   if (*a.ovf || (a.ovf1 && *a.ovf1)) return;  // the partitions are incomplete: the host runs the counted passes
+  unsigned long long* const slab =
+      a.slab + 2ULL * (unsigned)(blockIdx.x % a.reps) * (unsigned long long)a.n_groups;
   const int tid = threadIdx.x;
   for (int t = tid; t < SJF_TS; t += SJF_T) S.slot[t] = 0;
   for (int r = tid; r < SJF_CAP; r += SJF_T) {
@@ -1707,9 +1713,9 @@ __global__ void __launch_bounds__(SJF_T, PF_SJF_MINB) k_sjoin_fp(SJArgs a) {
         const bool gok = g >= 0 && g < a.n_groups;
         bad_group += !gok;
         if (c && gok) {
-          atomicAdd(&a.slab[2 * (unsigned long long)g],
+          atomicAdd(&slab[2 * (unsigned long long)g],
                     ((unsigned long long)S.hi[j] << 32) | S.lo[j]);
-          atomicAdd(&a.slab[2 * (unsigned long long)g + 1], (unsigned long long)c);
+          atomicAdd(&slab[2 * (unsigned long long)g + 1], (unsigned long long)c);
         }
         S.slot[S.slot_of[j]] = 0;
         S.lo[j] = 0;
@@ -1758,12 +1764,50 @@ Knobs resolve_knobs(const pf_join_knobs* k) {
   return r;
 }
 
-// The interleaved slab split into the caller's sum and count arrays.
-__global__ void k_split(const unsigned long long* __restrict__ slab, long long n,
-                        long long* __restrict__ sum, long long* __restrict__ count) {
-  for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < n;
-       g += (long long)gridDim.x * blockDim.x) {
-    const ulonglong2 v = reinterpret_cast<const ulonglong2*>(slab)[g];
+// The copies of the groups' sums that the join's blocks add into, each block
+// into its own by its number: a few groups' build rows would otherwise queue up
+// on a few addresses (25 groups: 9M x 45M rows 6.2 ms, with a copy a block
+// 1.13; 20M x 100M 13.6 and 2.36). More than 64K groups have one.
+constexpr long long SLAB_SPREAD = 1 << 17;  // pairs the copies take, at most
+int slab_reps(long long n_groups) {
+  return (int)std::max<long long>(1, std::min<long long>(512, SLAB_SPREAD / std::max(1LL, n_groups)));
+}
+
+// The interleaved slab (its copies added up) split into the caller's sum and
+// count arrays: a warp a group's copies where there are many, else a thread.
+__global__ void __launch_bounds__(256) k_split(const unsigned long long* __restrict__ slab,
+                                               long long n, int reps,
+                                               long long* __restrict__ sum,
+                                               long long* __restrict__ count) {
+  const ulonglong2* __restrict__ s = reinterpret_cast<const ulonglong2*>(slab);
+  const long long t = (long long)blockIdx.x * 256 + threadIdx.x, step = (long long)gridDim.x * 256;
+  if (reps >= 32) {
+    const int lane = threadIdx.x & 31;
+    for (long long g = t >> 5; g < n; g += step >> 5) {
+      unsigned long long x = 0, y = 0;
+      for (int r = lane; r < reps; r += 32) {
+        const ulonglong2 v = s[(long long)r * n + g];
+        x += v.x;
+        y += v.y;
+      }
+      for (int o = 16; o; o >>= 1) {
+        x += __shfl_xor_sync(FULL, x, o);
+        y += __shfl_xor_sync(FULL, y, o);
+      }
+      if (lane == 0) {
+        sum[g] = (long long)x;
+        count[g] = (long long)y;
+      }
+    }
+    return;
+  }
+  for (long long g = t; g < n; g += step) {
+    ulonglong2 v = s[g];
+    for (int r = 1; r < reps; ++r) {
+      const ulonglong2 w = s[(long long)r * n + g];
+      v.x += w.x;
+      v.y += w.y;
+    }
     sum[g] = (long long)v.x;
     count[g] = (long long)v.y;
   }
@@ -1876,7 +1920,8 @@ struct JaLayout {
   Slot* table;
   long long table_slots;
   long long* reg;      // [2B]: reg_off, reg_cap
-  unsigned long long* slab;  // [2 * n_groups]: (sum, count) per group
+  unsigned long long* slab;  // [reps][2 * n_groups]: (sum, count) per group
+  int reps;
   long long max_launches;
   unsigned* counters;        // [max_launches] work counters of the round launches
   // the shared-memory path
@@ -1952,7 +1997,8 @@ JaLayout ja_layout(Arena& a, long long nb, long long np, int B, long long n_grou
   l.start = a.take<long long>(2 * (size_t)B);
   l.total = a.take<long long>(2);
   l.reg = a.take<long long>(2 * (size_t)B);
-  l.slab = a.take<unsigned long long>(2 * (size_t)std::max<long long>(n_groups, 1));
+  l.reps = slab_reps(n_groups);
+  l.slab = a.take<unsigned long long>(2 * (size_t)std::max<long long>(n_groups, 1) * l.reps);
   l.ovf = a.take<unsigned long long>(2);
   if (!kn.smem) {
     l.pkey = a.take<long long>(std::max<long long>(nb, 1));
@@ -2344,6 +2390,7 @@ int join_smem(const JaLayout& l, const P1View& v, const Knobs& kn, int B, int lo
     a.group_min = group_min;
     a.n_groups = n_groups;
     a.slab = l.slab;
+    a.reps = l.reps;
     a.stats = (unsigned long long*)stats_out;
     a.counter = l.sj_counter;
     a.ovf = l.ovf + 1;
@@ -2368,8 +2415,10 @@ int join_smem(const JaLayout& l, const P1View& v, const Knobs& kn, int B, int lo
     {
       PF_KERNEL("k_split", st);
       k_split<<<(unsigned)std::max<long long>(
-                    1, std::min<long long>((n_groups + 255) / 256, sms * 8LL)),
-                256, 0, st>>>(l.slab, n_groups, (long long*)sum_out, (long long*)count_out);
+                    1, std::min<long long>((n_groups * (l.reps >= 32 ? 32 : 1) + 255) / 256,
+                                           sms * 8LL)),
+                256, 0, st>>>(l.slab, n_groups, l.reps, (long long*)sum_out,
+                              (long long*)count_out);
     }
     PF_LAUNCH("k_split");
     g_counted_passes = (g_counted_passes & 1) | (counted[0] || counted[1] ? 2 : 0);
@@ -2461,7 +2510,7 @@ extern "C" int pf_join_aggregate_ex(const int64_t* build_key, const int32_t* bui
     PF_CUDA(cudaMemsetAsync(count_out, 0, n_groups * sizeof(long long), st));
     return ok();
   }
-  PF_CUDA(cudaMemsetAsync(l.slab, 0, 2 * n_groups * sizeof(unsigned long long), st));
+  PF_CUDA(cudaMemsetAsync(l.slab, 0, 2 * n_groups * l.reps * sizeof(unsigned long long), st));
 
   long long* hc = pinned_counts(2 * (size_t)B + 8);
   if (!hc) return fail(PF_ECUDA, "join_aggregate: no pinned staging buffer");
@@ -2662,7 +2711,7 @@ extern "C" int pf_join_aggregate_ex(const int64_t* build_key, const int32_t* bui
   {
     PF_KERNEL("k_split", st);
     k_split<<<(unsigned)std::max<long long>(1, std::min<long long>((n_groups + 255) / 256, sms * 8LL)),
-              256, 0, st>>>(l.slab, n_groups, (long long*)sum_out, (long long*)count_out);
+              256, 0, st>>>(l.slab, n_groups, 1, (long long*)sum_out, (long long*)count_out);
   }
   PF_LAUNCH("k_split");
   return ok();
@@ -2763,7 +2812,8 @@ JaLayout buckets_layout(Arena& a, const int64_t* counts, int nbk, long long n_gr
       rows[side] += counts[(size_t)side * nbk + p];
       maxp[side] = std::max<long long>(maxp[side], counts[(size_t)side * nbk + p]);
     }
-  l.slab = a.take<unsigned long long>(2 * (size_t)std::max<long long>(n_groups, 1));
+  l.reps = slab_reps(n_groups);
+  l.slab = a.take<unsigned long long>(2 * (size_t)std::max<long long>(n_groups, 1) * l.reps);
   l.ovf = a.take<unsigned long long>(2);
   take_second_pass(a, l, rows[0], rows[1], nbk, maxp, kn.target);
   return l;
@@ -2863,7 +2913,7 @@ extern "C" int pf_join_aggregate_buckets(const int64_t* build_hash, const int32_
     PF_CUDA(cudaMemsetAsync(count_out, 0, n_groups * sizeof(long long), st));
     return ok();
   }
-  PF_CUDA(cudaMemsetAsync(l.slab, 0, 2 * n_groups * sizeof(unsigned long long), st));
+  PF_CUDA(cudaMemsetAsync(l.slab, 0, 2 * n_groups * l.reps * sizeof(unsigned long long), st));
   long long* hc = pinned_counts(8);
   if (!hc) return fail(PF_ECUDA, "join_aggregate_buckets: no pinned staging buffer");
   return join_smem(l, P1View{(const long long*)build_hash, build_group, (const P2Row*)probe_rec},

@@ -1,0 +1,799 @@
+// The fused join -> group-by without a radix pass, for builds whose hash table
+// fits L2: the build rows go into one table, each probe row is read once, its
+// group looked up and its value added, and the groups are written out.
+//
+//   k_dj_init    the table emptied, the sums zeroed
+//   k_dj_build   each build row into the table
+//   k_dj_probe   each probe row hashed and looked up, its value and 1 added to
+//                its group
+//   k_dj_finish  the sums and counts, and the occupied groups ascending
+//
+// The radix path (join_aggregate.cu) moves a build row through two passes and
+// a probe row through 24 + 16 + 16 + 16 + 16 bytes, over 20 launches and two
+// waits; here a probe row is 24 bytes read, one 32-byte sector of the table
+// and one RED.  What bounds it: L2's rate of requests (about 0.2 T/s reached
+// for a random read and a RED a row; the figures are at dj_table).
+//
+// The table.  2^q buckets of four 8-byte entries, a bucket one sector.  A key's
+// hash is a bijection of it, so its top q bits (the home bucket) and the 64 - q
+// others (the remainder, held in the entry) are the key itself.  An entry is
+// {remainder, distance of its bucket from home, group}; a lookup compares
+// whole remainders, never a fingerprint.  Buckets fill in order, so a bucket
+// with a free entry ends a lookup.  A row that finds no entry within the
+// distance field's reach raises the overflow word and the caller takes the
+// radix path (the hash is that path's bits rotated, so rows of one radix
+// bucket spread over the table).
+//
+// The sums.  Up to DJ_SMALL groups: a block adds into shared memory (as many
+// copies of a group as fit, a lane its own, so a warp's lanes meet on no
+// address), flushed once into one of DJ_REPS copies in global memory.  More
+// groups: count and sum in one 64-bit word {count, sum}, one RED a row instead
+// of two.  That is exact or known not to be: with every value in [0, 2^s) (s
+// the sum's bits; any other raises a word) group g's word gives the count
+// C_g + floor(S_g / 2^s) modulo 2^(64 - s), so the counts add up to the matched
+// rows, counted by themselves, only if no sum left its field; a wrapped count
+// would need sums of 2^64 in all, which a bound on them (added up by
+// themselves too) excludes.  Where the check fails the call runs again with
+// two words a group.  Groups that a block meets often (skewed keys) go through
+// a cache in shared memory, so that they do not queue up on one address;
+// up to 64K groups have several copies of their sums, so that four groups'
+// words of a sector do not queue up (18M rows into 5000 groups: 488 -> 354 us).
+#include <algorithm>
+#include <climits>
+
+#include "common.cuh"
+
+namespace pf {
+namespace {
+
+constexpr int DT = 256;
+#ifndef PF_DJ_R
+#define PF_DJ_R 2
+#endif
+#ifndef PF_DJ_MINB
+#define PF_DJ_MINB 5
+#endif
+// probe rows a thread takes at a time, at five blocks a SM (48 registers):
+// 20M rows against 3M, 203 us; at six blocks (40, spills) 265, 1 row 208-222,
+// 3 rows 207, 4 rows 215-274
+constexpr int DR = PF_DJ_R;
+#ifndef PF_DJ_B
+#define PF_DJ_B 2
+#endif
+constexpr int DB = PF_DJ_B;                  // build rows a thread takes at a time
+constexpr int FG = 4;                  // groups a thread of k_dj_finish takes
+constexpr int FTILE = DT * FG;
+constexpr int DJ_SMALL = 2048;         // groups summed in shared memory
+constexpr int DJ_REPS = 8;             // global copies of their sums
+constexpr int DJ_SPREAD = 1 << 17;     // words that a few groups' sums are spread over
+constexpr int DJ_MAX_REPS = 32;
+constexpr int DJ_CACHE = 1024;         // cached groups a block
+constexpr int DJ_REPEATS = 16;         // of a block's first rows, for the cache
+constexpr unsigned long long DJ_EMPTY = ~0ULL;
+
+struct DjHead {
+  unsigned overflow;            // a build row found no entry
+  unsigned bad_value;           // packed sums: a value outside [0, 2^s)
+  unsigned gave_up;             // k_dj_finish: a wait on another tile ran out
+  unsigned ticket, done;        // its tiles taken and done
+  unsigned pad;
+  unsigned long long matched;
+  unsigned long long high;      // sum of value >> 20 over the matched rows
+  unsigned long long counts;    // the groups' counts added up
+  long long groups;             // occupied groups
+};
+
+struct DjArgs {
+  const long long* bkey;
+  const int* bgrp;
+  long long nb;
+  const long long* fk;
+  const long long* price;
+  const long long* disc;
+  long long scale, np;
+  unsigned long long* table;
+  int q, gbits, dbits;
+  long long gmin, G;
+  unsigned long long* slab;     // pairs (small, wide) or packed words
+  int sbits;                    // packed: bits of the sum
+  int reps;                     // copies of the sums, a block's own by its number
+  int copies;                   // small: copies of a group in shared memory, log2
+  unsigned long long* stats;
+  DjHead* head;
+  unsigned long long* tiles;    // k_dj_finish: each tile's state
+  int ntiles;
+};
+
+// Bijective; mix64's bits rotated (their top ones choose a radix bucket).
+__device__ __forceinline__ unsigned long long dj_hash(long long key) {
+  const unsigned long long h = mix64((uint64_t)key);
+  return h << 21 | h >> 43;
+}
+
+struct Bucket {
+  unsigned long long e[4];
+};
+__device__ __forceinline__ Bucket ld_bucket(const unsigned long long* p) {
+  Bucket b;
+  asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];"
+               : "=l"(b.e[0]), "=l"(b.e[1]), "=l"(b.e[2]), "=l"(b.e[3])
+               : "l"(p)
+               : "memory");
+  return b;
+}
+
+enum { SUM_SMALL, SUM_PACKED, SUM_WIDE };
+
+__global__ void __launch_bounds__(DT) k_dj_init(DjArgs a, long long slab_words) {
+  const long long t = (long long)blockIdx.x * DT + threadIdx.x, step = (long long)gridDim.x * DT;
+  const long long words = 4LL << a.q;
+  ulonglong2* tab = reinterpret_cast<ulonglong2*>(a.table);
+  for (long long i = t; i < words / 2; i += step) tab[i] = make_ulonglong2(DJ_EMPTY, DJ_EMPTY);
+  for (long long i = t; i < slab_words; i += step) a.slab[i] = 0;
+  for (long long i = t; i < a.ntiles; i += step) a.tiles[i] = 0;
+  if (t < 4) a.stats[t] = 0;
+  if (t == 0) *a.head = DjHead{};
+}
+
+// DB rows a thread, their buckets read together, then each row's claim of the
+// bucket's first free entry.  (Claims without the read first, from an entry
+// the hash picks, took 33 against 13 us for 250K rows: a failed claim costs a
+// round trip of its own.)
+__global__ void __launch_bounds__(DT) k_dj_build(DjArgs a) {
+  const unsigned none = (1u << a.gbits) - 2u;  // a group outside the range
+  const unsigned long long bmask = (1ULL << a.q) - 1;
+  const int reach = (1 << a.dbits) - 1;  // never a distance field of all ones
+  unsigned bad = 0;
+  const long long tile = (long long)DT * DB;
+  for (long long t0 = (long long)blockIdx.x * tile; t0 < a.nb; t0 += (long long)gridDim.x * tile) {
+    unsigned long long h[DB], e[DB];
+    Bucket k[DB];
+    bool live[DB];
+#pragma unroll
+    for (int r = 0; r < DB; ++r) {
+      const long long i = t0 + r * DT + threadIdx.x;
+      live[r] = i < a.nb;
+      h[r] = live[r] ? (unsigned long long)__ldcs(a.bkey + i) : 0ULL;
+      e[r] = live[r] ? (unsigned long long)(long long)__ldcs(a.bgrp + i) : 0ULL;
+    }
+#pragma unroll
+    for (int r = 0; r < DB; ++r) {
+      const long long g = (long long)e[r] - a.gmin;
+      const bool in = g >= 0 && g < a.G;
+      bad += live[r] && !in;
+      h[r] = dj_hash((long long)h[r]);
+      // remainder | distance | group
+      e[r] = (h[r] << a.q >> a.q) << (a.dbits + a.gbits) | (in ? (unsigned)g : none);
+      k[r] = ld_bucket(a.table + 4 * (h[r] >> (64 - a.q)));
+    }
+#pragma unroll
+    for (int r = 0; r < DB; ++r) {
+      if (!live[r]) continue;
+      bool done = false;
+      unsigned long long b = h[r] >> (64 - a.q), x = e[r];
+      for (int d = 0; d < reach && !done; ++d) {
+        const Bucket y = d ? ld_bucket(a.table + 4 * b) : k[r];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (!done && y.e[j] == DJ_EMPTY)
+            done = atomicCAS(a.table + 4 * b + j, DJ_EMPTY, x) == DJ_EMPTY;
+        b = (b + 1) & bmask;
+        x += 1ULL << a.gbits;
+      }
+      if (!done) a.head->overflow = 1;
+    }
+  }
+  for (int o = 16; o; o >>= 1) bad += __shfl_xor_sync(FULL, bad, o);
+  if ((threadIdx.x & 31) == 0 && bad) atomicAdd(&a.stats[2], (unsigned long long)bad);
+}
+
+// The group of a matched entry.
+__device__ __forceinline__ unsigned group_in(const DjArgs& a, unsigned long long e) {
+  return (unsigned)(e & ((1ULL << a.gbits) - 1));
+}
+
+// Hash h among a bucket's entries at distance d: its entry (DJ_EMPTY: none);
+// *more: the lookup goes on in the next bucket.
+__device__ __forceinline__ unsigned long long among(const DjArgs& a, const Bucket& k,
+                                                    unsigned long long want, bool* more) {
+  unsigned long long r = DJ_EMPTY;
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    if ((k.e[j] ^ want) >> a.gbits == 0) r = k.e[j];
+  // (a free entry's distance field is all ones, which no row's is)
+  *more = r == DJ_EMPTY && k.e[3] != DJ_EMPTY;
+  return r;
+}
+
+struct DjSmem {
+  // small: [G << copies] each, then the cache's arrays for packed
+  unsigned* lo;
+  unsigned* hi;
+  unsigned* cnt;
+};
+
+__device__ __forceinline__ void add_shared(unsigned* lo, unsigned* hi, unsigned* cnt, unsigned s,
+                                           long long v) {
+  const unsigned l = (unsigned)(unsigned long long)v, h = (unsigned)((unsigned long long)v >> 32);
+  const unsigned old = atomicAdd(&lo[s], l);
+  const unsigned hc = h + (old + l < old ? 1u : 0u);
+  if (hc) atomicAdd(&hi[s], hc);
+  atomicAdd(&cnt[s], 1u);
+}
+
+template <int MODE, bool DISC>
+__global__ void __launch_bounds__(DT, PF_DJ_MINB) k_dj_probe(DjArgs a) {
+  extern __shared__ __align__(16) unsigned dj_smem[];
+  if (a.head->overflow) return;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const unsigned none = (1u << a.gbits) - 2u;
+  const unsigned long long bmask = (1ULL << a.q) - 1;
+  const int cells = MODE == SUM_SMALL ? (int)a.G << a.copies : DJ_CACHE;
+  unsigned* lo = dj_smem;
+  unsigned* hi = lo + cells;
+  unsigned* cnt = hi + cells;
+  int* tag = reinterpret_cast<int*>(cnt + cells);  // the cache's groups
+  for (int i = tid; i < cells; i += DT) {
+    lo[i] = hi[i] = cnt[i] = 0;
+    if (MODE != SUM_SMALL) tag[i] = -1;
+  }
+  __syncthreads();
+  const unsigned copy = lane & ((1u << a.copies) - 1);
+  unsigned long long* slab = MODE == SUM_SMALL
+                                 ? nullptr
+                                 : a.slab + (unsigned long long)(blockIdx.x % a.reps) *
+                                                (unsigned long long)a.G *
+                                                (MODE == SUM_PACKED ? 1 : 2);
+  unsigned matched = 0;
+  unsigned long long high = 0;
+  bool outside = false, cached = false;
+  const long long tile = (long long)DT * DR, first = (long long)blockIdx.x * tile;
+  for (long long t0 = first; t0 < a.np; t0 += (long long)gridDim.x * tile) {
+    unsigned long long h[DR], want[DR];
+    long long v[DR];
+    Bucket k[DR];
+    bool live[DR];
+#pragma unroll
+    for (int r = 0; r < DR; ++r) {
+      const long long i = t0 + r * DT + tid;
+      live[r] = i < a.np;
+      h[r] = live[r] ? (unsigned long long)__ldcs(a.fk + i) : 0ULL;
+    }
+#pragma unroll
+    for (int r = 0; r < DR; ++r) {
+      const long long i = t0 + r * DT + tid;
+      v[r] = live[r] ? __ldcs(a.price + i) : 0;
+    }
+    if (DISC) {
+      long long d[DR];
+#pragma unroll
+      for (int r = 0; r < DR; ++r) {
+        const long long i = t0 + r * DT + tid;
+        d[r] = live[r] ? __ldcs(a.disc + i) : 0;
+      }
+#pragma unroll
+      for (int r = 0; r < DR; ++r)
+        v[r] = (long long)((unsigned long long)v[r] * (unsigned long long)(a.scale - d[r]));
+    }
+#pragma unroll
+    for (int r = 0; r < DR; ++r) {
+      h[r] = dj_hash((long long)h[r]);
+      want[r] = (h[r] << a.q >> a.q) << (a.dbits + a.gbits);
+      k[r] = ld_bucket(a.table + 4 * (h[r] >> (64 - a.q)));
+    }
+    int repeats = 0;
+#pragma unroll
+    for (int r = 0; r < DR; ++r) {
+      if (!live[r]) continue;
+      bool more;
+      unsigned long long e = among(a, k[r], want[r], &more);
+      if (more) {
+        unsigned long long b = h[r] >> (64 - a.q), w = want[r];
+        for (int d = 1; d < (1 << a.dbits) - 1 && more; ++d) {
+          b = (b + 1) & bmask;
+          w += 1ULL << a.gbits;
+          e = among(a, ld_bucket(a.table + 4 * b), w, &more);
+        }
+      }
+      if (e == DJ_EMPTY) continue;
+      const unsigned g = group_in(a, e);
+      ++matched;
+      if (g == none) continue;
+      if (MODE == SUM_SMALL) {
+        add_shared(lo, hi, cnt, g << a.copies | copy, v[r]);
+        continue;
+      }
+      if (MODE == SUM_PACKED) {
+        outside |= (unsigned long long)v[r] >> a.sbits != 0;
+        high += (unsigned long long)v[r] >> 20;
+      }
+      const unsigned s = (g * 0x9E3779B1u) >> 22;  // of DJ_CACHE = 1024
+      if (cached) {
+        int t = *(volatile int*)&tag[s];
+        if (t == -1) {
+          t = atomicCAS(&tag[s], -1, (int)g);
+          if (t == -1) t = (int)g;
+        }
+        if (t == (int)g) {
+          add_shared(lo, hi, cnt, s, v[r]);
+          continue;
+        }
+      } else if (t0 == first) {
+        // the block's first rows: how often a group comes again
+        repeats += *(volatile int*)&tag[s] == (int)g;
+        *(volatile int*)&tag[s] = (int)g;
+      }
+      if (MODE == SUM_PACKED) {
+        atomicAdd(&slab[g], (1ULL << a.sbits) + (unsigned long long)v[r]);
+      } else {
+        atomicAdd(&slab[2 * (unsigned long long)g], (unsigned long long)v[r]);
+        atomicAdd(&slab[2 * (unsigned long long)g + 1], 1ULL);
+      }
+    }
+    if (MODE != SUM_SMALL && t0 == first) {
+      cached = __syncthreads_count(repeats > 0) >= DJ_REPEATS;
+      for (int i = tid; i < cells; i += DT) tag[i] = -1;
+      __syncthreads();
+    }
+  }
+  __syncthreads();
+  if (MODE == SUM_SMALL) {
+    unsigned long long* rep = a.slab + 2ULL * (blockIdx.x % DJ_REPS) * (unsigned long long)a.G;
+    for (int g = tid; g < (int)a.G; g += DT) {
+      unsigned long long s = 0, c = 0;
+      for (int j = 0; j < 1 << a.copies; ++j) {
+        const int x = g << a.copies | ((j + tid) & ((1 << a.copies) - 1));
+        s += (unsigned long long)hi[x] << 32 | lo[x];
+        c += cnt[x];
+      }
+      if (c) {
+        atomicAdd(&rep[2 * g], s);
+        atomicAdd(&rep[2 * g + 1], c);
+      }
+    }
+  } else if (cached) {
+    for (int i = tid; i < cells; i += DT) {
+      const int g = tag[i];
+      if (g < 0) continue;
+      const unsigned long long s = (unsigned long long)hi[i] << 32 | lo[i], c = cnt[i];
+      if (MODE == SUM_PACKED) {
+        atomicAdd(&slab[g], (c << a.sbits) + s);
+      } else {
+        atomicAdd(&slab[2 * (unsigned long long)g], s);
+        atomicAdd(&slab[2 * (unsigned long long)g + 1], c);
+      }
+    }
+  }
+  // the block's counts, one atomic each
+  __shared__ unsigned long long red[2][DT / 32];
+  unsigned long long m = matched;
+  for (int o = 16; o; o >>= 1) {
+    m += __shfl_xor_sync(FULL, m, o);
+    if (MODE == SUM_PACKED) high += __shfl_xor_sync(FULL, high, o);
+  }
+  if (lane == 0) {
+    red[0][tid >> 5] = m;
+    red[1][tid >> 5] = high;
+  }
+  if (MODE == SUM_PACKED && outside) a.head->bad_value = 1;
+  __syncthreads();
+  if (tid == 0) {
+    for (int w = 1; w < DT / 32; ++w) {
+      m += red[0][w];
+      high += red[1][w];
+    }
+    if (m) atomicAdd(&a.stats[0], m);
+    if (MODE == SUM_PACKED) {
+      if (m) atomicAdd(&a.head->matched, m);
+      if (high) atomicAdd(&a.head->high, high);
+    }
+  }
+}
+
+struct DjOut {
+  long long* sum;     // [G] dense
+  long long* count;
+  long long* keys;    // occupied groups (null: not wanted)
+  long long* sums;
+  long long* counts;
+  DjHead* host;
+};
+
+// Up to DJ_SMALL groups: one block adds up the copies and compacts.
+__global__ void __launch_bounds__(1024) k_dj_finish_small(DjArgs a, DjOut o) {
+  __shared__ int wsum[32];
+  constexpr int PER = DJ_SMALL / 1024;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  unsigned long long s[PER], c[PER];
+  int mine = 0;
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {
+    const int g = tid * PER + k;
+    s[k] = c[k] = 0;
+    if (g >= a.G) continue;
+    ulonglong2 x[DJ_REPS];
+#pragma unroll
+    for (int r = 0; r < DJ_REPS; ++r)
+      x[r] = reinterpret_cast<const ulonglong2*>(a.slab)[(long long)r * a.G + g];
+#pragma unroll
+    for (int r = 0; r < DJ_REPS; ++r) {
+      s[k] += x[r].x;
+      c[k] += x[r].y;
+    }
+    o.sum[g] = (long long)s[k];
+    o.count[g] = (long long)c[k];
+    mine += c[k] > 0;
+  }
+  int incl = mine;
+  for (int d = 1; d < 32; d <<= 1) {
+    const int y = __shfl_up_sync(FULL, incl, d);
+    if (lane >= d) incl += y;
+  }
+  if (lane == 31) wsum[w] = incl;
+  __syncthreads();
+  int at = incl - mine, tot = 0;
+  for (int q = 0; q < 32; ++q) {
+    at += q < w ? wsum[q] : 0;
+    tot += wsum[q];
+  }
+  if (o.keys) {
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+      if (!c[k]) continue;
+      o.keys[at] = a.gmin + tid * PER + k;
+      o.sums[at] = (long long)s[k];
+      o.counts[at] = (long long)c[k];
+      ++at;
+    }
+  }
+  if (tid == 0) {
+    DjHead h = *a.head;
+    h.groups = tot;
+    *o.host = h;
+  }
+}
+
+// A tile's state: 0, or its occupied groups with TILE_OWN, or all groups' up
+// to its end with TILE_ALL.
+constexpr unsigned long long TILE_OWN = 1ULL << 62, TILE_ALL = 2ULL << 62,
+                             TILE_VALUE = (1ULL << 62) - 1;
+constexpr int DJ_POLLS = 1 << 22;
+
+__device__ __forceinline__ unsigned long long ld_state(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_state(unsigned long long* p, unsigned long long v) {
+  asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+// One pass over the groups, a tile of FTILE a block, its sums and counts held
+// in registers; a tile's first output is the sum of the tiles before it, looked
+// up 32 at a time from the nearest back (tiles are taken in order, so the ones
+// before are at work or done; a wait is bounded).  The last tile done tells the
+// host.
+template <bool PACKED>
+__global__ void __launch_bounds__(DT) k_dj_finish(DjArgs a, DjOut o) {
+  __shared__ int wsum[DT / 32];
+  __shared__ unsigned long long csum[DT / 32];
+  __shared__ int tile_s;
+  __shared__ long long before_s;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  if (tid == 0) tile_s = (int)atomicAdd(&a.head->ticket, 1u);
+  __syncthreads();
+  const int t = tile_s;
+  if (t >= a.ntiles) return;
+  const long long g0 = (long long)t * FTILE + (long long)tid * FG;
+  const unsigned long long smask = PACKED ? (1ULL << a.sbits) - 1 : 0;
+  unsigned long long s[FG], c[FG], total = 0;
+  int mine = 0;
+#pragma unroll
+  for (int k = 0; k < FG; ++k) {
+    s[k] = c[k] = 0;
+    if (g0 + k >= a.G) continue;
+    if (PACKED) {
+      s[k] = a.slab[g0 + k];
+    } else {
+      const ulonglong2 x = reinterpret_cast<const ulonglong2*>(a.slab)[g0 + k];
+      s[k] = x.x;
+      c[k] = x.y;
+    }
+  }
+  for (int r = 1; r < a.reps; ++r) {
+#pragma unroll
+    for (int k = 0; k < FG; ++k) {
+      if (g0 + k >= a.G) continue;
+      const long long at = (long long)r * a.G + g0 + k;
+      if (PACKED) {
+        s[k] += a.slab[at];
+      } else {
+        const ulonglong2 x = reinterpret_cast<const ulonglong2*>(a.slab)[at];
+        s[k] += x.x;
+        c[k] += x.y;
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < FG; ++k) {
+    if (!PACKED) break;
+    c[k] = s[k] >> a.sbits;
+    s[k] &= smask;
+  }
+#pragma unroll
+  for (int k = 0; k < FG; ++k) {
+    if (g0 + k >= a.G) continue;
+    total += c[k];
+    mine += c[k] > 0;
+    o.sum[g0 + k] = (long long)s[k];
+    o.count[g0 + k] = (long long)c[k];
+  }
+  int incl = mine;
+  for (int d = 1; d < 32; d <<= 1) {
+    const int y = __shfl_up_sync(FULL, incl, d);
+    if (lane >= d) incl += y;
+  }
+  if (PACKED)
+    for (int d = 16; d; d >>= 1) total += __shfl_xor_sync(FULL, total, d);
+  if (lane == 31) wsum[w] = incl;
+  if (lane == 0) csum[w] = total;
+  __syncthreads();
+  int at = incl - mine, tot = 0;
+#pragma unroll
+  for (int q = 0; q < DT / 32; ++q) {
+    at += q < w ? wsum[q] : 0;
+    tot += wsum[q];
+  }
+  if (w == 0) {
+    long long before = 0;
+    if (lane == 0 && t > 0) st_state(&a.tiles[t], TILE_OWN | (unsigned long long)tot);
+    bool ok = true;
+    for (int end = t; end > 0 && ok;) {
+      const int q = end - 1 - lane;  // lane 0 the nearest
+      unsigned long long x = q >= 0 ? 0 : TILE_ALL;
+      for (int polls = 0; q >= 0 && polls < DJ_POLLS; ++polls) {
+        x = ld_state(&a.tiles[q]);
+        if (x) break;
+      }
+      ok = __all_sync(FULL, x != 0);
+      const unsigned all = __ballot_sync(FULL, (x & TILE_ALL) != 0);
+      const int stop = all ? __ffs(all) - 1 : 31;
+      long long add = lane <= stop ? (long long)(x & TILE_VALUE) : 0;
+      for (int d = 16; d; d >>= 1) add += __shfl_xor_sync(FULL, add, d);
+      before += add;
+      if (all) break;
+      end -= 32;
+    }
+    if (lane == 0) {
+      if (!ok) a.head->gave_up = 1;
+      st_state(&a.tiles[t], TILE_ALL | (unsigned long long)(before + tot));
+      before_s = before;
+      if (PACKED) {
+        for (int q = 1; q < DT / 32; ++q) total += csum[q];
+        if (total) atomicAdd(&a.head->counts, total);
+      }
+    }
+  }
+  __syncthreads();
+  long long j = before_s + at;
+  if (o.keys) {
+#pragma unroll
+    for (int k = 0; k < FG; ++k) {
+      if (!c[k]) continue;
+      o.keys[j] = a.gmin + g0 + k;
+      o.sums[j] = (long long)s[k];
+      o.counts[j] = (long long)c[k];
+      ++j;
+    }
+  }
+  if (tid != 0) return;
+  if (t == a.ntiles - 1) a.head->groups = before_s + tot;
+  __threadfence();
+  if (atomicAdd(&a.head->done, 1u) == (unsigned)a.ntiles - 1) {
+    __threadfence();
+    volatile DjHead* h = a.head;
+    o.host->overflow = h->overflow;
+    o.host->bad_value = h->bad_value;
+    o.host->gave_up = h->gave_up;
+    o.host->matched = h->matched;
+    o.host->high = h->high;
+    o.host->counts = h->counts;
+    o.host->groups = h->groups;
+  }
+}
+
+struct DjLayout {
+  DjHead* head;
+  unsigned long long* table;
+  unsigned long long* slab;
+  unsigned long long* tiles;
+  int q, gbits, dbits, ntiles, reps;
+};
+
+int bits_of(unsigned long long x) { return x ? 64 - __builtin_clzll(x) : 0; }
+
+// The table's bits for nb build rows and groups of g bits, or q = 0.
+//
+// How full it may be: a lookup that leaves its home bucket holds up its warp
+// for a round trip, so a table 0.72 full (a bucket in three full) took 553 us
+// for 3M x 18M rows where one of 0.36 takes 306. At most 0.3, or 0.4 from 64
+// MiB on, where the next size up leaves L2 (3M rows in 128 MiB 351).
+// How large: up to 128 MiB, a little over L2. Against the radix path, 8 M x 40M
+// and more rows lose (9M x 45M in 256 MiB 1.33 against 1.14 ms); 5.9M x 47M
+// rows take 1.02 against 1.08, 4.5M x 13.5M 0.42 against 0.50, 1M x 5M 0.15
+// against 0.29, 250K x 1M 0.07 against 0.17 to 0.35.
+// The entry: remainder, distance and group in 64 bits, at least 3 bits of
+// distance (a table that empty has no run of seven full buckets).
+constexpr int DJ_MAX_Q = 22;
+constexpr double DJ_LOAD = 0.3, DJ_LOAD_TOP = 0.4;
+void dj_table(long long nb, long long G, int* q, int* gbits, int* dbits) {
+  *gbits = bits_of((unsigned long long)G + 1);  // all ones and all ones but one are no group
+  for (*q = 6; *q <= DJ_MAX_Q; ++*q) {
+    const double load = (double)nb / (double)(4LL << *q);
+    const int room = *q - *gbits;
+    if (load <= (*q < DJ_MAX_Q - 1 ? DJ_LOAD : DJ_LOAD_TOP) && room >= 3) {
+      *dbits = std::min(room, 6);
+      return;
+    }
+  }
+  *q = 0;
+}
+
+DjLayout dj_layout(Arena& a, long long nb, long long G) {
+  DjLayout l{};
+  dj_table(nb, G, &l.q, &l.gbits, &l.dbits);
+  l.head = a.take<DjHead>(1);
+  l.table = a.take<unsigned long long>(l.q ? (size_t)4 << l.q : 1);
+  l.reps = G <= DJ_SMALL ? DJ_REPS
+                         : (int)std::max<long long>(1, std::min<long long>(DJ_MAX_REPS, DJ_SPREAD / G));
+  const long long words = 2LL * l.reps * G;
+  l.slab = a.take<unsigned long long>((size_t)std::max<long long>(words, 1));
+  l.ntiles = G <= DJ_SMALL ? 0 : (int)((G + FTILE - 1) / FTILE);
+  l.tiles = a.take<unsigned long long>((size_t)l.ntiles + 1);
+  return l;
+}
+
+DjHead* pinned_dj_head() {
+  thread_local DjHead* buf = nullptr;
+  if (!buf && cudaHostAlloc((void**)&buf, sizeof(DjHead),
+                            cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+    cudaGetLastError();
+    buf = nullptr;
+  }
+  return buf;
+}
+
+template <int MODE>
+int dj_probe(const DjArgs& a, cudaStream_t st) {
+  const size_t smem = MODE == SUM_SMALL ? (size_t)3 * 4 * (a.G << a.copies) : 4 * 4 * DJ_CACHE;
+  auto kern = a.disc ? k_dj_probe<MODE, true> : k_dj_probe<MODE, false>;
+  if (int rc = opt_in_smem((const void*)kern, smem)) return rc;
+  int per_sm = 0;
+  PF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, DT, smem));
+  const unsigned g = (unsigned)std::max<long long>(
+      1, std::min<long long>((a.np + DT * DR - 1) / (DT * DR),
+                             (long long)sm_count() * std::max(1, per_sm)));
+  {
+    PF_KERNEL("k_dj_probe", st);
+    kern<<<g, DT, smem, st>>>(a);
+  }
+  PF_LAUNCH("k_dj_probe");
+  return PF_OK;
+}
+
+}  // namespace
+}  // namespace pf
+
+using namespace pf;
+
+extern "C" int pf_join_direct_fits(int64_t n_build, int64_t n_probe, int64_t n_groups) {
+  if (n_build < 1 || n_probe < 1 || n_groups < 1 || n_groups > (1 << 28)) return 0;
+  int q, gbits, dbits;
+  dj_table(n_build, n_groups, &q, &gbits, &dbits);
+  return q > 0;
+}
+
+extern "C" size_t pf_join_direct_workspace(int64_t n_build, int64_t n_groups) {
+  Arena a(nullptr, 0);
+  dj_layout(a, n_build, n_groups);
+  return a.used + 256;
+}
+
+extern "C" int pf_join_direct(const int64_t* build_key, const int32_t* build_group,
+                              int64_t n_build, const int64_t* probe_fk,
+                              const int64_t* probe_price, const int64_t* probe_disc,
+                              int64_t scale, int64_t n_probe, int64_t group_min,
+                              int64_t n_groups, int64_t* sum_out, int64_t* count_out,
+                              int64_t* stats_out, int64_t* keys_out, int64_t* sums_out,
+                              int64_t* counts_out, int64_t* n_out, int* done, void* workspace,
+                              size_t workspace_bytes, void* stream) {
+  cudaStream_t st = (cudaStream_t)stream;
+  if (!pf_join_direct_fits(n_build, n_probe, n_groups))
+    return fail(PF_EINVAL, "join_direct: %lld build rows and %lld groups do not fit its table",
+                (long long)n_build, (long long)n_groups);
+  if (n_probe >= (1LL << 40)) return fail(PF_EINVAL, "join_direct: at most 2^40 probe rows");
+  if (!build_key || !build_group || !probe_fk || !probe_price || !sum_out || !count_out ||
+      !stats_out || !done || (keys_out && (!sums_out || !counts_out || !n_out)))
+    return fail(PF_EINVAL, "join_direct: null pointer");
+  Arena ar(workspace, workspace_bytes);
+  const DjLayout l = dj_layout(ar, n_build, n_groups);
+  if (!workspace || !ar.fits())
+    return fail(PF_ENOSPACE, "join_direct: workspace of %zu bytes, %zu needed", workspace_bytes,
+                ar.used);
+  DjHead* host = pinned_dj_head();
+  DjHead* host_dev = nullptr;
+  if (!host) return fail(PF_ECUDA, "join_direct: no pinned result words");
+  if (int rc = host_alias(host, (void**)&host_dev)) return rc;
+  DjArgs a{};
+  a.bkey = (const long long*)build_key;
+  a.bgrp = build_group;
+  a.nb = n_build;
+  a.fk = (const long long*)probe_fk;
+  a.price = (const long long*)probe_price;
+  a.disc = (const long long*)probe_disc;
+  a.scale = scale;
+  a.np = n_probe;
+  a.table = l.table;
+  a.q = l.q;
+  a.gbits = l.gbits;
+  a.dbits = l.dbits;
+  a.gmin = group_min;
+  a.G = n_groups;
+  a.slab = l.slab;
+  a.stats = (unsigned long long*)stats_out;
+  a.head = l.head;
+  a.tiles = l.tiles;
+  a.ntiles = l.ntiles;
+  a.reps = l.reps;
+  const bool small = n_groups <= DJ_SMALL;
+  // packed: the count's field for 16 times the mean rows a group (or for all
+  // rows), where that leaves a mean group's sum 31 bits a value: else the check
+  // would fail on ordinary values, and the call run twice
+  const int mean = bits_of((unsigned long long)(n_probe / n_groups));
+  a.sbits = 64 - std::min(bits_of((unsigned long long)n_probe), mean + 4);
+  const bool pack = a.sbits - mean >= 31;
+  while (a.copies < 5 && (n_groups << (a.copies + 1)) <= DJ_SMALL) ++a.copies;
+  DjOut o{(long long*)sum_out, (long long*)count_out, (long long*)keys_out, (long long*)sums_out,
+          (long long*)counts_out, host_dev};
+  const int sms = sm_count();
+  *done = 0;
+  for (int attempt = small || pack ? 0 : 1; attempt < 2; ++attempt) {
+    const bool packed = !small && attempt == 0;
+    const long long words = (packed ? 1LL : 2LL) * l.reps * n_groups;
+    {
+      const long long work = (4LL << a.q) / 2 + words;
+      PF_KERNEL("k_dj_init", st);
+      k_dj_init<<<(unsigned)std::max<long long>(
+                      1, std::min<long long>((work + DT * 4 - 1) / (DT * 4), sms * 8LL)),
+                  DT, 0, st>>>(a, words);
+    }
+    PF_LAUNCH("k_dj_init");
+    {
+      PF_KERNEL("k_dj_build", st);
+      k_dj_build<<<(unsigned)std::min<long long>((n_build + DT * DB - 1) / (DT * DB), sms * 8LL),
+                   DT, 0, st>>>(a);
+    }
+    PF_LAUNCH("k_dj_build");
+    if (int rc = small    ? dj_probe<SUM_SMALL>(a, st)
+                 : packed ? dj_probe<SUM_PACKED>(a, st)
+                          : dj_probe<SUM_WIDE>(a, st))
+      return rc;
+    {
+      PF_KERNEL("k_dj_finish", st);
+      if (small) k_dj_finish_small<<<1, 1024, 0, st>>>(a, o);
+      else if (packed) k_dj_finish<true><<<a.ntiles, DT, 0, st>>>(a, o);
+      else k_dj_finish<false><<<a.ntiles, DT, 0, st>>>(a, o);
+    }
+    PF_LAUNCH("k_dj_finish");
+    if (int rc = wait_stream(st)) return rc;
+    if (host->gave_up) return fail(PF_EDEVICE, "join_direct: a device wait gave up");
+    if (host->overflow) return ok();  // *done = 0
+    if (!packed || (!host->bad_value && host->counts == host->matched &&
+                    host->high + host->matched < 1ULL << 43)) {
+      *done = 1;
+      if (n_out) *n_out = host->groups;
+      return ok();
+    }
+  }
+  return ok();
+}

@@ -3,7 +3,9 @@ passes of both sides into sub-partitions, a shared-memory hash table per
 sub-partition, probe rows aggregated into their build row's cell and each
 build row flushed once into a dense group slab, then the occupied groups
 compacted.  The fan-out and the join's table are picked by the autotuner
-(pageflow_b200.autotune) unless given.
+(pageflow_b200.autotune) unless given.  A build whose hash table fits L2 is
+joined without a radix pass (pf_join_direct) unless a fan-out, knobs or an
+override asks for the radix path.
 
     keys, sums, counts = join_group_aggregate(build_key, build_group,
                                               probe_fk, price, disc)
@@ -59,10 +61,12 @@ class JoinAggregate:
         self.device = torch.device(device)
         L = N.lib()
         self.knobs = None if knobs is None else N.JoinKnobs(**knobs)
+        # the environment's overrides (sweeps, tests) fix the configuration
+        free = B is None and knobs is None and not any(os.environ.get(v) for v in _OVERRIDES)
         if autotune is None:
-            # the environment's overrides (sweeps, tests) fix the configuration
-            autotune = B is None and knobs is None and not any(
-                os.environ.get(v) for v in _OVERRIDES)
+            autotune = free
+        self.direct = free and bool(L.pf_join_direct_fits(self.n_build, self.n_probe,
+                                                          self.n_groups))
         self.autotune = bool(autotune)
         self.tuning = None          # the autotuner's Result once it has run
         self.B = int(B) if B else int(L.pf_join_aggregate_pick_b(self.n_build, self.n_probe))
@@ -87,6 +91,8 @@ class JoinAggregate:
 
     def _reserve(self, need: Optional[int] = None) -> None:
         need = self._ws_for(self.B, self.knobs) if need is None else need
+        if self.direct:
+            need = max(need, int(N.lib().pf_join_direct_workspace(self.n_build, self.n_groups)))
         if self.ws is None or self.ws_bytes < need:
             self.ws = None
             self.ws = N.workspace(need, self.device)
@@ -135,10 +141,29 @@ class JoinAggregate:
         self._reserve()
         self.autotune = False
 
+    def _launch_direct(self, args, finish: bool):
+        """The join without a radix pass, and with ``finish`` the occupied
+        groups' number; None when the build keys crowd its table."""
+        build_key, build_group, probe_fk, probe_price, probe_disc = args
+        n, done = ctypes.c_int64(), ctypes.c_int()
+        with torch.cuda.device(self.device):
+            rc = N.lib().pf_join_direct(
+                build_key.data_ptr(), build_group.data_ptr(), self.n_build, probe_fk.data_ptr(),
+                probe_price.data_ptr(), N.ptr(probe_disc), self.scale, self.n_probe,
+                self.group_min, self.n_groups, self.sum.data_ptr(), self.count.data_ptr(),
+                self.stats.data_ptr(), self.keys_out.data_ptr() if finish else None,
+                self.sums_out.data_ptr(), self.counts_out.data_ptr(), ctypes.byref(n),
+                ctypes.byref(done), self.ws.data_ptr(), self.ws_bytes, N.stream_of(self.device))
+        N.check(rc, "join_direct")
+        return n.value if done.value else None
+
     def aggregate(self, build_key, build_group, probe_fk, probe_price, probe_disc=None):
         """Queues the join + dense aggregation into ``self.sum`` /
         ``self.count`` (waits once, at the end, for the radix passes'
         overflow words; again only after an overflow)."""
+        self._aggregate(build_key, build_group, probe_fk, probe_price, probe_disc, False)
+
+    def _aggregate(self, build_key, build_group, probe_fk, probe_price, probe_disc, finish):
         for t, n, dt, name in ((build_key, self.n_build, torch.int64, "build_key"),
                                (build_group, self.n_build, torch.int32, "build_group"),
                                (probe_fk, self.n_probe, torch.int64, "probe_fk"),
@@ -153,7 +178,12 @@ class JoinAggregate:
         args = (build_key, build_group, probe_fk, probe_price, probe_disc)
         if self.autotune:
             self._tune(args)
+        if self.direct:
+            n = self._launch_direct(args, finish)
+            if n is not None:
+                return n
         self._launch(self.B, self.knobs, args)
+        return None
 
     def finish(self):
         """The occupied groups, ascending: (keys, sums, counts)."""
@@ -169,8 +199,10 @@ class JoinAggregate:
         return self.keys_out[:n], self.sums_out[:n], self.counts_out[:n]
 
     def run(self, build_key, build_group, probe_fk, probe_price, probe_disc=None):
-        self.aggregate(build_key, build_group, probe_fk, probe_price, probe_disc)
-        return self.finish()
+        n = self._aggregate(build_key, build_group, probe_fk, probe_price, probe_disc, True)
+        if n is None:
+            return self.finish()
+        return self.keys_out[:n], self.sums_out[:n], self.counts_out[:n]
 
     def run_stream(self, batches):
         """Joins a sequence of host-resident batches of this plan's shape,
