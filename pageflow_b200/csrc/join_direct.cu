@@ -14,15 +14,8 @@
 // and one RED.  What bounds it: L2's rate of requests (about 0.2 T/s reached
 // for a random read and a RED a row; the figures are at dj_table).
 //
-// The table.  2^q buckets of four 8-byte entries, a bucket one sector.  A key's
-// hash is a bijection of it, so its top q bits (the home bucket) and the 64 - q
-// others (the remainder, held in the entry) are the key itself.  An entry is
-// {remainder, distance of its bucket from home, group}; a lookup compares
-// whole remainders, never a fingerprint.  Buckets fill in order, so a bucket
-// with a free entry ends a lookup.  A row that finds no entry within the
-// distance field's reach raises the overflow word and the caller takes the
-// radix path (the hash is that path's bits rotated, so rows of one radix
-// bucket spread over the table).
+// The table is compact.cuh's; a build whose hashes crowd it raises the overflow
+// word and the caller takes the radix path.
 //
 // The sums.  Up to DJ_SMALL groups: a block adds into shared memory (as many
 // copies of a group as fit, a lane its own, so a warp's lanes meet on no
@@ -41,7 +34,7 @@
 #include <algorithm>
 #include <climits>
 
-#include "common.cuh"
+#include "compact.cuh"
 
 namespace pf {
 namespace {
@@ -57,10 +50,6 @@ constexpr int DT = 256;
 // 20M rows against 3M, 203 us; at six blocks (40, spills) 265, 1 row 208-222,
 // 3 rows 207, 4 rows 215-274
 constexpr int DR = PF_DJ_R;
-#ifndef PF_DJ_B
-#define PF_DJ_B 2
-#endif
-constexpr int DB = PF_DJ_B;                  // build rows a thread takes at a time
 constexpr int FG = 4;                  // groups a thread of k_dj_finish takes
 constexpr int FTILE = DT * FG;
 constexpr int DJ_SMALL = 2048;         // groups summed in shared memory
@@ -69,7 +58,6 @@ constexpr int DJ_SPREAD = 1 << 17;     // words that a few groups' sums are spre
 constexpr int DJ_MAX_REPS = 32;
 constexpr int DJ_CACHE = 1024;         // cached groups a block
 constexpr int DJ_REPEATS = 16;         // of a block's first rows, for the cache
-constexpr unsigned long long DJ_EMPTY = ~0ULL;
 
 struct DjHead {
   unsigned overflow;            // a build row found no entry
@@ -91,8 +79,7 @@ struct DjArgs {
   const long long* price;
   const long long* disc;
   long long scale, np;
-  unsigned long long* table;
-  int q, gbits, dbits;
+  CompactTable table;
   long long gmin, G;
   unsigned long long* slab;     // pairs (small, wide) or packed words
   int sbits;                    // packed: bits of the sum
@@ -104,113 +91,33 @@ struct DjArgs {
   int ntiles;
 };
 
-// Bijective; mix64's bits rotated (their top ones choose a radix bucket).
-__device__ __forceinline__ unsigned long long dj_hash(long long key) {
-  const unsigned long long h = mix64((uint64_t)key);
-  return h << 21 | h >> 43;
-}
-
-struct Bucket {
-  unsigned long long e[4];
-};
-__device__ __forceinline__ Bucket ld_bucket(const unsigned long long* p) {
-  Bucket b;
-  asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];"
-               : "=l"(b.e[0]), "=l"(b.e[1]), "=l"(b.e[2]), "=l"(b.e[3])
-               : "l"(p)
-               : "memory");
-  return b;
-}
-
 enum { SUM_SMALL, SUM_PACKED, SUM_WIDE };
 
 __global__ void __launch_bounds__(DT) k_dj_init(DjArgs a, long long slab_words) {
   const long long t = (long long)blockIdx.x * DT + threadIdx.x, step = (long long)gridDim.x * DT;
-  const long long words = 4LL << a.q;
-  ulonglong2* tab = reinterpret_cast<ulonglong2*>(a.table);
-  for (long long i = t; i < words / 2; i += step) tab[i] = make_ulonglong2(DJ_EMPTY, DJ_EMPTY);
+  const long long words = 4LL << a.table.q;
+  ulonglong2* tab = reinterpret_cast<ulonglong2*>(a.table.e);
+  for (long long i = t; i < words / 2; i += step) tab[i] = make_ulonglong2(CT_EMPTY, CT_EMPTY);
   for (long long i = t; i < slab_words; i += step) a.slab[i] = 0;
   for (long long i = t; i < a.ntiles; i += step) a.tiles[i] = 0;
   if (t < 4) a.stats[t] = 0;
   if (t == 0) *a.head = DjHead{};
 }
 
-// DB rows a thread, their buckets read together, then each row's claim of the
-// bucket's first free entry.  (Claims without the read first, from an entry
-// the hash picks, took 33 against 13 us for 250K rows: a failed claim costs a
-// round trip of its own.)
+// (3M rows 55 us; 86 with the bucket read before the claim. Two or four rows a
+// thread claiming together measured no faster.)
 __global__ void __launch_bounds__(DT) k_dj_build(DjArgs a) {
-  const unsigned none = (1u << a.gbits) - 2u;  // a group outside the range
-  const unsigned long long bmask = (1ULL << a.q) - 1;
-  const int reach = (1 << a.dbits) - 1;  // never a distance field of all ones
   unsigned bad = 0;
-  const long long tile = (long long)DT * DB;
-  for (long long t0 = (long long)blockIdx.x * tile; t0 < a.nb; t0 += (long long)gridDim.x * tile) {
-    unsigned long long h[DB], e[DB];
-    Bucket k[DB];
-    bool live[DB];
-#pragma unroll
-    for (int r = 0; r < DB; ++r) {
-      const long long i = t0 + r * DT + threadIdx.x;
-      live[r] = i < a.nb;
-      h[r] = live[r] ? (unsigned long long)__ldcs(a.bkey + i) : 0ULL;
-      e[r] = live[r] ? (unsigned long long)(long long)__ldcs(a.bgrp + i) : 0ULL;
-    }
-#pragma unroll
-    for (int r = 0; r < DB; ++r) {
-      const long long g = (long long)e[r] - a.gmin;
-      const bool in = g >= 0 && g < a.G;
-      bad += live[r] && !in;
-      h[r] = dj_hash((long long)h[r]);
-      // remainder | distance | group
-      e[r] = (h[r] << a.q >> a.q) << (a.dbits + a.gbits) | (in ? (unsigned)g : none);
-      k[r] = ld_bucket(a.table + 4 * (h[r] >> (64 - a.q)));
-    }
-#pragma unroll
-    for (int r = 0; r < DB; ++r) {
-      if (!live[r]) continue;
-      bool done = false;
-      unsigned long long b = h[r] >> (64 - a.q), x = e[r];
-      for (int d = 0; d < reach && !done; ++d) {
-        const Bucket y = d ? ld_bucket(a.table + 4 * b) : k[r];
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (!done && y.e[j] == DJ_EMPTY)
-            done = atomicCAS(a.table + 4 * b + j, DJ_EMPTY, x) == DJ_EMPTY;
-        b = (b + 1) & bmask;
-        x += 1ULL << a.gbits;
-      }
-      if (!done) a.head->overflow = 1;
-    }
+  for (long long i = (long long)blockIdx.x * DT + threadIdx.x; i < a.nb;
+       i += (long long)gridDim.x * DT) {
+    const long long key = __ldcs(a.bkey + i), g = (long long)__ldcs(a.bgrp + i) - a.gmin;
+    const bool in = g >= 0 && g < a.G;
+    bad += !in;
+    if (!ct_insert(a.table, key, in ? g : -1)) a.head->overflow = 1;
   }
   for (int o = 16; o; o >>= 1) bad += __shfl_xor_sync(FULL, bad, o);
   if ((threadIdx.x & 31) == 0 && bad) atomicAdd(&a.stats[2], (unsigned long long)bad);
 }
-
-// The group of a matched entry.
-__device__ __forceinline__ unsigned group_in(const DjArgs& a, unsigned long long e) {
-  return (unsigned)(e & ((1ULL << a.gbits) - 1));
-}
-
-// Hash h among a bucket's entries at distance d: its entry (DJ_EMPTY: none);
-// *more: the lookup goes on in the next bucket.
-__device__ __forceinline__ unsigned long long among(const DjArgs& a, const Bucket& k,
-                                                    unsigned long long want, bool* more) {
-  unsigned long long r = DJ_EMPTY;
-#pragma unroll
-  for (int j = 0; j < 4; ++j)
-    if ((k.e[j] ^ want) >> a.gbits == 0) r = k.e[j];
-  // (a free entry's distance field is all ones, which no row's is)
-  *more = r == DJ_EMPTY && k.e[3] != DJ_EMPTY;
-  return r;
-}
-
-struct DjSmem {
-  // small: [G << copies] each, then the cache's arrays for packed
-  unsigned* lo;
-  unsigned* hi;
-  unsigned* cnt;
-};
 
 __device__ __forceinline__ void add_shared(unsigned* lo, unsigned* hi, unsigned* cnt, unsigned s,
                                            long long v) {
@@ -226,8 +133,6 @@ __global__ void __launch_bounds__(DT, PF_DJ_MINB) k_dj_probe(DjArgs a) {
   extern __shared__ __align__(16) unsigned dj_smem[];
   if (a.head->overflow) return;
   const int tid = threadIdx.x, lane = tid & 31;
-  const unsigned none = (1u << a.gbits) - 2u;
-  const unsigned long long bmask = (1ULL << a.q) - 1;
   const int cells = MODE == SUM_SMALL ? (int)a.G << a.copies : DJ_CACHE;
   unsigned* lo = dj_smem;
   unsigned* hi = lo + cells;
@@ -251,7 +156,7 @@ __global__ void __launch_bounds__(DT, PF_DJ_MINB) k_dj_probe(DjArgs a) {
   for (long long t0 = first; t0 < a.np; t0 += (long long)gridDim.x * tile) {
     unsigned long long h[DR], want[DR];
     long long v[DR];
-    Bucket k[DR];
+    CtBucket k[DR];
     bool live[DR];
 #pragma unroll
     for (int r = 0; r < DR; ++r) {
@@ -277,28 +182,22 @@ __global__ void __launch_bounds__(DT, PF_DJ_MINB) k_dj_probe(DjArgs a) {
     }
 #pragma unroll
     for (int r = 0; r < DR; ++r) {
-      h[r] = dj_hash((long long)h[r]);
-      want[r] = (h[r] << a.q >> a.q) << (a.dbits + a.gbits);
-      k[r] = ld_bucket(a.table + 4 * (h[r] >> (64 - a.q)));
+      h[r] = ct_hash((long long)h[r]);
+      want[r] = ct_want(a.table, h[r]);
+      k[r] = ct_load(ct_home(a.table, h[r]));
     }
     int repeats = 0;
 #pragma unroll
     for (int r = 0; r < DR; ++r) {
       if (!live[r]) continue;
       bool more;
-      unsigned long long e = among(a, k[r], want[r], &more);
-      if (more) {
-        unsigned long long b = h[r] >> (64 - a.q), w = want[r];
-        for (int d = 1; d < (1 << a.dbits) - 1 && more; ++d) {
-          b = (b + 1) & bmask;
-          w += 1ULL << a.gbits;
-          e = among(a, ld_bucket(a.table + 4 * b), w, &more);
-        }
-      }
-      if (e == DJ_EMPTY) continue;
-      const unsigned g = group_in(a, e);
+      unsigned long long e = ct_among(a.table, k[r], want[r], &more);
+      if (more) e = ct_walk(a.table, h[r], want[r]);
+      if (e == CT_EMPTY) continue;
+      const long long grp = ct_group(a.table, e);
       ++matched;
-      if (g == none) continue;
+      if (grp < 0) continue;
+      const unsigned g = (unsigned)grp;
       if (MODE == SUM_SMALL) {
         add_shared(lo, hi, cnt, g << a.copies | copy, v[r]);
         continue;
@@ -610,33 +509,18 @@ struct DjLayout {
   int q, gbits, dbits, ntiles, reps;
 };
 
-int bits_of(unsigned long long x) { return x ? 64 - __builtin_clzll(x) : 0; }
-
 // The table's bits for nb build rows and groups of g bits, or q = 0.
 //
-// How full it may be: a lookup that leaves its home bucket holds up its warp
-// for a round trip, so a table 0.72 full (a bucket in three full) took 553 us
-// for 3M x 18M rows where one of 0.36 takes 306. At most 0.3, or 0.4 from 64
-// MiB on, where the next size up leaves L2 (3M rows in 128 MiB 351).
+// At most 0.3 full, or 0.4 from 64 MiB on, where the next size up leaves L2
+// (3M x 18M rows: 306 us in 64 MiB, 351 in 128).
 // How large: up to 128 MiB, a little over L2. Against the radix path, 8 M x 40M
 // and more rows lose (9M x 45M in 256 MiB 1.33 against 1.14 ms); 5.9M x 47M
 // rows take 1.02 against 1.08, 4.5M x 13.5M 0.42 against 0.50, 1M x 5M 0.15
 // against 0.29, 250K x 1M 0.07 against 0.17 to 0.35.
-// The entry: remainder, distance and group in 64 bits, at least 3 bits of
-// distance (a table that empty has no run of seven full buckets).
 constexpr int DJ_MAX_Q = 22;
 constexpr double DJ_LOAD = 0.3, DJ_LOAD_TOP = 0.4;
 void dj_table(long long nb, long long G, int* q, int* gbits, int* dbits) {
-  *gbits = bits_of((unsigned long long)G + 1);  // all ones and all ones but one are no group
-  for (*q = 6; *q <= DJ_MAX_Q; ++*q) {
-    const double load = (double)nb / (double)(4LL << *q);
-    const int room = *q - *gbits;
-    if (load <= (*q < DJ_MAX_Q - 1 ? DJ_LOAD : DJ_LOAD_TOP) && room >= 3) {
-      *dbits = std::min(room, 6);
-      return;
-    }
-  }
-  *q = 0;
+  ct_size(nb, G, DJ_MAX_Q, DJ_LOAD, DJ_LOAD_TOP, q, gbits, dbits);
 }
 
 DjLayout dj_layout(Arena& a, long long nb, long long G) {
@@ -733,10 +617,7 @@ extern "C" int pf_join_direct(const int64_t* build_key, const int32_t* build_gro
   a.disc = (const long long*)probe_disc;
   a.scale = scale;
   a.np = n_probe;
-  a.table = l.table;
-  a.q = l.q;
-  a.gbits = l.gbits;
-  a.dbits = l.dbits;
+  a.table = CompactTable{l.table, l.q, l.gbits, l.dbits};
   a.gmin = group_min;
   a.G = n_groups;
   a.slab = l.slab;
@@ -761,7 +642,7 @@ extern "C" int pf_join_direct(const int64_t* build_key, const int32_t* build_gro
     const bool packed = !small && attempt == 0;
     const long long words = (packed ? 1LL : 2LL) * l.reps * n_groups;
     {
-      const long long work = (4LL << a.q) / 2 + words;
+      const long long work = (4LL << a.table.q) / 2 + words;
       PF_KERNEL("k_dj_init", st);
       k_dj_init<<<(unsigned)std::max<long long>(
                       1, std::min<long long>((work + DT * 4 - 1) / (DT * 4), sms * 8LL)),
@@ -770,7 +651,7 @@ extern "C" int pf_join_direct(const int64_t* build_key, const int32_t* build_gro
     PF_LAUNCH("k_dj_init");
     {
       PF_KERNEL("k_dj_build", st);
-      k_dj_build<<<(unsigned)std::min<long long>((n_build + DT * DB - 1) / (DT * DB), sms * 8LL),
+      k_dj_build<<<(unsigned)std::min<long long>((n_build + DT - 1) / DT, sms * 8LL),
                    DT, 0, st>>>(a);
     }
     PF_LAUNCH("k_dj_build");
