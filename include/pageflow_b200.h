@@ -631,18 +631,19 @@ typedef struct {
 } pf_batch_instance;
 /*
  * The batch engine: pf_batch_prepare uploads the instances' descriptors into
- * the workspace and lays out a hash table per instance (twice its build rows
- * in 16-byte slots) and a dense (sum, count) slab per instance; it waits
- * once.  pf_batch_run then queues only device work (a reset of the slabs and
- * the work counters, then one persistent launch in which blocks take build
- * and probe work items from a device queue, a probe item waiting, bounded,
- * for its instance's build items), so it can be captured in a CUDA graph and
- * replayed; each run bumps a device epoch that tags the table slots, so the
- * tables are never cleared.  pf_batch_slab gives instance i's slab: int64
- * pairs (sum, count) per group, interleaved.  stats (device int64[4]):
- * matched probe rows, device error word (a bounded wait gave up), build rows
- * out of group range, table overflows.  No counterpart in the reference
- * (which launches per instance); it serves the batching workload.
+ * the workspace and lays out a hash table per instance (8-byte entries at most
+ * 0.4 full, or 16-byte slots where the groups' numbers leave an entry no room)
+ * and a dense (sum, count) slab per instance; it waits once.  pf_batch_run
+ * then queues only device work (a reset of the tables, sums and work counters;
+ * a persistent launch in which blocks take build and probe work items from a
+ * device queue, a probe item waiting, bounded, for its instance's build items;
+ * the sums' check; a second launch over the instances that failed it, which
+ * exits at once when there is none), so it can be captured in a CUDA graph and
+ * replayed.  pf_batch_slab gives instance i's slab: int64 pairs (sum, count)
+ * per group, interleaved.  stats (device int64[4]): matched probe rows, device
+ * error word (a bounded wait gave up), build rows out of group range, table
+ * overflows.  No counterpart in the reference (which launches per instance);
+ * it serves the batching workload.
  */
 size_t pf_batch_workspace(const pf_batch_instance* instances, int n);
 int pf_batch_prepare(const pf_batch_instance* instances, int n, void* workspace,

@@ -2,79 +2,98 @@
 // one persistent launch fed by a device work queue.
 //
 // Layout (the workspace, laid out by pf_batch_prepare):
-//   header       epoch, work counter, item totals, error word
+//   header       epoch, work counters, item totals, error word
 //   descriptors  per instance: its columns, table region, slab, item ranges
 //   remaining    per instance: build items not yet done
-//   tables       per instance, 2 x build rows 16-byte slots {key, group | tag}
+//   checks       per instance: a run's matched rows and what its packed sums
+//                are checked by
+//   flags        per instance: how its runs go (below), kept from run to run
+//   tables       per instance: a compact table (compact.cuh) where its groups
+//                leave an entry room, else 2 x build rows 16-byte slots {key,
+//                group | tag}; a region holds either
+//   packed       per instance and group: {count, sum} in one word
 //   slabs        per instance, n_groups (sum, count) int64 pairs
 //
 // Work items, instance by instance: its build rows in items of BITEM rows,
-// then its probe rows in items of PITEM rows (so the tables in use at any
+// then its probe rows in items of `pitem` rows (so the tables in use at any
 // time are those of the few instances in flight, which stay in L2).  A block
 // takes the next item from the counter; a probe item waits (bounded) until
 // its instance's build items are all done.  Those items were taken before it,
-// by blocks that are running, so the wait always ends.  A slot is free for this run when
-// its tag is below the run's epoch; the claim is an atomicMax of the tag.
-// Matches aggregate with warp-level combining of equal groups (hot keys of a
-// skewed probe side become one atomic per warp, not one per row).
+// by blocks that are running, so the wait always ends.  The compact tables
+// are cleared by each run (22 bytes a build row written); a 16-byte slot is
+// free for this run when its tag is below the run's epoch, and the claim is an
+// atomicMax of the tag.
+//
+// What bounds it: L2's rate of requests.  A probe row costs one table sector and
+// one RED, where 16-byte slots half full took two or three dependent reads and a
+// group's (sum, count) pair two REDs: 48 instances (29M build, 290M probe rows,
+// FKs of Zipf 0, 0.8 and 1.2) 8.7 -> 5.6 ms, 8 of up to 50K rows 285 -> 90 us.
+// One instance of 2M x 20M rows and 20 groups 548 -> 260 us.  Its value and 1 go into the
+// group's packed word, or, for the groups a block meets often (skewed keys),
+// through a cache in shared memory flushed into the slab at the item's end.
+// The values are offset by 2^(b - 1) to take negative ones, b bits each.  What
+// the packed words hold is checked after the run, instance by instance, as in
+// join_direct.cu: every offset value in [0, 2^b), the words' counts add up to
+// the rows put into them, and the sum of the values is bounded, or else some
+// sum may have left its field.  k_batch_sums adds the packed words to the slab
+// and decides; an instance that fails, or whose hashes crowd its compact table,
+// is run again in the same call (k_batch<true>: two words a group, 16-byte
+// slots) and goes that way in later runs of the batch from the start.
 #include <algorithm>
 #include <map>
 #include <mutex>
 #include <vector>
 
 #include "agg.cuh"
+#include "compact.cuh"
 
 namespace pf {
 namespace {
 
 constexpr int BT2 = 256;
 #ifndef PF_BATCH_BV
-#define PF_BATCH_BV 1
+#define PF_BATCH_BV 2
 #endif
-// 1: the probe loop loads the next round's keys and values while this round
-// probes its slots (loading two rounds ahead and prefetching the next
-// round's first slots into L2 measured slower: 35.5 against 42.1 G rows/s)
-#ifndef PF_BATCH_PIPE
-#define PF_BATCH_PIPE 1
+#ifndef PF_BATCH_MINB
+#define PF_BATCH_MINB 4
 #endif
-// rows a thread keeps in flight (all 4096 instances of the batch workload:
-// 1 row 42.7 G rows/s, 2 rows 36.9, 4 rows 29.4: more registers a thread
-// cost more resident warps than the extra loads in flight gain)
+// probe rows a thread takes at a time, at four blocks a SM (62 registers): 48
+// instances 5.6 ms, 1 row at six blocks 6.4
 constexpr int BV = PF_BATCH_BV;
-// 1: a probe item adds into the block's group cache (agg.cuh) and flushes it
-// at the item's end, so the hot groups of a skewed instance cost one global
-// atomic pair a block and item instead of one a warp and step; 0:
-// warp-combined global atomics only.
-#ifndef PF_BATCH_CACHE
-#define PF_BATCH_CACHE 1
-#endif
-// with the cache: 1 combine equal groups of a warp before the cache
-#ifndef PF_BATCH_CACHE_COMBINE
-#define PF_BATCH_CACHE_COMBINE 0
-#endif
-constexpr size_t BATCH_SMEM = PF_BATCH_CACHE ? sizeof(GroupCache) : 0;
-// Warp-combined add whose leaders go through the cache.
-__device__ __forceinline__ void combined_to(GroupCache& gc, unsigned long long* slab, long long g,
-                                            long long value) {
-  const unsigned act = __activemask();
-  const unsigned peers = __match_any_sync(act, g);
-  if (g < 0) return;
-  const unsigned long long v = (unsigned long long)value;
-  const unsigned s0 = __reduce_add_sync(peers, (unsigned)(v & 0x3fffff));
-  const unsigned s1 = __reduce_add_sync(peers, (unsigned)((v >> 22) & 0x3fffff));
-  const unsigned s2 = __reduce_add_sync(peers, (unsigned)(v >> 44));
-  if ((int)(threadIdx.x & 31) == __ffs(peers) - 1)
-    cache_add(gc, slab, g,
-              (unsigned long long)s0 + ((unsigned long long)s1 << 22) +
-                  ((unsigned long long)s2 << 44),
-              (unsigned long long)__popc(peers));
-}
+// The block's own sums in shared memory: lo, hi and count of CELLS cells.  An
+// instance of few groups has all of them there, as many copies of each as fit,
+// a lane its own.  Else, where an item's first rows show groups again, its hot
+// groups (48 instances: 5.6 ms; 256 groups of 4 copies 5.8, and twice the time
+// with 54 KB of cells, whose blocks leave no L1): one is let in when it comes again before another group of its `seen`
+// entry (so one row in about a thousand or more; one that frequent would queue
+// up on its address in L2, which takes a RED every 14 clocks, while groups met
+// once an item would fill the cells), HOT_COPIES copies of each.
+constexpr int CELLS = 1024;
+constexpr int SMALL_GROUPS = 512;
+constexpr int HOT_LOG = 9, HOT = 1 << HOT_LOG, HOT_COPIES = 2;
+constexpr int SEEN_LOG = 10;
+static_assert(HOT * HOT_COPIES <= CELLS && SMALL_GROUPS <= CELLS, "cells");
+struct BatchSmem {
+  unsigned lo[CELLS], hi[CELLS], cnt[CELLS];
+  int tag[HOT];
+  int seen[1 << SEEN_LOG];
+  int inst;    // the instance whose hot groups the tags are, and
+  int cached;  // whether it has any: kept from one item to the block's next
+};
+constexpr size_t BATCH_SMEM = sizeof(BatchSmem);
+constexpr int BATCH_REPEATS = 16;   // of an item's first rows, groups met again: the cache pays
+constexpr int BATCH_MAX_Q = 23;     // 256 MiB tables, 0.4 full at most
+constexpr double BATCH_LOAD = 0.4;
+constexpr int SUM_CHUNK = 4096;     // groups a block of k_batch_sums adds up at a time
 
 constexpr int BITEM = 4096;
-#ifndef PF_BATCH_PITEM
-#define PF_BATCH_PITEM 16384
-#endif
-constexpr int PITEM = PF_BATCH_PITEM;
+// Probe rows of an item: more rows an item, fewer of its barriers, flushes and
+// waits; fewer, and a small batch still has items for every block (8 instances
+// of up to 50K build rows, 1M probe rows: 140 us at 16384, 94 at 4096; 24 of up
+// to 400K, 20M rows: 623 and 809).
+long long probe_item(unsigned long long probe_rows) {
+  return probe_rows <= 2000000 ? 4096 : probe_rows <= 5000000 ? 8192 : 16384;
+}
 constexpr unsigned WAIT_LIMIT = 1u << 24;  // polls of a probe item's wait (x ~0.5 us)
 
 struct Desc {
@@ -86,17 +105,34 @@ struct Desc {
   long long np;
   long long gmin, ng;
   unsigned long long toff;   // first slot of the table region
-  unsigned long long tcap;   // slots
+  unsigned long long tcap;   // 16-byte slots
   unsigned long long soff;   // first (sum, count) pair of the slab
-  long long item0;             // first work item (its build items, then its probe items)
-  long long nbi;               // build items
+  long long item0;           // first work item (its build items, then its probe items)
+  long long nbi;             // build items
+  long long pitem;           // probe rows of an item
+  long long chunk0;          // first chunk of k_batch_sums
+  unsigned long long region; // slots of the table region
+  int q, gbits, dbits;       // compact table (q = 0: none)
+  int sbits, vbits;          // packed word: bits of the sum, of an offset value
+};
+
+// How an instance's runs go: bits of its flags word.
+constexpr unsigned WIDE_SUMS = 1, WIDE_TABLE = 2, REDO = 4;
+
+struct Check {
+  unsigned long long matched;  // probe rows that found their build row
+  unsigned long long rows;     // rows put into packed words
+  unsigned long long high;     // their offset values >> 20, added up
+  unsigned long long counts;   // the packed words' counts, added up
+  unsigned bad_value, crowded;
 };
 
 struct Header {
   unsigned epoch;
-  unsigned pad;
-  unsigned long long counter;
-  long long n_build_items, n_items;
+  unsigned n_redo;
+  unsigned long long counter, counter2;  // items of the first pass, of the second
+  unsigned chunks_done, pad;
+  long long n_build_items, n_items, n_chunks;
   int n_inst;
   int pad2;
   unsigned long long error;
@@ -107,273 +143,536 @@ struct Slot {
   unsigned long long tagged;  // (tag << 32) | group offset
 };
 
+struct Sizes {
+  unsigned long long table_slots, cleared_slots, slab_pairs, items, chunks;
+  long long pitem;
+};
+
 struct Layout {
   Header* header;
   Desc* desc;
   unsigned* remaining;
+  Check* check;
+  unsigned* flags;
   int* imap;  // work item -> instance
+  int* cmap;  // chunk of groups -> instance
   Slot* tables;
+  unsigned long long* packed;
   unsigned long long* slabs;
-  unsigned long long table_slots, slab_pairs;
 };
 
-Layout layout(char* base, int n, unsigned long long table_slots, unsigned long long slab_pairs,
-              unsigned long long items, size_t* used) {
+Layout layout(char* base, int n, const Sizes& z, size_t* used) {
   Arena a(base, ~(size_t)0);
   Layout l{};
   l.header = a.take<Header>(1);
   l.desc = a.take<Desc>(std::max(n, 1));
   l.remaining = a.take<unsigned>(std::max(n, 1));
-  l.imap = a.take<int>(std::max<unsigned long long>(items, 1));
-  l.tables = a.take<Slot>(std::max<unsigned long long>(table_slots, 1));
-  l.slabs = a.take<unsigned long long>(2 * std::max<unsigned long long>(slab_pairs, 1));
-  l.table_slots = table_slots;
-  l.slab_pairs = slab_pairs;
+  l.check = a.take<Check>(std::max(n, 1));
+  l.flags = a.take<unsigned>(std::max(n, 1));
+  l.imap = a.take<int>(std::max<unsigned long long>(z.items, 1));
+  l.cmap = a.take<int>(std::max<unsigned long long>(z.chunks, 1));
+  l.tables = a.take<Slot>(std::max<unsigned long long>(z.table_slots, 1));
+  l.packed = a.take<unsigned long long>(std::max<unsigned long long>(z.slab_pairs, 1));
+  l.slabs = a.take<unsigned long long>(2 * std::max<unsigned long long>(z.slab_pairs, 1));
   if (used) *used = a.used;
   return l;
 }
 
-void totals(const pf_batch_instance* in, int n, unsigned long long* ts, unsigned long long* sp,
-            unsigned long long* items) {
-  *ts = 0;
-  *sp = 0;
-  *items = 0;
+// An instance's compact table (q = 0: none) and the slots of its region.
+unsigned long long table_of(long long nb, long long ng, int* q, int* gbits, int* dbits,
+                            unsigned long long* tcap) {
+  *q = 0;
+  *tcap = 0;
+  if (nb < 1) return 0;
+  // 16-byte slots: a quarter full to 64 MiB (a sector of two in ten full), half
+  // full past it
+  *tcap = (64LL * nb <= (64LL << 20) ? 4ULL : 2ULL) * (unsigned long long)nb;
+  ct_size(nb, std::max<long long>(ng, 1), BATCH_MAX_Q, BATCH_LOAD, BATCH_LOAD, q, gbits, dbits);
+  const unsigned long long least = 2ULL * (unsigned long long)nb;
+  // groups numbered far past the rows would need a table far larger than them
+  if (*q && (2ULL << *q) > 4 * least + 256) *q = 0;
+  if (!*q) return *tcap;
+  *tcap = least;  // only where the compact table fails
+  return std::max(least, 2ULL << *q);
+}
+
+Sizes totals(const pf_batch_instance* in, int n) {
+  Sizes z{};
+  unsigned long long probes = 0;
+  for (int i = 0; i < n; ++i)
+    if (in[i].n_build > 0) probes += (unsigned long long)std::max<int64_t>(in[i].n_probe, 0);
+  z.pitem = probe_item(probes);
   for (int i = 0; i < n; ++i) {
     const long long nb = std::max<int64_t>(in[i].n_build, 0);
     const long long np = nb > 0 ? std::max<int64_t>(in[i].n_probe, 0) : 0;
-    *ts += 2ULL * (unsigned long long)nb;
-    *sp += (unsigned long long)std::max<int64_t>(in[i].n_groups, 0);
-    *items += (unsigned long long)((nb + BITEM - 1) / BITEM + (np + PITEM - 1) / PITEM);
+    const long long ng = std::max<int64_t>(in[i].n_groups, 0);
+    int q, gbits, dbits;
+    unsigned long long tcap;
+    const unsigned long long slots = table_of(nb, ng, &q, &gbits, &dbits, &tcap);
+    z.table_slots += slots;
+    if (q) z.cleared_slots += slots;
+    z.slab_pairs += (unsigned long long)ng;
+    z.items += (unsigned long long)((nb + BITEM - 1) / BITEM + (np + z.pitem - 1) / z.pitem);
+    z.chunks += (unsigned long long)((ng + SUM_CHUNK - 1) / SUM_CHUNK);
   }
+  return z;
 }
 
-// Run start: bump the epoch, zero the counter, the error word and the slabs,
-// and set every instance's remaining build items.
-__global__ void k_batch_reset(Header* h, Desc* d, unsigned* remaining, int n,
-                              unsigned long long* slabs, unsigned long long words) {
-  const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long stride = (long long)gridDim.x * blockDim.x;
+// Run start: bump the epoch, zero the counters, the error word, the checks, the
+// sums and the compact tables, and set every instance's remaining build items.
+__global__ void __launch_bounds__(BT2) k_batch_reset(Header* h, const Desc* d,
+                                                     unsigned* remaining, Check* check, int n,
+                                                     Slot* tables,
+                                                     unsigned long long cleared_slots,
+                                                     unsigned long long* packed,
+                                                     unsigned long long* slabs,
+                                                     unsigned long long pairs) {
+  const unsigned long long tid = (unsigned long long)blockIdx.x * BT2 + threadIdx.x;
+  const unsigned long long stride = (unsigned long long)gridDim.x * BT2;
   if (tid == 0) {
     h->epoch += 1;
-    h->counter = 0;
+    h->n_redo = 0;
+    h->counter = h->counter2 = 0;
+    h->chunks_done = 0;
     h->error = 0;
   }
-  for (long long i = tid; i < n; i += stride) remaining[i] = (unsigned)d[i].nbi;
-  for (long long i = tid; i < (long long)words; i += stride) slabs[i] = 0;
+  for (unsigned long long i = tid; i < (unsigned long long)n; i += stride) {
+    remaining[i] = (unsigned)d[i].nbi;
+    check[i] = Check{0, 0, 0, 0, 0, 0};
+  }
+  const ulonglong2 zero = make_ulonglong2(0ULL, 0ULL);
+  ulonglong2* t = reinterpret_cast<ulonglong2*>(tables);
+  for (unsigned long long i = tid; i < cleared_slots; i += stride) t[i] = zero;
+  ulonglong2* s = reinterpret_cast<ulonglong2*>(slabs);
+  for (unsigned long long i = tid; i < pairs; i += stride) {
+    s[i] = zero;
+    packed[i] = 0;
+  }
 }
 
-__device__ __forceinline__ unsigned first_slot(uint64_t h, unsigned long long cap) {
-  return (unsigned)(((h >> 32) * cap) >> 32);
+// A wide table's slots lie two a sector; a key's home sector.
+__device__ __forceinline__ unsigned first_sector(uint64_t h, unsigned long long cap) {
+  return (unsigned)(((h >> 32) * (cap >> 1)) >> 32);
 }
 
-__global__ void __launch_bounds__(BT2) k_batch(Header* h, const Desc* d, const int* __restrict__ imap,
-                                               unsigned* remaining,
-                                               Slot* tables, unsigned long long* slabs,
-                                               unsigned long long* stats) {
+// One build row into a table of 16-byte slots.
+__device__ __forceinline__ bool wide_insert(const Desc& D, Slot* tables, unsigned epoch,
+                                            unsigned long long key, uint32_t goff) {
+  unsigned p = 2 * first_sector(mix64(key), D.tcap);
+  for (unsigned long long left = D.tcap; left > 0; --left) {
+    Slot* sl = tables + D.toff + p;
+    unsigned* tag = reinterpret_cast<unsigned*>(&sl->tagged) + 1;
+    if (atomicMax(tag, epoch) < epoch) {
+      *reinterpret_cast<ulonglong2*>(sl) =
+          make_ulonglong2(key, ((unsigned long long)epoch << 32) | goff);
+      return true;
+    }
+    if (++p == D.tcap) p = 0;
+  }
+  return false;
+}
+
+// A key in a table of 16-byte slots, x its home sector p: -2 not there, -1
+// there without a group, else the group.
+__device__ __forceinline__ long long wide_lookup(const Desc& D, const Slot* tables,
+                                                 unsigned epoch, unsigned long long key,
+                                                 unsigned p, CtBucket x) {
+  for (unsigned long long probes = 0; probes < D.tcap >> 1; ++probes) {
+#pragma unroll
+    for (int j = 0; j < 4; j += 2) {
+      if ((uint32_t)(x.e[j + 1] >> 32) != epoch) return -2;
+      if (x.e[j] == key) {
+        const uint32_t go = (uint32_t)x.e[j + 1];
+        return go == 0xffffffffu ? -1 : (long long)go;
+      }
+    }
+    if (++p == D.tcap >> 1) p = 0;
+    x = ct_load(reinterpret_cast<const unsigned long long*>(tables + D.toff + 2ULL * p));
+  }
+  return -2;
+}
+
+struct BatchArgs {
+  Header* h;
+  const Desc* d;
+  const int* imap;
+  unsigned* remaining;
+  Check* check;
+  const unsigned* flags;
+  Slot* tables;
+  unsigned long long* packed;
+  unsigned long long* slabs;
+  unsigned long long* stats;
+};
+
+// The probe rows [lo, hi) of an instance, BV rows a thread a step: every key,
+// value and home sector (or slot) loaded before the first is looked at.
+// PACK: a row's value and 1 in one packed word, else in the slab's two.
+template <bool COMPACT, bool PACK>
+__device__ __forceinline__ void probe_rows(const Desc& D, const BatchArgs& a, unsigned epoch,
+                                           BatchSmem& S, bool cached, bool look,
+                                           long long lo, long long hi,
+                                           unsigned& matched, unsigned& rows,
+                                           unsigned long long& high, bool& outside) {
+  unsigned long long* slab = a.slabs + 2 * D.soff;
+  unsigned long long* packed = a.packed + D.soff;
+  const CompactTable t{reinterpret_cast<unsigned long long*>(a.tables + D.toff), D.q, D.gbits,
+                       D.dbits};
+  const long long bias = 1LL << (D.vbits - 1);
+  const int lane = threadIdx.x & 31;
+  // few groups: copies of each (a power of two)
+  const bool small = D.ng <= SMALL_GROUPS;
+  int lcopies = 0;
+  if (small)
+    while (lcopies < 5 && (D.ng << (lcopies + 1)) <= CELLS) ++lcopies;
+  const unsigned copy = lane & ((1u << lcopies) - 1);
+  auto add_cell = [&](unsigned c, long long v) {
+    const unsigned l = (unsigned)(unsigned long long)v;
+    const unsigned hw = (unsigned)((unsigned long long)v >> 32);
+    const unsigned old = atomicAdd(&S.lo[c], l);
+    const unsigned hc = hw + (old + l < old ? 1u : 0u);
+    if (hc) atomicAdd(&S.hi[c], hc);
+    atomicAdd(&S.cnt[c], 1u);
+  };
+  for (long long i0 = lo; i0 < hi; i0 += BT2 * BV) {
+    unsigned long long key[BV], hash[BV];
+    long long value[BV], g[BV];
+    bool live[BV];
+#pragma unroll
+    for (int k = 0; k < BV; ++k) {
+      const long long i = i0 + k * BT2 + threadIdx.x;
+      live[k] = i < hi;
+      key[k] = live[k] ? (unsigned long long)__ldcs(D.pfk + i) : 0ULL;
+    }
+#pragma unroll
+    for (int k = 0; k < BV; ++k) {
+      const long long i = i0 + k * BT2 + threadIdx.x;
+      value[k] = live[k] ? __ldcs(D.pval + i) : 0;
+    }
+    if (COMPACT) {
+      CtBucket b[BV];
+#pragma unroll
+      for (int k = 0; k < BV; ++k) {
+        hash[k] = ct_hash((long long)key[k]);
+        b[k] = ct_load(ct_home(t, hash[k]));
+      }
+#pragma unroll
+      for (int k = 0; k < BV; ++k) {
+        g[k] = -2;
+        if (!live[k]) continue;
+        bool more;
+        const unsigned long long want = ct_want(t, hash[k]);
+        unsigned long long e = ct_among(t, b[k], want, &more);
+        if (more) e = ct_walk(t, hash[k], want);
+        if (e != CT_EMPTY) g[k] = ct_group(t, e);
+      }
+    } else {
+      CtBucket x[BV];
+#pragma unroll
+      for (int k = 0; k < BV; ++k) {
+        hash[k] = first_sector(mix64(key[k]), D.tcap);
+        x[k] = ct_load(
+            reinterpret_cast<const unsigned long long*>(a.tables + D.toff + 2ULL * hash[k]));
+      }
+#pragma unroll
+      for (int k = 0; k < BV; ++k)
+        g[k] = live[k] ? wide_lookup(D, a.tables, epoch, key[k], (unsigned)hash[k], x[k]) : -2;
+    }
+    int repeats = 0;
+#pragma unroll
+    for (int k = 0; k < BV; ++k) {
+      matched += g[k] >= -1;
+      if (g[k] < 0) continue;
+      if (small) {
+        add_cell((unsigned)g[k] << lcopies | copy, value[k]);
+        continue;
+      }
+      const unsigned mixed = (unsigned)g[k] * 0x9E3779B1u;
+      volatile int* seen = &S.seen[mixed >> (32 - SEEN_LOG)];
+      if (cached) {
+        unsigned slot = mixed >> (32 - HOT_LOG);
+        const int t0 = *(volatile int*)&S.tag[slot], t1 = *(volatile int*)&S.tag[slot ^ 1];
+        if (t1 == (int)g[k]) slot ^= 1;
+        if (t0 == (int)g[k] || t1 == (int)g[k]) {
+          add_cell(slot * HOT_COPIES + (lane & (HOT_COPIES - 1)), value[k]);
+          continue;
+        }
+        if (*seen == (int)g[k]) {
+          if (t0 == -1) atomicCAS(&S.tag[slot], -1, (int)g[k]);
+          else if (t1 == -1) atomicCAS(&S.tag[slot ^ 1], -1, (int)g[k]);
+        } else {
+          *seen = (int)g[k];
+        }
+      } else if (look && i0 == lo) {
+        // the instance's first rows here: how often a group comes again
+        repeats += *seen == (int)g[k];
+        *seen = (int)g[k];
+      }
+      if (PACK) {
+        const unsigned long long v = (unsigned long long)(value[k] + bias);
+        outside |= v >> D.vbits != 0;
+        high += v >> 20;
+        ++rows;
+        atomicAdd(&packed[g[k]], (1ULL << D.sbits) + v);
+      } else {
+        atomicAdd(&slab[2 * (unsigned long long)g[k]], (unsigned long long)value[k]);
+        atomicAdd(&slab[2 * (unsigned long long)g[k] + 1], 1ULL);
+      }
+    }
+    if (look && i0 == lo && !small) {
+      cached = __syncthreads_count(repeats > 0) >= BATCH_REPEATS;
+      if (threadIdx.x == 0) S.cached = cached;
+    }
+  }
+  __syncthreads();
+  // the item's own sums into the slab, and emptied
+  if (small) {
+    for (int g0 = threadIdx.x; g0 < (int)D.ng; g0 += BT2) {
+      unsigned long long sum = 0, n = 0;
+      for (int j = 0; j < 1 << lcopies; ++j) {
+        const int c = g0 << lcopies | ((j + lane) & ((1 << lcopies) - 1));
+        sum += (unsigned long long)S.hi[c] << 32 | S.lo[c];
+        n += S.cnt[c];
+        S.lo[c] = S.hi[c] = S.cnt[c] = 0;
+      }
+      if (n) {
+        atomicAdd(&slab[2 * g0], sum);
+        atomicAdd(&slab[2 * g0 + 1], n);
+      }
+    }
+  } else if (cached) {
+    for (int i = threadIdx.x; i < HOT; i += BT2) {
+      const int g0 = S.tag[i];
+      if (g0 < 0) continue;
+      unsigned long long sum = 0, n = 0;
+      for (int j = 0; j < HOT_COPIES; ++j) {
+        const int c = i * HOT_COPIES + ((j + lane) & (HOT_COPIES - 1));
+        sum += (unsigned long long)S.hi[c] << 32 | S.lo[c];
+        n += S.cnt[c];
+        S.lo[c] = S.hi[c] = S.cnt[c] = 0;
+      }
+      if (!n) continue;
+      atomicAdd(&slab[2 * (unsigned long long)g0], sum);
+      atomicAdd(&slab[2 * (unsigned long long)g0 + 1], n);
+    }
+  }
+  __syncthreads();
+}
+
+// SECOND: the instances to be run again, two words a group, 16-byte slots.
+template <bool SECOND>
+__global__ void __launch_bounds__(BT2, PF_BATCH_MINB) k_batch(BatchArgs a) {
+  Header* h = a.h;
+  if (SECOND && h->n_redo == 0) return;
   __shared__ long long item_s;
   __shared__ int ok_s;
+  __shared__ unsigned long long red[3][BT2 / 32];
+  __shared__ unsigned outside_s;
   const unsigned epoch = h->epoch;
   const long long ni = h->n_items;
-  unsigned long long matched = 0, bad_group = 0, overflow = 0;
-#if PF_BATCH_CACHE
+  unsigned long long bad_group = 0, overflow = 0;
   extern __shared__ __align__(16) unsigned char batch_smem[];
-  GroupCache& gc = *reinterpret_cast<GroupCache*>(batch_smem);
-  cache_init(gc);
-#endif
-  // With PF_PREFETCH_ITEMS, thread 0 takes the block's next item while the
-  // block works on the current one (measured no faster, so off by default).
+  BatchSmem& S = *reinterpret_cast<BatchSmem*>(batch_smem);
+  for (int i = threadIdx.x; i < CELLS; i += BT2) S.lo[i] = S.hi[i] = S.cnt[i] = 0;
+  if (threadIdx.x == 0) S.inst = -1;
+  for (int i = threadIdx.x; i < 1 << SEEN_LOG; i += BT2) S.seen[i] = -1;
   // Items are taken in increasing order and an item waits only for items
   // before it, so the smallest unfinished item is always some block's
   // current item with nothing left to wait for: the launch progresses.
-  if (threadIdx.x == 0) item_s = (long long)atomicAdd(&h->counter, 1ULL);
+  unsigned long long* counter = SECOND ? &h->counter2 : &h->counter;
   while (true) {
+    if (threadIdx.x == 0) item_s = (long long)atomicAdd(counter, 1ULL);
     __syncthreads();
     const long long it = item_s;
+    __syncthreads();  // every thread has read item_s
     if (it >= ni) break;
-    unsigned long long next = 0;
-    if (PF_PREFETCH_ITEMS && threadIdx.x == 0) next = atomicAdd(&h->counter, 1ULL);
-    const int inst = imap[it];
+    const int inst = a.imap[it];
+    const unsigned flags = a.flags[inst];
+    if (SECOND && !(flags & REDO)) continue;
     // the instance's descriptor in registers for the item (read through a
     // reference, every store to the tables or slabs would reload it)
-    const Desc D = d[inst];
+    const Desc D = a.d[inst];
+    const bool compact = !SECOND && D.q > 0 && !(flags & WIDE_TABLE);
     const long long local = it - D.item0;
     if (local < D.nbi) {
-      // BV rows a thread at a time: loads, then every first claim, then the
-      // (rare) collisions
+      const CompactTable t{reinterpret_cast<unsigned long long*>(a.tables + D.toff), D.q,
+                           D.gbits, D.dbits};
       const long long lo = local * BITEM, hi = min(D.nb, lo + BITEM);
-      for (long long i0 = lo; i0 < hi; i0 += BT2 * BV) {
-        unsigned long long key[BV];
-        uint32_t goff[BV];
-        unsigned pos[BV];
-        bool live[BV], done[BV];
-#pragma unroll
-        for (int k = 0; k < BV; ++k) {
-          const long long i = i0 + k * BT2 + threadIdx.x;
-          live[k] = i < hi;
-          key[k] = live[k] ? (unsigned long long)D.bkey[i] : 0ULL;
-          const long long g = live[k] ? (long long)D.bgrp[i] - D.gmin : 0;
-          goff[k] = 0xffffffffu;
-          if (g >= 0 && g < D.ng) goff[k] = (uint32_t)g;
-          else if (live[k]) ++bad_group;
-        }
-#pragma unroll
-        for (int k = 0; k < BV; ++k) {
-          pos[k] = first_slot(mix64(key[k]), D.tcap);
-          done[k] = false;
-          if (!live[k]) continue;
-          Slot* sl = tables + D.toff + pos[k];
-          unsigned* tag = reinterpret_cast<unsigned*>(&sl->tagged) + 1;
-          if (atomicMax(tag, epoch) < epoch) {
-            *reinterpret_cast<ulonglong2*>(sl) =
-                make_ulonglong2(key[k], ((unsigned long long)epoch << 32) | goff[k]);
-            done[k] = true;
-          }
-        }
-#pragma unroll
-        for (int k = 0; k < BV; ++k) {
-          if (!live[k] || done[k]) continue;
-          unsigned p = pos[k];
-          for (unsigned long long left = D.tcap - 1; left > 0; --left) {
-            if (++p == D.tcap) p = 0;
-            Slot* sl = tables + D.toff + p;
-            unsigned* tag = reinterpret_cast<unsigned*>(&sl->tagged) + 1;
-            if (atomicMax(tag, epoch) < epoch) {
-              *reinterpret_cast<ulonglong2*>(sl) =
-                  make_ulonglong2(key[k], ((unsigned long long)epoch << 32) | goff[k]);
-              done[k] = true;
-              break;
-            }
-          }
-          overflow += !done[k];
+      for (long long i = lo + threadIdx.x; i < hi; i += BT2) {
+        const long long key = __ldcs(D.bkey + i), g = (long long)__ldcs(D.bgrp + i) - D.gmin;
+        const bool in = g >= 0 && g < D.ng;
+        if (!SECOND) bad_group += !in;
+        if (compact) {
+          if (!ct_insert(t, key, in ? g : -1)) a.check[inst].crowded = 1;
+        } else {
+          overflow += !wide_insert(D, a.tables, epoch, (unsigned long long)key,
+                                   in ? (uint32_t)g : 0xffffffffu);
         }
       }
       __syncthreads();
       if (threadIdx.x == 0) {
         __threadfence();
-        atomicSub(&remaining[inst], 1u);
+        atomicSub(&a.remaining[inst], 1u);
       }
     } else {
       if (threadIdx.x == 0) {
         unsigned polls = 0;
-        while (ld_acquire_u32(&remaining[inst]) != 0 && polls < WAIT_LIMIT) {
+        while (ld_acquire_u32(&a.remaining[inst]) != 0 && polls < WAIT_LIMIT) {
           __nanosleep(256);
           ++polls;
         }
         ok_s = polls < WAIT_LIMIT;
         if (!ok_s) atomicOr(&h->error, 1ULL);
+        outside_s = 0;
         __threadfence();
       }
       __syncthreads();
-      if (!ok_s) {
-        if (threadIdx.x == 0) item_s = (long long)(PF_PREFETCH_ITEMS ? next : atomicAdd(&h->counter, 1ULL));
-        continue;
+      if (!ok_s) continue;
+      const bool look = S.inst != inst;
+      const bool cached = !look && S.cached;
+      if (look) {
+        for (int i = threadIdx.x; i < HOT; i += BT2) S.tag[i] = -1;
+        __syncthreads();  // every thread has read S.inst
+        if (threadIdx.x == 0) {
+          S.inst = inst;
+          S.cached = 0;
+        }
+        __syncthreads();
       }
-      // BV rows a thread at a time: keys, then every first slot and value,
-      // then the (rare) collisions
-      const long long lo = (local - D.nbi) * PITEM, hi = min(D.np, lo + PITEM);
-#if PF_BATCH_PIPE
-      // the next round's keys and values load while this round probes
-      unsigned long long key[BV];
-      long long value[BV];
-#pragma unroll
-      for (int k = 0; k < BV; ++k) {
-        const long long i = lo + k * BT2 + threadIdx.x;
-        const bool l = i < hi && D.tcap > 0;
-        key[k] = l ? (unsigned long long)D.pfk[i] : 0ULL;
-        value[k] = l ? D.pval[i] : 0;
+      const long long lo = (local - D.nbi) * D.pitem, hi = min(D.np, lo + D.pitem);
+      unsigned matched = 0, rows = 0;
+      unsigned long long high = 0;
+      bool outside = false;
+      const bool pack = !SECOND && !(flags & WIDE_SUMS);
+      if (compact && pack)
+        probe_rows<true, true>(D, a, epoch, S, cached, look, lo, hi, matched, rows, high, outside);
+      else if (compact)
+        probe_rows<true, false>(D, a, epoch, S, cached, look, lo, hi, matched, rows, high, outside);
+      else if (pack)
+        probe_rows<false, true>(D, a, epoch, S, cached, look, lo, hi, matched, rows, high, outside);
+      else
+        probe_rows<false, false>(D, a, epoch, S, cached, look, lo, hi, matched, rows, high, outside);
+      // the item's counts, one atomic each
+      unsigned long long m = __reduce_add_sync(FULL, matched), r = __reduce_add_sync(FULL, rows);
+      for (int o = 16; o; o >>= 1) high += __shfl_xor_sync(FULL, high, o);
+      if (outside) outside_s = 1;
+      if ((threadIdx.x & 31) == 0) {
+        red[0][threadIdx.x >> 5] = m;
+        red[1][threadIdx.x >> 5] = r;
+        red[2][threadIdx.x >> 5] = high;
       }
-#endif
-      for (long long i0 = lo; i0 < hi; i0 += BT2 * BV) {
-        unsigned pos[BV];
-        ulonglong2 sl[BV];
-        long long g[BV];
-        bool live[BV];
-#if PF_BATCH_PIPE
-        unsigned long long nkey[BV];
-        long long nval[BV];
-#pragma unroll
-        for (int k = 0; k < BV; ++k) {
-          const long long i = i0 + (long long)BT2 * BV + k * BT2 + threadIdx.x;
-          const bool l = i < hi && D.tcap > 0;
-          nkey[k] = l ? (unsigned long long)D.pfk[i] : 0ULL;
-          nval[k] = l ? D.pval[i] : 0;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        for (int w = 1; w < BT2 / 32; ++w) {
+          m += red[0][w];
+          r += red[1][w];
+          high += red[2][w];
         }
-#pragma unroll
-        for (int k = 0; k < BV; ++k) {
-          live[k] = i0 + k * BT2 + threadIdx.x < hi && D.tcap > 0;
-          pos[k] = live[k] ? first_slot(mix64(key[k]), D.tcap) : 0u;
-          sl[k] = live[k] ? __ldcg(reinterpret_cast<const ulonglong2*>(tables + D.toff + pos[k]))
-                          : make_ulonglong2(0ULL, 0ULL);
-        }
-#else
-        unsigned long long key[BV];
-        long long value[BV];
-#pragma unroll
-        for (int k = 0; k < BV; ++k) {
-          const long long i = i0 + k * BT2 + threadIdx.x;
-          live[k] = i < hi && D.tcap > 0;
-          key[k] = live[k] ? (unsigned long long)D.pfk[i] : 0ULL;
-        }
-#pragma unroll
-        for (int k = 0; k < BV; ++k) {
-          const long long i = i0 + k * BT2 + threadIdx.x;
-          pos[k] = live[k] ? first_slot(mix64(key[k]), D.tcap) : 0u;
-          sl[k] = live[k] ? __ldcg(reinterpret_cast<const ulonglong2*>(tables + D.toff + pos[k]))
-                          : make_ulonglong2(0ULL, 0ULL);
-          value[k] = live[k] ? D.pval[i] : 0;
-        }
-#endif
-#pragma unroll
-        for (int k = 0; k < BV; ++k) {
-          g[k] = -1;
-          if (!live[k]) continue;
-          ulonglong2 x = sl[k];
-          unsigned p = pos[k];
-          for (unsigned long long probes = 0; probes < D.tcap; ++probes) {
-            if ((uint32_t)(x.y >> 32) != epoch) break;
-            if (x.x == key[k]) {
-              ++matched;
-              const uint32_t go = (uint32_t)x.y;
-              if (go != 0xffffffffu) g[k] = go;
-              break;
-            }
-            if (++p == D.tcap) p = 0;
-            x = __ldcg(reinterpret_cast<const ulonglong2*>(tables + D.toff + p));
-          }
-        }
-#pragma unroll
-        for (int k = 0; k < BV; ++k) {
-#if PF_BATCH_CACHE && PF_BATCH_CACHE_COMBINE
-          combined_to(gc, slabs + 2 * D.soff, g[k], g[k] >= 0 ? value[k] : 0);
-#elif PF_BATCH_CACHE
-          if (g[k] >= 0) cache_add(gc, slabs + 2 * D.soff, g[k], (unsigned long long)value[k], 1ULL);
-#else
-          combined_add(slabs + 2 * D.soff, g[k], g[k] >= 0 ? value[k] : 0);
-#endif
-        }
-#if PF_BATCH_PIPE
-#pragma unroll
-        for (int k = 0; k < BV; ++k) {
-          key[k] = nkey[k];
-          value[k] = nval[k];
-        }
-#endif
+        Check* c = a.check + inst;
+        if (m) atomicAdd(&c->matched, m);
+        if (r) atomicAdd(&c->rows, r);
+        if (high) atomicAdd(&c->high, high);
+        if (outside_s) c->bad_value = 1;
       }
-#if PF_BATCH_CACHE
-      cache_flush(gc, slabs + 2 * D.soff);
-#endif
     }
-    __syncthreads();  // every thread has read item_s
-    if (threadIdx.x == 0) item_s = (long long)(PF_PREFETCH_ITEMS ? next : atomicAdd(&h->counter, 1ULL));
   }
-  for (int o = 16; o; o >>= 1) matched += __shfl_xor_sync(FULL, matched, o);
-  if ((threadIdx.x & 31) == 0 && matched) atomicAdd(&stats[0], matched);
-  if (bad_group) atomicAdd(&stats[2], bad_group);
-  if (overflow) atomicAdd(&stats[3], overflow);
+  if (bad_group) atomicAdd(&a.stats[2], bad_group);
+  if (overflow) atomicAdd(&a.stats[3], overflow);
 }
 
-__global__ void k_batch_error(const Header* h, unsigned long long* stats) {
-  if (threadIdx.x == 0 && h->error) stats[1] |= h->error;
+// The packed words added to the slabs; the last block decides which instances
+// are run again and how, and readies them (their tables and sums are cleared
+// by k_batch_again).
+__global__ void __launch_bounds__(BT2) k_batch_sums(BatchArgs a, const int* __restrict__ cmap,
+                                                    unsigned* flags) {
+  Header* h = a.h;
+  __shared__ unsigned long long red[BT2 / 32];
+  __shared__ int last_s;
+  for (long long c = blockIdx.x; c < h->n_chunks; c += gridDim.x) {
+    const int inst = cmap[c];
+    const Desc& D = a.d[inst];
+    const long long g0 = (c - D.chunk0) * SUM_CHUNK, g1 = min(D.ng, g0 + SUM_CHUNK);
+    const unsigned long long smask = (1ULL << D.sbits) - 1;
+    const unsigned long long bias = 1ULL << (D.vbits - 1);
+    ulonglong2* slab = reinterpret_cast<ulonglong2*>(a.slabs) + D.soff;
+    unsigned long long total = 0;
+    for (long long g = g0 + threadIdx.x; g < g1; g += BT2) {
+      const unsigned long long x = a.packed[D.soff + g];
+      if (!x) continue;
+      const unsigned long long n = x >> D.sbits;
+      ulonglong2 v = slab[g];
+      v.x += (x & smask) - n * bias;
+      v.y += n;
+      slab[g] = v;
+      total += n;
+    }
+    for (int o = 16; o; o >>= 1) total += __shfl_xor_sync(FULL, total, o);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = total;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int w = 1; w < BT2 / 32; ++w) total += red[w];
+      if (total) atomicAdd(&a.check[inst].counts, total);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last_s = atomicAdd(&h->chunks_done, 1u) == gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!last_s) return;
+  unsigned redo = 0;
+  for (int i = threadIdx.x; i < h->n_inst; i += BT2) {
+    Check* c = a.check + i;
+    const unsigned f = flags[i] & ~REDO;
+    unsigned add = 0;
+    if (*(volatile unsigned*)&c->crowded) add |= WIDE_TABLE | REDO;
+    const unsigned long long rows = *(volatile unsigned long long*)&c->rows;
+    if (!(f & WIDE_SUMS) &&
+        (*(volatile unsigned*)&c->bad_value ||
+         *(volatile unsigned long long*)&c->counts != rows ||
+         *(volatile unsigned long long*)&c->high + rows >= 1ULL << 43))
+      add |= WIDE_SUMS | REDO;
+    flags[i] = f | add;
+    if (add & REDO) {
+      ++redo;
+      a.remaining[i] = (unsigned)a.d[i].nbi;
+      c->matched = 0;
+    }
+  }
+  if (redo) atomicAdd(&h->n_redo, redo);
+}
+
+// The tables and sums of the instances to be run again, cleared.
+__global__ void __launch_bounds__(BT2) k_batch_again(BatchArgs a) {
+  if (a.h->n_redo == 0) return;
+  const unsigned long long tid = (unsigned long long)blockIdx.x * BT2 + threadIdx.x;
+  const unsigned long long stride = (unsigned long long)gridDim.x * BT2;
+  const ulonglong2 zero = make_ulonglong2(0ULL, 0ULL);
+  for (int i = 0; i < a.h->n_inst; ++i) {
+    if (!(a.flags[i] & REDO)) continue;
+    const Desc& D = a.d[i];
+    ulonglong2* t = reinterpret_cast<ulonglong2*>(a.tables + D.toff);
+    for (unsigned long long k = tid; k < D.region; k += stride) t[k] = zero;
+    ulonglong2* s = reinterpret_cast<ulonglong2*>(a.slabs) + D.soff;
+    for (unsigned long long k = tid; k < (unsigned long long)D.ng; k += stride) s[k] = zero;
+  }
+}
+
+// The run's end: the instances' matched rows added up, the error word.
+__global__ void __launch_bounds__(BT2) k_batch_end(BatchArgs a) {
+  __shared__ unsigned long long red[BT2 / 32];
+  unsigned long long m = 0;
+  for (int i = threadIdx.x; i < a.h->n_inst; i += BT2) m += a.check[i].matched;
+  for (int o = 16; o; o >>= 1) m += __shfl_xor_sync(FULL, m, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  for (int w = 1; w < BT2 / 32; ++w) m += red[w];
+  a.stats[0] = m;
+  if (a.h->error) a.stats[1] |= a.h->error;
 }
 
 // What pf_batch_run and pf_batch_slab need of a prepared workspace, kept on
@@ -381,7 +680,7 @@ __global__ void k_batch_error(const Header* h, unsigned long long* stats) {
 // copy of device memory and can be captured.
 struct HostPlan {
   int n = 0;
-  unsigned long long table_slots = 0, slab_pairs = 0, items = 0;
+  Sizes sizes{};
   std::vector<unsigned long long> slab_off;
 };
 
@@ -396,11 +695,13 @@ bool find_plan(void* ws, HostPlan* out) {
   return true;
 }
 
-// The persistent grid: every block resident at once.
+// A persistent grid: every block resident at once.
+template <bool SECOND>
 int batch_grid(int* grid) {
   int per_sm = 0;
-  if (int rc = opt_in_smem((const void*)k_batch, BATCH_SMEM)) return rc;
-  PF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch, BT2, BATCH_SMEM));
+  if (int rc = opt_in_smem((const void*)k_batch<SECOND>, BATCH_SMEM)) return rc;
+  PF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch<SECOND>, BT2,
+                                                        BATCH_SMEM));
   *grid = std::max(1, per_sm) * sm_count();
   return PF_OK;
 }
@@ -411,10 +712,8 @@ int batch_grid(int* grid) {
 using namespace pf;
 
 extern "C" size_t pf_batch_workspace(const pf_batch_instance* in, int n) {
-  unsigned long long ts, sp, items;
-  totals(in, n, &ts, &sp, &items);
   size_t used = 0;
-  layout(nullptr, n, ts, sp, items, &used);
+  layout(nullptr, n, totals(in, n), &used);
   return used + 256;
 }
 
@@ -422,17 +721,18 @@ extern "C" int pf_batch_prepare(const pf_batch_instance* in, int n, void* worksp
                                 size_t workspace_bytes, void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
   if (n < 1) return fail(PF_EINVAL, "batch: at least one instance");
-  unsigned long long ts, sp, items;
-  totals(in, n, &ts, &sp, &items);
+  const Sizes z = totals(in, n);
+  const unsigned long long ts = z.table_slots, items = z.items;
   size_t used = 0;
-  Layout l = layout((char*)workspace, n, ts, sp, items, &used);
+  Layout l = layout((char*)workspace, n, z, &used);
   if (!workspace || used > workspace_bytes || ((uintptr_t)workspace & 255))
     return fail(PF_ENOSPACE,
                 "batch: workspace of %zu bytes at %p, %zu needed on a 256-byte boundary",
                 workspace_bytes, workspace, used);
   std::vector<Desc> d(n);
-  unsigned long long toff = 0, soff = 0;
-  long long bi = 0, pi = 0;
+  // the regions of compact tables first: a run clears them in one piece
+  unsigned long long toff = 0, wide_off = z.cleared_slots, soff = 0;
+  long long bi = 0, pi = 0, chunks = 0;
   for (int i = 0; i < n; ++i) {
     const pf_batch_instance& x = in[i];
     if (x.n_build < 0 || x.n_probe < 0 || x.n_groups < 0 || x.n_groups > 0xfffffffeLL)
@@ -450,41 +750,60 @@ extern "C" int pf_batch_prepare(const pf_batch_instance* in, int n, void* worksp
     D.np = (x.n_build > 0) ? x.n_probe : 0;
     D.gmin = x.group_min;
     D.ng = x.n_groups;
-    D.toff = toff;
-    D.tcap = 2ULL * (unsigned long long)x.n_build;
-    if (D.tcap > 0xffffffffULL) return fail(PF_EINVAL, "batch: instance %d is over 2^31 build rows", i);
+    D.region = table_of(x.n_build, x.n_groups, &D.q, &D.gbits, &D.dbits, &D.tcap);
+    unsigned long long& at = D.q ? toff : wide_off;
+    D.toff = at;
+    at += D.region;
+    if (2ULL * (unsigned long long)x.n_build > 0xffffffffULL) return fail(PF_EINVAL, "batch: instance %d is over 2^31 build rows", i);
+    // the packed word: the count's field for 16 times the mean rows a group (or
+    // for all rows), a value's bits what a group of four times the mean leaves,
+    // 40 at most (the offset counts in every sum)
+    const int mean = bits_of((unsigned long long)(D.np / std::max<long long>(x.n_groups, 1)));
+    const int cbits = std::min(bits_of((unsigned long long)D.np), mean + 4);
+    D.sbits = std::min(64 - cbits, 62);
+    D.vbits = std::max(8, std::min(D.sbits - mean - 2, 40));
     D.soff = soff;
     D.item0 = bi + pi;
     D.nbi = (D.nb + BITEM - 1) / BITEM;
-    toff += D.tcap;
+    D.pitem = z.pitem;
+    D.chunk0 = chunks;
+    chunks += (x.n_groups + SUM_CHUNK - 1) / SUM_CHUNK;
     soff += (unsigned long long)x.n_groups;
     bi += (D.nb + BITEM - 1) / BITEM;
-    pi += (D.np + PITEM - 1) / PITEM;
+    pi += (D.np + z.pitem - 1) / z.pitem;
   }
   Header hh{};
   hh.epoch = 0;
   hh.counter = 0;
   hh.n_build_items = bi;
   hh.n_items = bi + pi;
+  hh.n_chunks = chunks;
   hh.n_inst = n;
   if ((unsigned long long)(bi + pi) != items)
     return fail(PF_EINVAL, "batch: %lld work items, %llu planned", bi + pi, items);
   std::vector<int> imap((size_t)std::max<unsigned long long>(items, 1), 0);
   for (int i = 0; i < n; ++i) {
-    const long long nit = d[i].nbi + (d[i].np + PITEM - 1) / PITEM;
+    const long long nit = d[i].nbi + (d[i].np + z.pitem - 1) / z.pitem;
     for (long long k = 0; k < nit; ++k) imap[(size_t)(d[i].item0 + k)] = i;
   }
+  std::vector<int> cmap((size_t)std::max<unsigned long long>(z.chunks, 1), 0);
+  for (int i = 0; i < n; ++i)
+    for (long long k = 0; k < (d[i].ng + SUM_CHUNK - 1) / SUM_CHUNK; ++k)
+      cmap[(size_t)(d[i].chunk0 + k)] = i;
+  PF_CUDA(cudaMemcpyAsync(l.cmap, cmap.data(), sizeof(int) * cmap.size(), cudaMemcpyHostToDevice,
+                          st));
+  PF_CUDA(cudaMemsetAsync(l.flags, 0, sizeof(unsigned) * n, st));
   PF_CUDA(cudaMemcpyAsync(l.imap, imap.data(), sizeof(int) * imap.size(), cudaMemcpyHostToDevice,
                           st));
   PF_CUDA(cudaMemcpyAsync(l.desc, d.data(), sizeof(Desc) * n, cudaMemcpyHostToDevice, st));
   PF_CUDA(cudaMemcpyAsync(l.header, &hh, sizeof(Header), cudaMemcpyHostToDevice, st));
-  PF_CUDA(cudaMemsetAsync(l.tables, 0, sizeof(Slot) * std::max<unsigned long long>(ts, 1), st));
-  if (int rc = wait_stream(st)) return rc;  // the host copies above read d and hh
+  // (each run clears the compact tables)
+  PF_CUDA(cudaMemsetAsync(l.tables + z.cleared_slots, 0, sizeof(Slot) * (ts - z.cleared_slots),
+                          st));
+  if (int rc = wait_stream(st)) return rc;  // the host copies above read d, hh and the maps
   HostPlan hp;
   hp.n = n;
-  hp.table_slots = ts;
-  hp.slab_pairs = sp;
-  hp.items = items;
+  hp.sizes = z;
   hp.slab_off.resize(n);
   for (int i = 0; i < n; ++i) hp.slab_off[i] = d[i].soff;
   {
@@ -499,36 +818,57 @@ extern "C" int pf_batch_run(void* workspace, int64_t* stats, void* stream) {
   HostPlan hp;
   if (!find_plan(workspace, &hp)) return fail(PF_EINVAL, "batch: workspace was not prepared");
   if (!stats) return fail(PF_EINVAL, "batch: null stats");
-  Layout l = layout((char*)workspace, hp.n, hp.table_slots, hp.slab_pairs, hp.items, nullptr);
-  int grid = 0;
-  if (int rc = batch_grid(&grid)) return rc;
+  Layout l = layout((char*)workspace, hp.n, hp.sizes, nullptr);
+  int grid = 0, grid2 = 0;
+  if (int rc = batch_grid<false>(&grid)) return rc;
+  if (int rc = batch_grid<true>(&grid2)) return rc;
+  const BatchArgs a{l.header,   l.desc,   l.imap,  l.remaining, l.check,
+                    l.flags,    l.tables, l.packed, l.slabs,    (unsigned long long*)stats};
+  const int sms = sm_count();
   PF_CUDA(cudaMemsetAsync(stats, 0, 4 * sizeof(int64_t), st));
   {
     PF_KERNEL("k_batch_reset", st);
-    const long long words = 2LL * (long long)hp.slab_pairs;
-    const unsigned g = (unsigned)std::max<long long>(
-        1, std::min<long long>((words + 255) / 256, (long long)sm_count() * 8));
-    k_batch_reset<<<g, 256, 0, st>>>(l.header, l.desc, l.remaining, hp.n, l.slabs,
-                                      (unsigned long long)words);
+    const long long words = (long long)std::max(hp.sizes.slab_pairs, hp.sizes.cleared_slots);
+    k_batch_reset<<<(unsigned)std::max<long long>(
+                        1, std::min<long long>((words + BT2 - 1) / BT2, sms * 8LL)),
+                    BT2, 0, st>>>(l.header, l.desc, l.remaining, l.check, hp.n, l.tables,
+                                  hp.sizes.cleared_slots, l.packed, l.slabs,
+                                  hp.sizes.slab_pairs);
   }
   PF_LAUNCH("k_batch_reset");
   {
     PF_KERNEL("k_batch", st);
-    k_batch<<<grid, BT2, BATCH_SMEM, st>>>(l.header, l.desc, l.imap, l.remaining, l.tables, l.slabs,
-                                  (unsigned long long*)stats);
+    k_batch<false><<<grid, BT2, BATCH_SMEM, st>>>(a);
   }
   PF_LAUNCH("k_batch");
   {
-    PF_KERNEL("k_batch_error", st);
-    k_batch_error<<<1, 32, 0, st>>>(l.header, (unsigned long long*)stats);
+    PF_KERNEL("k_batch_sums", st);
+    k_batch_sums<<<(unsigned)std::max<long long>(
+                       1, std::min<long long>((long long)hp.sizes.chunks, sms * 4LL)),
+                   BT2, 0, st>>>(a, l.cmap, l.flags);
   }
-  PF_LAUNCH("k_batch_error");
+  PF_LAUNCH("k_batch_sums");
+  {
+    PF_KERNEL("k_batch_again", st);
+    k_batch_again<<<sms * 4, BT2, 0, st>>>(a);
+  }
+  PF_LAUNCH("k_batch_again");
+  {
+    PF_KERNEL("k_batch", st);
+    k_batch<true><<<grid2, BT2, BATCH_SMEM, st>>>(a);
+  }
+  PF_LAUNCH("k_batch");
+  {
+    PF_KERNEL("k_batch_end", st);
+    k_batch_end<<<1, BT2, 0, st>>>(a);
+  }
+  PF_LAUNCH("k_batch_end");
   return ok();
 }
 
 extern "C" int64_t* pf_batch_slab(void* workspace, int i) {
   HostPlan hp;
   if (!find_plan(workspace, &hp) || i < 0 || i >= hp.n) return nullptr;
-  Layout l = layout((char*)workspace, hp.n, hp.table_slots, hp.slab_pairs, hp.items, nullptr);
+  Layout l = layout((char*)workspace, hp.n, hp.sizes, nullptr);
   return (int64_t*)(l.slabs + 2 * hp.slab_off[i]);
 }
