@@ -653,8 +653,9 @@ int64_t* pf_batch_slab(void* workspace, int i);
 
 /* ---- serving: resident dimension tables, requests in persistent launches -- */
 /*
- * A dimension table's hash table, built once and kept across requests:
- * 16-byte slots, a power of two of at least 2 x n_keys.  Keys must be unique
+ * A dimension table's hash table, built once and kept across requests: 8-byte
+ * entries at most a quarter full, or 16-byte slots at most half full where the
+ * groups' numbers leave an entry no room.  Keys must be unique
  * (as the reference's unique-hash join requires of its build side); groups
  * outside [0, n_groups) are kept but never aggregated.  stats (device
  * int64[2]): rows with a group out of range, rows that found no slot.

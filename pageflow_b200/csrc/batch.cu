@@ -60,28 +60,7 @@ constexpr int BT2 = 256;
 // probe rows a thread takes at a time, at four blocks a SM (62 registers): 48
 // instances 5.6 ms, 1 row at six blocks 6.4
 constexpr int BV = PF_BATCH_BV;
-// The block's own sums in shared memory: lo, hi and count of CELLS cells.  An
-// instance of few groups has all of them there, as many copies of each as fit,
-// a lane its own.  Else, where an item's first rows show groups again, its hot
-// groups (48 instances: 5.6 ms; 256 groups of 4 copies 5.8, and twice the time
-// with 54 KB of cells, whose blocks leave no L1): one is let in when it comes again before another group of its `seen`
-// entry (so one row in about a thousand or more; one that frequent would queue
-// up on its address in L2, which takes a RED every 14 clocks, while groups met
-// once an item would fill the cells), HOT_COPIES copies of each.
-constexpr int CELLS = 1024;
-constexpr int SMALL_GROUPS = 512;
-constexpr int HOT_LOG = 9, HOT = 1 << HOT_LOG, HOT_COPIES = 2;
-constexpr int SEEN_LOG = 10;
-static_assert(HOT * HOT_COPIES <= CELLS && SMALL_GROUPS <= CELLS, "cells");
-struct BatchSmem {
-  unsigned lo[CELLS], hi[CELLS], cnt[CELLS];
-  int tag[HOT];
-  int seen[1 << SEEN_LOG];
-  int inst;    // the instance whose hot groups the tags are, and
-  int cached;  // whether it has any: kept from one item to the block's next
-};
-constexpr size_t BATCH_SMEM = sizeof(BatchSmem);
-constexpr int BATCH_REPEATS = 16;   // of an item's first rows, groups met again: the cache pays
+constexpr size_t BATCH_SMEM = sizeof(OwnSums);
 constexpr int BATCH_MAX_Q = 23;     // 256 MiB tables, 0.4 full at most
 constexpr double BATCH_LOAD = 0.4;
 constexpr int SUM_CHUNK = 4096;     // groups a block of k_batch_sums adds up at a time
@@ -310,8 +289,7 @@ struct BatchArgs {
 // PACK: a row's value and 1 in one packed word, else in the slab's two.
 template <bool COMPACT, bool PACK>
 __device__ __forceinline__ void probe_rows(const Desc& D, const BatchArgs& a, unsigned epoch,
-                                           BatchSmem& S, bool cached, bool look,
-                                           long long lo, long long hi,
+                                           Own& own, long long lo, long long hi,
                                            unsigned& matched, unsigned& rows,
                                            unsigned long long& high, bool& outside) {
   unsigned long long* slab = a.slabs + 2 * D.soff;
@@ -319,21 +297,6 @@ __device__ __forceinline__ void probe_rows(const Desc& D, const BatchArgs& a, un
   const CompactTable t{reinterpret_cast<unsigned long long*>(a.tables + D.toff), D.q, D.gbits,
                        D.dbits};
   const long long bias = 1LL << (D.vbits - 1);
-  const int lane = threadIdx.x & 31;
-  // few groups: copies of each (a power of two)
-  const bool small = D.ng <= SMALL_GROUPS;
-  int lcopies = 0;
-  if (small)
-    while (lcopies < 5 && (D.ng << (lcopies + 1)) <= CELLS) ++lcopies;
-  const unsigned copy = lane & ((1u << lcopies) - 1);
-  auto add_cell = [&](unsigned c, long long v) {
-    const unsigned l = (unsigned)(unsigned long long)v;
-    const unsigned hw = (unsigned)((unsigned long long)v >> 32);
-    const unsigned old = atomicAdd(&S.lo[c], l);
-    const unsigned hc = hw + (old + l < old ? 1u : 0u);
-    if (hc) atomicAdd(&S.hi[c], hc);
-    atomicAdd(&S.cnt[c], 1u);
-  };
   for (long long i0 = lo; i0 < hi; i0 += BT2 * BV) {
     unsigned long long key[BV], hash[BV];
     long long value[BV], g[BV];
@@ -378,36 +341,10 @@ __device__ __forceinline__ void probe_rows(const Desc& D, const BatchArgs& a, un
       for (int k = 0; k < BV; ++k)
         g[k] = live[k] ? wide_lookup(D, a.tables, epoch, key[k], (unsigned)hash[k], x[k]) : -2;
     }
-    int repeats = 0;
 #pragma unroll
     for (int k = 0; k < BV; ++k) {
       matched += g[k] >= -1;
-      if (g[k] < 0) continue;
-      if (small) {
-        add_cell((unsigned)g[k] << lcopies | copy, value[k]);
-        continue;
-      }
-      const unsigned mixed = (unsigned)g[k] * 0x9E3779B1u;
-      volatile int* seen = &S.seen[mixed >> (32 - SEEN_LOG)];
-      if (cached) {
-        unsigned slot = mixed >> (32 - HOT_LOG);
-        const int t0 = *(volatile int*)&S.tag[slot], t1 = *(volatile int*)&S.tag[slot ^ 1];
-        if (t1 == (int)g[k]) slot ^= 1;
-        if (t0 == (int)g[k] || t1 == (int)g[k]) {
-          add_cell(slot * HOT_COPIES + (lane & (HOT_COPIES - 1)), value[k]);
-          continue;
-        }
-        if (*seen == (int)g[k]) {
-          if (t0 == -1) atomicCAS(&S.tag[slot], -1, (int)g[k]);
-          else if (t1 == -1) atomicCAS(&S.tag[slot ^ 1], -1, (int)g[k]);
-        } else {
-          *seen = (int)g[k];
-        }
-      } else if (look && i0 == lo) {
-        // the instance's first rows here: how often a group comes again
-        repeats += *seen == (int)g[k];
-        *seen = (int)g[k];
-      }
+      if (g[k] < 0 || own.add((unsigned)g[k], value[k], i0 == lo)) continue;
       if (PACK) {
         const unsigned long long v = (unsigned long long)(value[k] + bias);
         outside |= v >> D.vbits != 0;
@@ -419,44 +356,9 @@ __device__ __forceinline__ void probe_rows(const Desc& D, const BatchArgs& a, un
         atomicAdd(&slab[2 * (unsigned long long)g[k] + 1], 1ULL);
       }
     }
-    if (look && i0 == lo && !small) {
-      cached = __syncthreads_count(repeats > 0) >= BATCH_REPEATS;
-      if (threadIdx.x == 0) S.cached = cached;
-    }
+    if (i0 == lo) own.after_first();
   }
-  __syncthreads();
-  // the item's own sums into the slab, and emptied
-  if (small) {
-    for (int g0 = threadIdx.x; g0 < (int)D.ng; g0 += BT2) {
-      unsigned long long sum = 0, n = 0;
-      for (int j = 0; j < 1 << lcopies; ++j) {
-        const int c = g0 << lcopies | ((j + lane) & ((1 << lcopies) - 1));
-        sum += (unsigned long long)S.hi[c] << 32 | S.lo[c];
-        n += S.cnt[c];
-        S.lo[c] = S.hi[c] = S.cnt[c] = 0;
-      }
-      if (n) {
-        atomicAdd(&slab[2 * g0], sum);
-        atomicAdd(&slab[2 * g0 + 1], n);
-      }
-    }
-  } else if (cached) {
-    for (int i = threadIdx.x; i < HOT; i += BT2) {
-      const int g0 = S.tag[i];
-      if (g0 < 0) continue;
-      unsigned long long sum = 0, n = 0;
-      for (int j = 0; j < HOT_COPIES; ++j) {
-        const int c = i * HOT_COPIES + ((j + lane) & (HOT_COPIES - 1));
-        sum += (unsigned long long)S.hi[c] << 32 | S.lo[c];
-        n += S.cnt[c];
-        S.lo[c] = S.hi[c] = S.cnt[c] = 0;
-      }
-      if (!n) continue;
-      atomicAdd(&slab[2 * (unsigned long long)g0], sum);
-      atomicAdd(&slab[2 * (unsigned long long)g0 + 1], n);
-    }
-  }
-  __syncthreads();
+  own.flush(slab);
 }
 
 // SECOND: the instances to be run again, two words a group, 16-byte slots.
@@ -472,10 +374,8 @@ __global__ void __launch_bounds__(BT2, PF_BATCH_MINB) k_batch(BatchArgs a) {
   const long long ni = h->n_items;
   unsigned long long bad_group = 0, overflow = 0;
   extern __shared__ __align__(16) unsigned char batch_smem[];
-  BatchSmem& S = *reinterpret_cast<BatchSmem*>(batch_smem);
-  for (int i = threadIdx.x; i < CELLS; i += BT2) S.lo[i] = S.hi[i] = S.cnt[i] = 0;
-  if (threadIdx.x == 0) S.inst = -1;
-  for (int i = threadIdx.x; i < 1 << SEEN_LOG; i += BT2) S.seen[i] = -1;
+  OwnSums& S = *reinterpret_cast<OwnSums*>(batch_smem);
+  own_init(S);
   // Items are taken in increasing order and an item waits only for items
   // before it, so the smallest unfinished item is always some block's
   // current item with nothing left to wait for: the launch progresses.
@@ -528,30 +428,21 @@ __global__ void __launch_bounds__(BT2, PF_BATCH_MINB) k_batch(BatchArgs a) {
       }
       __syncthreads();
       if (!ok_s) continue;
-      const bool look = S.inst != inst;
-      const bool cached = !look && S.cached;
-      if (look) {
-        for (int i = threadIdx.x; i < HOT; i += BT2) S.tag[i] = -1;
-        __syncthreads();  // every thread has read S.inst
-        if (threadIdx.x == 0) {
-          S.inst = inst;
-          S.cached = 0;
-        }
-        __syncthreads();
-      }
+      Own own(S);
+      own.begin(inst, D.ng);
       const long long lo = (local - D.nbi) * D.pitem, hi = min(D.np, lo + D.pitem);
       unsigned matched = 0, rows = 0;
       unsigned long long high = 0;
       bool outside = false;
       const bool pack = !SECOND && !(flags & WIDE_SUMS);
       if (compact && pack)
-        probe_rows<true, true>(D, a, epoch, S, cached, look, lo, hi, matched, rows, high, outside);
+        probe_rows<true, true>(D, a, epoch, own, lo, hi, matched, rows, high, outside);
       else if (compact)
-        probe_rows<true, false>(D, a, epoch, S, cached, look, lo, hi, matched, rows, high, outside);
+        probe_rows<true, false>(D, a, epoch, own, lo, hi, matched, rows, high, outside);
       else if (pack)
-        probe_rows<false, true>(D, a, epoch, S, cached, look, lo, hi, matched, rows, high, outside);
+        probe_rows<false, true>(D, a, epoch, own, lo, hi, matched, rows, high, outside);
       else
-        probe_rows<false, false>(D, a, epoch, S, cached, look, lo, hi, matched, rows, high, outside);
+        probe_rows<false, false>(D, a, epoch, own, lo, hi, matched, rows, high, outside);
       // the item's counts, one atomic each
       unsigned long long m = __reduce_add_sync(FULL, matched), r = __reduce_add_sync(FULL, rows);
       for (int o = 16; o; o >>= 1) high += __shfl_xor_sync(FULL, high, o);

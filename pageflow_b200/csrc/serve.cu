@@ -2,17 +2,18 @@
 // dimension tables, folded into persistent launches.
 //
 // A dimension table's hash table is built once (pf_dim_build) and stays in
-// HBM across requests: 16-byte slots {key, OCCUPIED | group}, a power of two
-// of at least twice its keys, linear probing from the multiply-shift of the
-// key's mix64.  A slot is claimed by a CAS of its second word from zero, then
-// its key is stored; probes run in later launches only.
+// HBM across requests.  After a 256-byte head it has a compact table
+// (compact.cuh) at most a quarter full, or, where the groups' numbers leave an
+// entry no room or the keys' hashes crowd it, 16-byte slots {key, OCCUPIED |
+// group}, at most half full, linear probing from the key's mix64; the head says
+// which.  Probes run in later launches only.
 //
 // pf_serve_run runs one launch over a list of requests, each a range of its
 // probe rows [row_begin, row_end) and, for a request's last launch, its
 // finish.  Work items, request by request in the order given:
 //   probe items   PROBE_ROWS rows each: keep date in [lo, hi), look the FK up,
-//                 add (value, 1) into the request's (sum, count) slab with
-//                 warp-combined REDs
+//                 add (value, 1) into the block's own sums (agg.cuh) or the
+//                 request's (sum, count) slab
 //   count items   (finish) GROUP_CHUNK groups each: occupied groups, after
 //                 the request's probe items of this launch are done
 //   emit items    (finish) the chunk's occupied groups in ascending order at
@@ -29,29 +30,14 @@
 #include <map>
 
 #include "agg.cuh"
+#include "compact.cuh"
 
 namespace pf {
 namespace {
 
 constexpr int ST = 256;
-#ifndef PF_SERVE_SV
-#define PF_SERVE_SV 2
-#endif
-// 1: the probe loop loads the next round's dates while this round runs;
-// 2: its keys too, filtered or not (the kernel is bound by its dependent
-// loads, not by bytes: with 2 rows a thread, 91.1 against 85.4 G rows/s for
-// dates only at 4 rows a thread, saturated)
-#ifndef PF_SERVE_PIPE
-#define PF_SERVE_PIPE 2
-#endif
-constexpr int SV = PF_SERVE_SV;  // probe rows a thread keeps in flight
-// 1: probe items add through the block's group cache (agg.cuh), flushed at
-// the item's end; 0: hot_add into the slab directly.
-#ifndef PF_SERVE_CACHE
-#define PF_SERVE_CACHE 1
-#endif
-constexpr size_t SERVE_CACHE_SMEM = PF_SERVE_CACHE ? sizeof(GroupCache) : 0;
-constexpr long long PROBE_ROWS = 16384;
+constexpr int DV = 8;  // dates a lane reads at a time
+constexpr long long PROBE_ROWS = 16384;  // at most 65536: a list's offsets are 16 bits
 constexpr long long GROUP_CHUNK = 16384;
 constexpr long long MAX_CHUNKS = 256;  // groups <= 4M a request
 constexpr unsigned WAIT_LIMIT = 1u << 22;
@@ -68,36 +54,78 @@ __device__ __forceinline__ unsigned long long dim_first_slot(uint64_t h, int log
   return h >> (64 - logcap);
 }
 
+// A dimension table's first 256 bytes.
+struct DimHead {
+  int compact;  // 1: a compact table, 0: 16-byte slots
+  int q, gbits, dbits;
+  int logcap;   // 16-byte slots, log2
+  int crowded;  // the compact table took not every key
+  int pad[58];
+};
+static_assert(sizeof(DimHead) == 256, "the slots start on a 256-byte boundary");
+
+// The table as a lookup takes it.
+struct DimTable {
+  const unsigned long long* slots;
+  int compact, q, gbits, dbits, logcap;
+};
+
+__global__ void k_dim_head(DimHead* h, DimHead v) {
+  if (threadIdx.x == 0) *h = v;
+}
+
+__device__ __forceinline__ bool wide_dim_insert(DimSlot* table, int logcap,
+                                                unsigned long long key, unsigned long long v) {
+  const unsigned long long mask = (1ULL << logcap) - 1;
+  unsigned long long s = dim_first_slot(mix64(key), logcap);
+  for (unsigned long long probes = 0; probes <= mask; ++probes) {
+    if (atomicCAS(&table[s].val, 0ULL, v) == 0ULL) {
+      table[s].key = key;
+      return true;
+    }
+    s = (s + 1) & mask;
+  }
+  return false;
+}
+
+// AGAIN: 16-byte slots, where the compact table (cleared by k_dim_clear) did
+// not take every key.
+template <bool AGAIN>
 __global__ void __launch_bounds__(256) k_dim_build(const long long* __restrict__ keys,
                                                    const int* __restrict__ groups, long long n,
-                                                   long long n_groups, DimSlot* table,
-                                                   int logcap,
+                                                   long long n_groups, DimHead* head,
                                                    unsigned long long* __restrict__ stats) {
-  const unsigned long long mask = (1ULL << logcap) - 1;
+  const DimHead h = *head;
+  if (AGAIN && !h.crowded) return;
+  unsigned long long* slots = reinterpret_cast<unsigned long long*>(head + 1);
+  const CompactTable t{slots, h.q, h.gbits, h.dbits};
   unsigned long long bad = 0, overflow = 0;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
-    const unsigned long long key = (unsigned long long)keys[i];
+    const long long key = keys[i];
     const int g = groups[i];
-    unsigned long long v = OCCUPIED | (unsigned long long)(unsigned)g;
-    if (g < 0 || (long long)g >= n_groups) {
-      v = OCCUPIED | NO_GROUP;
-      ++bad;
+    const bool in = g >= 0 && (long long)g < n_groups;
+    if (!AGAIN) bad += !in;
+    if (!AGAIN && h.compact) {
+      if (!ct_insert(t, key, in ? g : -1)) head->crowded = 1;
+    } else {
+      overflow += !wide_dim_insert(reinterpret_cast<DimSlot*>(slots), h.logcap,
+                                   (unsigned long long)key,
+                                   OCCUPIED | (in ? (unsigned long long)(unsigned)g : NO_GROUP));
     }
-    unsigned long long s = dim_first_slot(mix64(key), logcap);
-    bool done = false;
-    for (unsigned long long probes = 0; probes <= mask; ++probes) {
-      if (atomicCAS(&table[s].val, 0ULL, v) == 0ULL) {
-        table[s].key = key;
-        done = true;
-        break;
-      }
-      s = (s + 1) & mask;
-    }
-    overflow += !done;
   }
   if (bad) atomicAdd(&stats[0], bad);
   if (overflow) atomicAdd(&stats[1], overflow);
+}
+
+__global__ void __launch_bounds__(256) k_dim_clear(DimHead* head) {
+  if (!head->crowded) return;
+  const unsigned long long words = 2ULL << head->logcap;
+  unsigned long long* slots = reinterpret_cast<unsigned long long*>(head + 1);
+  for (unsigned long long i = (unsigned long long)blockIdx.x * 256 + threadIdx.x; i < words;
+       i += (unsigned long long)gridDim.x * 256)
+    slots[i] = 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) head->compact = 0;
 }
 
 struct SReq {
@@ -105,7 +133,7 @@ struct SReq {
   const int* date;
   const long long* value;
   long long r0, r1;
-  const DimSlot* table;
+  const DimHead* table;
   long long ng;
   unsigned long long* slab;
   long long* okeys;
@@ -115,8 +143,6 @@ struct SReq {
   unsigned long long* done;  // device alias of the pinned done word, or null
   long long item0, npi, nch;  // first item; probe items; finish chunks (0: no finish)
   int lo, hi;
-  int logcap;
-  int pad;
 };
 
 struct SCounters {
@@ -174,13 +200,100 @@ __device__ __forceinline__ long long block_sum(long long v, long long* red) {
   return t;
 }
 
-__global__ void __launch_bounds__(ST) k_serve(SHead* h, const SReq* __restrict__ reqs,
-                                              SCounters* cnt, long long* chunk_counts,
-                                              unsigned long long* stats) {
+// A key's group in the dimension table: -2 not there, -1 there without a group.
+__device__ __forceinline__ long long dim_lookup(const DimTable& t, unsigned long long key) {
+  if (t.compact) {
+    const CompactTable c{const_cast<unsigned long long*>(t.slots), t.q, t.gbits, t.dbits};
+    bool more;
+    const unsigned long long hash = ct_hash((long long)key), want = ct_want(c, hash);
+    unsigned long long e = ct_among(c, ct_load(ct_home(c, hash)), want, &more);
+    if (more) e = ct_walk(c, hash, want);
+    return e == CT_EMPTY ? -2 : ct_group(c, e);
+  }
+  const unsigned long long mask = (1ULL << t.logcap) - 1;
+  unsigned long long s = dim_first_slot(mix64(key), t.logcap);
+  for (unsigned long long probes = 0; probes <= mask; ++probes) {
+    const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(t.slots + 2 * s);
+    if (x.y == 0) return -2;
+    if (x.x == key) {
+      const unsigned long long go = x.y & ~OCCUPIED;
+      return go == NO_GROUP ? -1 : (long long)go;
+    }
+    s = (s + 1) & mask;
+  }
+  return -2;
+}
+
+// Probe rows [lo, hi) of a request.  A warp reads its dates, DV a lane and the
+// next step's while this one runs, and keeps the offsets of the rows that pass
+// in its own list: a quarter of them pass, and warps that look up and add with
+// a quarter of their lanes were the whole time (487M rows: 4350 us, so 3200).
+// It takes 32 off the list's end while that has them (at the item's end, and
+// where the block has yet to see the request's groups, whatever is there):
+// key and value, then the home sector, then the sums.  (Three takes in flight
+// at a time, or two rows a lane: no faster.)
+__device__ __forceinline__ void serve_rows(const SReq& R, const DimTable& t, Own& own,
+                                           unsigned short* list, long long lo, long long hi,
+                                           unsigned& kept, unsigned& matched) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned below = (1u << lane) - 1;
+  const int rows = (int)(hi - lo);
+  const int steps = (rows + ST * DV - 1) / (ST * DV);
+  const int* date = R.date + lo;
+  const long long* fk = R.fk + lo;
+  const long long* val = R.value + lo;
+  unsigned long long* slab = R.slab;
+  const int dlo = R.lo, dhi = R.hi;
+  int n = 0;
+  int dt[DV];
+  int at = warp * 32 * DV + lane;
+#pragma unroll
+  for (int k = 0; k < DV; ++k) dt[k] = at + 32 * k < rows ? __ldcs(date + at + 32 * k) : INT_MIN;
+  for (int s = 0; s < steps; ++s) {
+#pragma unroll
+    for (int k = 0; k < DV; ++k) {
+      const bool keep = at + 32 * k < rows && dt[k] >= dlo && dt[k] < dhi;
+      const unsigned m = __ballot_sync(FULL, keep);
+      if (keep) list[n + __popc(m & below)] = (unsigned short)(at + 32 * k);
+      n += __popc(m);
+      kept += keep;
+    }
+    at += ST * DV;
+#pragma unroll
+    for (int k = 0; k < DV; ++k)
+      dt[k] = at + 32 * k < rows ? __ldcs(date + at + 32 * k) : INT_MIN;
+    __syncwarp();
+    const int least = s == steps - 1 || (s == 0 && own.look) ? 1 : 32;
+    while (n >= least) {
+      const int take = min(n, 32);
+      n -= take;
+      if (lane < take) {
+        const int i = list[n + lane];
+        const unsigned long long key = (unsigned long long)__ldcs(fk + i);
+        const long long value = __ldcs(val + i);
+        const long long g = dim_lookup(t, key);
+        matched += g >= -1;
+        if (g >= 0 && !own.add((unsigned)g, value, s == 0)) {
+          atomicAdd(&slab[2 * (unsigned long long)g], (unsigned long long)value);
+          atomicAdd(&slab[2 * (unsigned long long)g + 1], 1ULL);
+        }
+      }
+      __syncwarp();
+    }
+    if (s == 0) own.after_first();
+  }
+  own.flush(slab);
+}
+
+__global__ void __launch_bounds__(ST, 4) k_serve(SHead* h,
+                                                 const SReq* __restrict__ reqs,
+                                                 SCounters* cnt, long long* chunk_counts,
+                                                 unsigned long long* stats) {
   extern __shared__ __align__(16) unsigned char serve_smem[];
-  GroupCache& gc = *reinterpret_cast<GroupCache*>(serve_smem);
-  int* first_item = reinterpret_cast<int*>(serve_smem + SERVE_CACHE_SMEM);
-  if (PF_SERVE_CACHE) cache_init(gc);
+  OwnSums& S = *reinterpret_cast<OwnSums*>(serve_smem);
+  int* first_item = reinterpret_cast<int*>(serve_smem + sizeof(OwnSums));
+  __shared__ unsigned short lists[ST / 32][32 * (DV + 1)];
+  own_init(S);
   __shared__ long long item_s;
   __shared__ int ok_s;
   __shared__ long long red[ST / 32];
@@ -189,9 +302,6 @@ __global__ void __launch_bounds__(ST) k_serve(SHead* h, const SReq* __restrict__
   const int n = h->n_req;
   for (int i = threadIdx.x; i < n; i += ST) first_item[i] = (int)reqs[i].item0;
   unsigned long long matched = 0, kept = 0;
-  long long hot = -1;  // the warp's hot group (hot_add)
-  // With PF_PREFETCH_ITEMS, thread 0 takes the block's next item while the
-  // block works on the current one (measured no faster, so off by default).
   // Items are taken in increasing order and an item waits only for items
   // before it, so the smallest unfinished item is always some block's
   // current item with nothing left to wait for: the launch progresses.
@@ -200,99 +310,21 @@ __global__ void __launch_bounds__(ST) k_serve(SHead* h, const SReq* __restrict__
     __syncthreads();
     const long long it = item_s;
     if (it >= ni) break;
-    unsigned long long next = 0;
-    if (PF_PREFETCH_ITEMS && threadIdx.x == 0) next = atomicAdd(&h->counter, 1ULL);
     const int q = request_of(first_item, n, it);
     const SReq& R = reqs[q];
     const long long local = it - R.item0;
     if (local < R.npi) {
-      // ---- probe rows, SV a thread at a time: every stage (dates, keys, first
-      // slots, values) is issued for all SV rows before any is used, so a
-      // thread keeps SV independent loads in flight
+      // ---- probe rows
       const long long lo = R.r0 + local * PROBE_ROWS, hi = min(R.r1, lo + PROBE_ROWS);
-      const unsigned long long mask = (1ULL << R.logcap) - 1;
-#if PF_SERVE_PIPE
-      // the next round's dates (and, with PF_SERVE_PIPE 2, its keys, whether
-      // the rows pass the filter or not) load while this round runs
-      int dt[SV];
-      unsigned long long kf[PF_SERVE_PIPE >= 2 ? SV : 1];
-#pragma unroll
-      for (int k = 0; k < SV; ++k) {
-        const long long i = lo + k * ST + threadIdx.x;
-        dt[k] = i < hi ? R.date[i] : INT_MIN;
-        if (PF_SERVE_PIPE >= 2) kf[k < SV ? k : 0] = i < hi ? (unsigned long long)R.fk[i] : 0ULL;
-      }
-#endif
-      for (long long i0 = lo; i0 < hi; i0 += ST * SV) {
-        bool keep[SV];
-        unsigned long long key[SV], slot[SV];
-        ulonglong2 sl[SV];
-        long long g[SV], value[SV];
-#if PF_SERVE_PIPE
-#pragma unroll
-        for (int k = 0; k < SV; ++k) {
-          keep[k] = dt[k] >= R.lo && dt[k] < R.hi;
-          if (PF_SERVE_PIPE >= 2) key[k] = keep[k] ? kf[k < SV ? k : 0] : 0ULL;
-        }
-#pragma unroll
-        for (int k = 0; k < SV; ++k) {
-          const long long i = i0 + (long long)ST * SV + k * ST + threadIdx.x;
-          dt[k] = i < hi ? R.date[i] : INT_MIN;
-          if (PF_SERVE_PIPE >= 2) kf[k < SV ? k : 0] = i < hi ? (unsigned long long)R.fk[i] : 0ULL;
-        }
-#else
-#pragma unroll
-        for (int k = 0; k < SV; ++k) {
-          const long long i = i0 + k * ST + threadIdx.x;
-          const int d = i < hi ? R.date[i] : INT_MIN;
-          keep[k] = d >= R.lo && d < R.hi;
-        }
-#endif
-#pragma unroll
-        for (int k = 0; k < (PF_SERVE_PIPE >= 2 ? 0 : SV); ++k) {
-          const long long i = i0 + k * ST + threadIdx.x;
-          key[k] = keep[k] ? (unsigned long long)R.fk[i] : 0ULL;
-        }
-#pragma unroll
-        for (int k = 0; k < SV; ++k) {
-          slot[k] = dim_first_slot(mix64(key[k]), R.logcap);
-          sl[k] = keep[k] ? *reinterpret_cast<const ulonglong2*>(R.table + slot[k])
-                          : make_ulonglong2(0ULL, 0ULL);
-        }
-#pragma unroll
-        for (int k = 0; k < SV; ++k) {
-          g[k] = -1;
-          if (!keep[k]) continue;
-          ++kept;
-          unsigned long long sk = slot[k];
-          ulonglong2 x = sl[k];
-          for (unsigned long long probes = 0; probes <= mask; ++probes) {
-            if (x.y == 0) break;
-            if (x.x == key[k]) {
-              ++matched;
-              const unsigned long long go = x.y & ~OCCUPIED;
-              if (go != NO_GROUP) g[k] = (long long)go;
-              break;
-            }
-            sk = (sk + 1) & mask;
-            x = *reinterpret_cast<const ulonglong2*>(R.table + sk);
-          }
-        }
-#pragma unroll
-        for (int k = 0; k < SV; ++k) {
-          const long long i = i0 + k * ST + threadIdx.x;
-          value[k] = g[k] >= 0 ? R.value[i] : 0;
-        }
-#pragma unroll
-        for (int k = 0; k < SV; ++k) {
-          if (PF_SERVE_CACHE) {
-            if (g[k] >= 0) cache_add(gc, R.slab, g[k], (unsigned long long)value[k], 1ULL);
-          } else {
-            hot_add(R.slab, g[k], value[k], hot);
-          }
-        }
-      }
-      if (PF_SERVE_CACHE) cache_flush(gc, R.slab);
+      const DimTable t{reinterpret_cast<const unsigned long long*>(R.table + 1),
+                       R.table->compact, R.table->q, R.table->gbits, R.table->dbits,
+                       R.table->logcap};
+      unsigned kp = 0, ma = 0;
+      Own own(S);
+      own.begin(q, R.ng);
+      serve_rows(R, t, own, lists[threadIdx.x >> 5], lo, hi, kp, ma);
+      kept += kp;
+      matched += ma;
       __syncthreads();
       if (threadIdx.x == 0) {
         __threadfence();
@@ -304,7 +336,7 @@ __global__ void __launch_bounds__(ST) k_serve(SHead* h, const SReq* __restrict__
       if (threadIdx.x == 0) ok_s = wait_zero(&cnt[q].probe_left, h, R.done);
       __syncthreads();
       if (!ok_s) {
-        if (threadIdx.x == 0) item_s = (long long)(PF_PREFETCH_ITEMS ? next : atomicAdd(&h->counter, 1ULL));
+        if (threadIdx.x == 0) item_s = (long long)atomicAdd(&h->counter, 1ULL);
         continue;
       }
       const long long g0 = c * GROUP_CHUNK, g1 = min(R.ng, g0 + GROUP_CHUNK);
@@ -322,7 +354,7 @@ __global__ void __launch_bounds__(ST) k_serve(SHead* h, const SReq* __restrict__
       if (threadIdx.x == 0) ok_s = wait_zero(&cnt[q].count_left, h, R.done);
       __syncthreads();
       if (!ok_s) {
-        if (threadIdx.x == 0) item_s = (long long)(PF_PREFETCH_ITEMS ? next : atomicAdd(&h->counter, 1ULL));
+        if (threadIdx.x == 0) item_s = (long long)atomicAdd(&h->counter, 1ULL);
         continue;
       }
       const long long* cc = chunk_counts + (long long)q * MAX_CHUNKS;
@@ -370,7 +402,7 @@ __global__ void __launch_bounds__(ST) k_serve(SHead* h, const SReq* __restrict__
       }
     }
     __syncthreads();  // every thread has read item_s
-    if (threadIdx.x == 0) item_s = (long long)(PF_PREFETCH_ITEMS ? next : atomicAdd(&h->counter, 1ULL));
+    if (threadIdx.x == 0) item_s = (long long)atomicAdd(&h->counter, 1ULL);
   }
   for (int o = 16; o; o >>= 1) {
     matched += __shfl_xor_sync(FULL, matched, o);
@@ -447,9 +479,15 @@ int serve_grid(int* grid, size_t smem) {
 
 using namespace pf;
 
+namespace {
+// 16-byte slots of a table, log2: at least twice the keys, and 256 (64 buckets).
+int dim_logcap(int64_t n_keys) {
+  return std::max(8, log2_exact(pow2_at_least((uint64_t)std::max<int64_t>(2 * n_keys, 2))));
+}
+}  // namespace
+
 extern "C" size_t pf_dim_table_bytes(int64_t n_keys) {
-  const uint64_t cap = pow2_at_least((uint64_t)std::max<int64_t>(2 * n_keys, 2));
-  return (size_t)cap * sizeof(DimSlot);
+  return sizeof(DimHead) + (sizeof(DimSlot) << dim_logcap(n_keys));
 }
 
 extern "C" int pf_dim_build(const int64_t* keys, const int32_t* groups, int64_t n_keys,
@@ -462,16 +500,39 @@ extern "C" int pf_dim_build(const int64_t* keys, const int32_t* groups, int64_t 
   const size_t need = pf_dim_table_bytes(n_keys);
   if (table_bytes < need)
     return fail(PF_ENOSPACE, "dim_build: table of %zu bytes, %zu needed", table_bytes, need);
-  const uint64_t cap = need / sizeof(DimSlot);
+  // the same bytes as a compact table: four entries for two slots
+  DimHead hd{};
+  hd.logcap = dim_logcap(n_keys);
+  hd.q = hd.logcap - 1;
+  hd.gbits = bits_of((unsigned long long)n_groups + 1);
+  // its loads are 32 bytes
+  hd.compact = hd.gbits < 32 && hd.q - hd.gbits >= 3 && ((uintptr_t)table & 31) == 0;
+  hd.dbits = hd.compact ? std::min(6, hd.q - hd.gbits) : 0;
+  DimHead* head = (DimHead*)table;
   PF_CUDA(cudaMemsetAsync(table, 0, need, st));
   PF_CUDA(cudaMemsetAsync(stats, 0, 2 * sizeof(int64_t), st));
+  {
+    PF_KERNEL("k_dim_head", st);
+    k_dim_head<<<1, 32, 0, st>>>(head, hd);
+  }
+  PF_LAUNCH("k_dim_head");
   const unsigned grid = (unsigned)std::max<long long>(
       1, std::min<long long>((n_keys + 255) / 256, (long long)sm_count() * 16));
   {
     PF_KERNEL("k_dim_build", st);
-    k_dim_build<<<grid, 256, 0, st>>>((const long long*)keys, groups, n_keys, n_groups,
-                                      (DimSlot*)table, log2_exact(cap),
-                                      (unsigned long long*)stats);
+    k_dim_build<false><<<grid, 256, 0, st>>>((const long long*)keys, groups, n_keys, n_groups,
+                                             head, (unsigned long long*)stats);
+  }
+  PF_LAUNCH("k_dim_build");
+  if (hd.compact) {
+    {
+      PF_KERNEL("k_dim_clear", st);
+      k_dim_clear<<<sm_count() * 4, 256, 0, st>>>(head);
+    }
+    PF_LAUNCH("k_dim_clear");
+    PF_KERNEL("k_dim_build", st);
+    k_dim_build<true><<<grid, 256, 0, st>>>((const long long*)keys, groups, n_keys, n_groups,
+                                            head, (unsigned long long*)stats);
   }
   PF_LAUNCH("k_dim_build");
   return ok();
@@ -522,8 +583,7 @@ extern "C" int pf_serve_run(const pf_serve_request* reqs, int n, void* workspace
     R.value = (const long long*)x.value;
     R.r0 = x.row_begin;
     R.r1 = x.row_end;
-    R.table = (const DimSlot*)x.table;
-    R.logcap = log2_exact(pf_dim_table_bytes(x.n_keys) / sizeof(DimSlot));
+    R.table = (const DimHead*)x.table;
     R.ng = x.n_groups;
     R.slab = (unsigned long long*)x.slab;
     R.okeys = (long long*)x.out_keys;
@@ -550,13 +610,13 @@ extern "C" int pf_serve_run(const pf_serve_request* reqs, int n, void* workspace
   H->n_req = n;
   H->error = 0;
   int grid = 0;
-  if (int rc = serve_grid(&grid, SERVE_CACHE_SMEM + sizeof(int) * n)) return rc;
+  if (int rc = serve_grid(&grid, sizeof(OwnSums) + sizeof(int) * n)) return rc;
   PF_CUDA(cudaMemcpyAsync(l.head, img, bytes, cudaMemcpyHostToDevice, st));
   PF_CUDA(cudaEventRecord(stg->ev, st));
   stg->pending = true;
   {
     PF_KERNEL("k_serve", st);
-    k_serve<<<grid, ST, SERVE_CACHE_SMEM + sizeof(int) * n, st>>>(l.head, l.reqs, l.cnt, l.chunks,
+    k_serve<<<grid, ST, sizeof(OwnSums) + sizeof(int) * n, st>>>(l.head, l.reqs, l.cnt, l.chunks,
                                                 (unsigned long long*)stats);
   }
   PF_LAUNCH("k_serve");
