@@ -670,7 +670,8 @@ int pf_dim_build(const int64_t* keys, const int32_t* groups, int64_t n_keys, int
  * launch.  slab: device int64[2 x n_groups] (sum, count) pairs, zero before
  * the request's first launch, accumulated across its launches.  In the
  * launch with finish = 1 the occupied groups are written in ascending order
- * (out_keys / out_sums / out_counts, n_groups rows each; out_n the count)
+ * (out_keys / out_sums / out_counts, n_groups rows each; out_n the count; device
+ * memory or pinned host memory, which is complete when *done says so)
  * and the pinned host word *done (may be NULL) is set to 1 + groups once
  * they are written (all ones if the launch gave up on it).  n_groups <=
  * 4,194,304.
@@ -703,6 +704,8 @@ typedef struct {
  * it serves the serving workload (requests against resident tables).
  */
 size_t pf_serve_workspace(int max_requests);
+/* Zeroes n slabs (n_groups pairs each, on 16 bytes) in one launch per 128. */
+int pf_serve_clear(int64_t* const* slabs, const int64_t* n_groups, int n, void* stream);
 int pf_serve_run(const pf_serve_request* requests, int n, void* workspace,
                  size_t workspace_bytes, int64_t* stats, void* stream);
 

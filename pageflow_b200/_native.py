@@ -123,6 +123,7 @@ _SIGS = {
     "pf_paged_scan": (_int, [_vp, _vp, _i64, _int, _vp, _i64, _i64, _int, _int, _i64, _i64,
                              _int, _int, _int, _vp, _i64, _vp, _vp, _vp, _sz, _vp]),
     "pf_dim_table_bytes": (_sz, [_i64]),
+    "pf_serve_clear": (_int, [_vp, _vp, _int, _vp]),
     "pf_dim_build": (_int, [_vp, _vp, _i64, _i64, _vp, _sz, _vp, _vp]),
     "pf_serve_workspace": (_sz, [_int]),
     "pf_serve_run": (_int, [_vp, _int, _vp, _sz, _vp, _vp]),

@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(ST, 4) k_serve(SHead* h,
       }
       __syncthreads();
       if (threadIdx.x == 0) {
-        __threadfence();
+        __threadfence_system();  // the outputs may be host memory
         if (atomicSub(&cnt[q].emit_left, 1u) == 1u) {
           *R.on = total;
           __threadfence_system();
@@ -416,6 +416,21 @@ __global__ void __launch_bounds__(ST, 4) k_serve(SHead* h,
 
 __global__ void k_serve_error(const SHead* h, unsigned long long* stats) {
   if (threadIdx.x == 0 && h->error) stats[1] |= h->error;
+}
+
+// Slabs to be cleared in one launch: 32 of them in 2 us.  A launch each, and an
+// array view for each pointer, kept a burst's first rows waiting for 2.5 ms.
+constexpr int CLEAR_SLABS = 128;
+struct ClearList {
+  ulonglong2* slab[CLEAR_SLABS];
+  long long ng[CLEAR_SLABS];
+};
+
+__global__ void __launch_bounds__(256) k_serve_clear(const __grid_constant__ ClearList c) {
+  ulonglong2* slab = c.slab[blockIdx.y];
+  const long long ng = c.ng[blockIdx.y];
+  for (long long g = (long long)blockIdx.x * 256 + threadIdx.x; g < ng; g += 256LL * gridDim.x)
+    slab[g] = make_ulonglong2(0, 0);
 }
 
 struct ServeLayout {
@@ -542,6 +557,32 @@ extern "C" size_t pf_serve_workspace(int max_requests) {
   Arena a(nullptr, 0);
   serve_layout(a, max_requests);
   return a.used + 256;
+}
+
+extern "C" int pf_serve_clear(int64_t* const* slabs, const int64_t* n_groups, int n,
+                              void* stream) {
+  cudaStream_t st = (cudaStream_t)stream;
+  if (n < 1 || !slabs || !n_groups) return fail(PF_EINVAL, "serve_clear: bad arguments");
+  for (int i = 0; i < n; ++i)
+    if (!slabs[i] || ((uintptr_t)slabs[i] & 15) || n_groups[i] < 1)
+      return fail(PF_EINVAL, "serve_clear: slab %d: null, not on 16 bytes or empty", i);
+  for (int i0 = 0; i0 < n; i0 += CLEAR_SLABS) {
+    ClearList c{};
+    const int m = std::min(n - i0, CLEAR_SLABS);
+    long long most = 0;
+    for (int i = 0; i < m; ++i) {
+      c.slab[i] = (ulonglong2*)slabs[i0 + i];
+      c.ng[i] = n_groups[i0 + i];
+      most = std::max(most, c.ng[i]);
+    }
+    const unsigned gx = (unsigned)std::min<long long>((most + 1023) / 1024, sm_count());
+    {
+      PF_KERNEL("k_serve_clear", st);
+      k_serve_clear<<<dim3(gx, m), 256, 0, st>>>(c);
+    }
+    PF_LAUNCH("k_serve_clear");
+  }
+  return ok();
 }
 
 extern "C" int pf_serve_run(const pf_serve_request* reqs, int n, void* workspace,

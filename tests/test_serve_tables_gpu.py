@@ -1,5 +1,6 @@
 """Dimension tables of every form and groups of every kind of sum: requests
 against the oracle, whole numbers equal."""
+import ctypes
 import dataclasses
 
 import numpy as np
@@ -96,3 +97,20 @@ def test_groups_outside_are_counted_once():
         check(L.pf_dim_build(ptr(k), ptr(g), 3000, 2990, ptr(t), tb, ptr(stats),
                              stream_of(dev)), "dim_build")
         assert stats.tolist() == [10, 0]
+
+
+def test_slabs_are_cleared_and_their_neighbours_kept():
+    """More slabs than one launch takes, of sizes around a block's and a grid's
+    share, each with a guard pair behind it."""
+    dev = torch.device("cuda", 0)
+    L = lib()
+    sizes = [1, 2, 255, 256, 257, 1023, 1025, 40_000] * 33
+    ends = np.cumsum([s + 1 for s in sizes])
+    pool = torch.full((int(ends[-1]), 2), -1, dtype=torch.int64, device=dev)
+    starts = ends - np.array(sizes) - 1
+    at = (ctypes.c_void_p * len(sizes))(*[pool.data_ptr() + 16 * int(a) for a in starts])
+    ng = (ctypes.c_int64 * len(sizes))(*sizes)
+    check(L.pf_serve_clear(at, ng, len(sizes), stream_of(dev)), "serve_clear")
+    want = np.zeros((int(ends[-1]), 2), np.int64)
+    want[ends - 1] = -1
+    assert np.array_equal(pool.cpu().numpy(), want)
