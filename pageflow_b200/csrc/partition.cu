@@ -11,15 +11,16 @@
 // at work at one time are neighbours:
 //
 //   k_hist      one histogram row per chunk, hist[chunk][b] (coalesced)
-//   k_scan      per bucket, exclusive offsets over the chunks (k_scan_sum,
-//               k_scan_groups, k_scan_write: the chunks in 64 groups, each
-//               group's sums, a scan over the groups, the offsets)
-//   k_bases     bucket counts, each row-width class's padded bucket starts and
-//               total, all written into the caller's pinned host_out through
-//               its device alias; an overflow check against n_valid
+//   k_scan      per bucket, exclusive offsets over the chunks, in 64 groups:
+//               k_scan_sum, each group's sums; k_scan_write, the offsets
+//   k_bases     between the two: a scan over the groups, bucket counts, each
+//               row-width class's padded bucket starts and total, written into
+//               the caller's pinned host_out through its device alias; an
+//               overflow check against n_valid
 //   k_scatter   per sub-tile: warp-match ranks (stable), the sub-tile's bucket
 //               runs, the rows staged in shared memory in bucket order, every
-//               column and the gidx written as coalesced bucket runs
+//               column and the gidx written as coalesced bucket runs; with
+//               few buckets the same a warp (k_scatter_few)
 //
 // Mask prologues (same chunking as the main walk):
 //   compacted-input  k_mask_count + k_scan_chunks: each chunk's first row in
@@ -315,10 +316,10 @@ __global__ void __launch_bounds__(PT) k_hist_plain(Params p) {
 
 // The chunks are cut into SCAN_G groups; block (x, y) owns buckets
 // [32x, 32x + 32) (lane = bucket) of group y, its warps splitting the group's
-// chunks.  k_scan_sum: each group's rows a bucket; k_scan_groups: per bucket,
-// each group's first row (exclusive over the groups) and counts[b], the
-// bucket's rows; k_scan_write: every chunk's exclusive offset into hist.
-constexpr int SCAN_G = 64;
+// chunks.  k_scan_sum: each group's rows a bucket; k_bases: per bucket, each
+// group's first row (exclusive over the groups) and the bucket's rows;
+// k_scan_write: every chunk's exclusive offset into hist.
+constexpr int SCAN_G = 64;  // two a lane in k_bases
 
 __device__ __forceinline__ void scan_range(int nchunks, int cg, int& c0, int& c1) {
   const int g0 = blockIdx.y * cg, g1 = min(nchunks, g0 + cg);
@@ -346,20 +347,6 @@ __global__ void __launch_bounds__(PT) k_scan_sum(const int* __restrict__ hist, i
     for (int j = 0; j < PW; ++j) t += part[j][lane];
     gsum[(long long)blockIdx.y * B + b] = t;
   }
-}
-
-__global__ void k_scan_groups(long long* __restrict__ gsum, int B, long long* __restrict__ counts,
-                              const int* flags) {
-  if (flags[0]) return;
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= B) return;
-  long long run = 0;
-  for (int g = 0; g < SCAN_G; ++g) {
-    const long long t = gsum[(long long)g * B + b];
-    gsum[(long long)g * B + b] = run;
-    run += t;
-  }
-  counts[b] = run;
 }
 
 __global__ void __launch_bounds__(PT) k_scan_write(int* __restrict__ hist, int nchunks, int B,
@@ -403,10 +390,12 @@ struct Rpu {
   long long v[MAXCLS];
 };
 
-// One block of 1024.  host[b] = count b; host[B + cls] = the class's padded
+// One block of 1024.  The groups' first rows, a warp a bucket (one thread a
+// bucket, in a launch of its own, took 10 us for its chain of loads); then
+// host[b] = count b; host[B + cls] = the class's padded
 // total; host[B + MAXCLS] = the prologue's kept rows or -1.  Flag 1 when the
 // counts total more than n_valid.
-__global__ void __launch_bounds__(1024) k_bases(const long long* __restrict__ counts, int B,
+__global__ void __launch_bounds__(1024) k_bases(long long* gsum, long long* counts, int B,
                                                 Rpu rpu, int ncls, long long* __restrict__ bases,
                                                 long long* host, int* flags, long long n_valid,
                                                 const long long* prologue_total) {
@@ -416,6 +405,22 @@ __global__ void __launch_bounds__(1024) k_bases(const long long* __restrict__ co
   const int per = (B + 1023) / 1024;
   const int st = tid * per;
   const bool bad = flags[0] != 0;
+  for (int b = w; b < B && !bad; b += 32) {
+    const long long x0 = gsum[(long long)lane * B + b], x1 = gsum[(long long)(32 + lane) * B + b];
+    long long i0 = x0, i1 = x1;
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long y0 = __shfl_up_sync(FULL, i0, o), y1 = __shfl_up_sync(FULL, i1, o);
+      if (lane >= o) {
+        i0 += y0;
+        i1 += y1;
+      }
+    }
+    i1 += __shfl_sync(FULL, i0, 31);
+    gsum[(long long)lane * B + b] = i0 - x0;
+    gsum[(long long)(32 + lane) * B + b] = i1 - x1;
+    if (lane == 31) counts[b] = i1;
+  }
+  __syncthreads();
   for (int cls = -1; cls < ncls; ++cls) {
     // cls -1: the raw counts (their total); else the class's padded sizes
     const long long r = cls < 0 ? 1 : rpu.v[cls];
@@ -643,7 +648,7 @@ __global__ void __launch_bounds__(PT, PF_PART_PLAIN_MINB) k_scatter_plain(Params
   const int B = p.B;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const long long t0 = (long long)blockIdx.x * SUB;
-  for (int x = tid; x < PW * BMAX; x += PT) (&S.wh[0][0])[x] = 0;
+  for (int x = tid; x < PW << p.logB; x += PT) S.wh[x >> p.logB][x & (B - 1)] = 0;
   bool valid[PITEMS];
   int bk[PITEMS];
   unsigned long long v[PITEMS];
@@ -766,6 +771,312 @@ __global__ void __launch_bounds__(PT, PF_PART_PLAIN_MINB) k_scatter_plain(Params
     const int e = t * PT + tid;
     if (e < tvalid) p.gout[gbg[eb[t]] + e] = p.goff + t0 + S.srow[e];
   }
+}
+
+// The scatter for few buckets: no compacted column, one sub-tile a chunk,
+// every column one word a row and aligned.  A warp's 256 rows are long enough a
+// run in every bucket, so the warps stage and write their own: one barrier a
+// tile, for their starts in the tile's runs, where a block that stages its 2048
+// rows together takes 16.  A lane has eight rows in a row, loaded as one or two
+// vectors, and their buckets' counts as eight fields of a word, which the warp
+// adds up as such: the kernel is bound by its instructions as much as by its
+// bytes.  (16.8M rows of 8 + 8 + 4 + 1 bytes and the gidx into 8 buckets: 178
+// us, 4.7 TB/s; staged by the block 265, a row a lane with a ballot a bit of the
+// bucket 228; three or five blocks a SM 177 and 196.  The whole call 348 -> 247
+// us, under a mask of half the rows 644 -> 246.)
+// MODE 0: every row, 1: those of a mask, 2: those of src (their numbers).
+constexpr int FB = 8;
+constexpr int FT = 256, FW = FT / 32, FI = SUB / FT, FSEG = 32 * FI;
+static_assert(FI == 8 && FSEG == 256, "eight rows a lane, a row of a segment a byte");
+
+struct FewWarp {
+  unsigned long long stage[FSEG];
+  unsigned short meta[FSEG];      // staged row: bucket << 8 | row of the segment
+  unsigned dst[MAXCLS][FB];       // bucket's staged row 0 would land there (mod 2^32)
+  unsigned char first[FB];        // bucket's first staged row (256: 0, it has none)
+};
+
+// Eight rows of a column at its row i (a multiple of 8), as 8-byte values; where
+// not ALL, those of the set bits of `live`, the vectors that have one.
+template <bool ALL>
+__device__ __forceinline__ void few_rows(const unsigned char* in, int rb, long long i,
+                                         unsigned live, unsigned long long (&v)[FI]) {
+  const unsigned char* at = in + i * rb;
+  if (rb == 8) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (ALL || (live >> 4 * h & 15))
+        asm("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];"
+            : "=l"(v[4 * h]), "=l"(v[4 * h + 1]), "=l"(v[4 * h + 2]), "=l"(v[4 * h + 3])
+            : "l"(at + 32 * h));
+  } else if (ALL || live) {
+    if (rb == 4) {
+      unsigned x[FI];
+      asm("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+          : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]), "=r"(x[4]), "=r"(x[5]), "=r"(x[6]),
+            "=r"(x[7])
+          : "l"(at));
+#pragma unroll
+      for (int k = 0; k < FI; ++k) v[k] = x[k];
+    } else if (rb == 2) {
+      const uint4 x = *reinterpret_cast<const uint4*>(at);
+      const unsigned y[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+      for (int k = 0; k < FI; ++k) v[k] = y[k / 2] >> 16 * (k & 1) & 0xffff;
+    } else {
+      const uint2 x = *reinterpret_cast<const uint2*>(at);
+#pragma unroll
+      for (int k = 0; k < FI; ++k) v[k] = (k < 4 ? x.x : x.y) >> 8 * (k & 3) & 0xff;
+    }
+  }
+}
+
+// The same of the rows that a list names, or of a ragged end.
+__device__ __forceinline__ void few_gather(const unsigned char* in, int rb, const int (&at)[FI],
+                                           unsigned live, unsigned long long (&v)[FI]) {
+#pragma unroll
+  for (int k = 0; k < FI; ++k) {
+    if (!(live >> k & 1)) continue;
+    const unsigned char* x = in + (long long)at[k] * rb;
+    v[k] = rb == 8   ? *reinterpret_cast<const unsigned long long*>(x)
+           : rb == 4 ? *reinterpret_cast<const unsigned*>(x)
+           : rb == 2 ? *reinterpret_cast<const unsigned short*>(x)
+                     : *x;
+  }
+}
+
+// Which of the lane's eight rows from i on are there; MODE 2: their numbers.
+// ALL: the tile is full.
+template <int MODE, bool ALL>
+__device__ __forceinline__ unsigned few_live(const Params& p, long long i, int (&at)[FI]) {
+  unsigned live = 255;
+  if (!ALL) {
+    const long long left = p.ndom - i;
+    live = left >= FI ? 255u : left > 0 ? (1u << left) - 1 : 0u;
+  }
+  if (MODE == 1) {
+    unsigned long long m = 0;
+    if (ALL) {
+      m = *reinterpret_cast<const unsigned long long*>(p.mask + i);
+    } else {
+#pragma unroll
+      for (int k = 0; k < FI; ++k)
+        if (live >> k & 1) m |= (unsigned long long)p.mask[i + k] << 8 * k;
+    }
+#pragma unroll
+    for (int k = 0; k < FI; ++k)
+      if (!(m >> 8 * k & 0xff)) live &= ~(1u << k);
+  }
+  if (MODE == 2 || !ALL) {
+#pragma unroll
+    for (int k = 0; k < FI; ++k)
+      at[k] = !(live >> k & 1) ? 0 : MODE == 2 ? p.src[i + k] : (int)(i + k);
+  }
+  return live;
+}
+
+template <int MODE, bool ALL>
+__device__ __forceinline__ void few_column(const Params& p, const unsigned char* in, int rb,
+                                           long long i, unsigned live, const int (&at)[FI],
+                                           unsigned long long (&v)[FI]) {
+  if (MODE == 2 || !ALL) few_gather(in, rb, at, live, v);
+  else few_rows<MODE == 0>(in, rb, i, live, v);
+}
+
+// The rows' buckets (a nibble each) and how many each bucket has, a nibble a
+// bucket; rank: how many of its bucket come before a row in the lane, a nibble.
+template <bool ALL>
+__device__ __forceinline__ void few_buckets(int logB, const unsigned long long (&key)[FI],
+                                            unsigned live, unsigned& bk, unsigned& rank,
+                                            unsigned& count) {
+  bk = rank = count = 0;
+#pragma unroll
+  for (int k = 0; k < FI; ++k) {
+    const unsigned b = bucket_of_hash(mix64((uint64_t)key[k]), logB);
+    bk |= b << 4 * k;
+    rank |= (count >> 4 * b & 15) << 4 * k;
+    if (ALL || (live >> k & 1)) count += 1u << 4 * b;
+  }
+}
+// Four nibbles as four bytes.
+__device__ __forceinline__ unsigned nibbles_to_bytes(unsigned x) {
+  x = (x | x << 8) & 0x00ff00ff;
+  return (x | x << 4) & 0x0f0f0f0f;
+}
+
+template <int MODE, bool ALL>
+__device__ __forceinline__ void few_hist(const Params& p, int (&h)[FW][FB]) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const long long i = (long long)blockIdx.x * SUB + w * FSEG + lane * FI;
+  int at[FI];
+  unsigned long long key[FI] = {};
+  const unsigned live = few_live<MODE, ALL>(p, i, at);
+  few_column<MODE, ALL>(p, reinterpret_cast<const unsigned char*>(p.key), 8, i, live, at, key);
+  unsigned bk, rank, count;
+  few_buckets<ALL && MODE != 1>(p.logB, key, live, bk, rank, count);
+  const unsigned b0 = nibbles_to_bytes(count & 0xffff), b1 = nibbles_to_bytes(count >> 16);
+  // two 16-bit fields a word: buckets 0 and 2, 1 and 3, 4 and 6, 5 and 7
+  const unsigned s0 = __reduce_add_sync(FULL, b0 & 0x00ff00ff);
+  const unsigned s1 = __reduce_add_sync(FULL, b0 >> 8 & 0x00ff00ff);
+  const unsigned s2 = __reduce_add_sync(FULL, b1 & 0x00ff00ff);
+  const unsigned s3 = __reduce_add_sync(FULL, b1 >> 8 & 0x00ff00ff);
+  if (lane < FB) {
+    const unsigned x = lane < 4 ? (lane & 1 ? s1 : s0) : (lane & 1 ? s3 : s2);
+    h[w][lane] = x >> (lane & 2 ? 16 : 0) & 0xffff;
+  }
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(FT) k_hist_few(Params p) {
+  if (failed(p)) return;
+  __shared__ int h[FW][FB];
+  if ((long long)(blockIdx.x + 1) * SUB <= p.ndom) few_hist<MODE, true>(p, h);
+  else few_hist<MODE, false>(p, h);
+  __syncthreads();
+  if ((int)threadIdx.x < p.B) {
+    int t = 0;
+#pragma unroll
+    for (int q = 0; q < FW; ++q) t += h[q][threadIdx.x];
+    p.hist[(long long)blockIdx.x * p.B + threadIdx.x] = t;
+  }
+}
+
+template <bool ALL, typename T>
+__device__ __forceinline__ void few_stage(FewWarp& S, unsigned s0, unsigned s1, unsigned live,
+                                          const unsigned long long (&v)[FI]) {
+  T* stage = reinterpret_cast<T*>(S.stage);
+#pragma unroll
+  for (int k = 0; k < FI; ++k)
+    if (ALL || (live >> k & 1)) stage[(k < 4 ? s0 : s1) >> 8 * (k & 3) & 0xff] = (T)v[k];
+}
+template <bool ALL, typename T>
+__device__ __forceinline__ void few_write(const FewWarp& S, unsigned char* out_,
+                                          const unsigned* dst, int n,
+                                          const unsigned (&meta)[FI]) {
+  const T* stage = reinterpret_cast<const T*>(S.stage);
+  T* out = reinterpret_cast<T*>(out_);
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int t = 0; t < FI; ++t) {
+    const int e = t * 32 + lane;
+    if (ALL || e < n) out[dst[meta[t] >> 8] + (unsigned)e] = stage[e];
+  }
+}
+
+template <int MODE, bool ALL>
+__device__ __forceinline__ void few_scatter(const Params& p, FewWarp& S, int (&wh)[FW][FB]) {
+  constexpr bool EVERY = ALL && MODE != 1;  // no row is left out
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const long long r0 = (long long)blockIdx.x * SUB + w * FSEG, i = r0 + lane * FI;
+  int at[FI];
+  unsigned long long v[FI] = {};
+  const unsigned live = few_live<MODE, ALL>(p, i, at);
+  unsigned bk, rank, count;
+  {
+    unsigned long long key[FI] = {};
+    few_column<MODE, ALL>(p, reinterpret_cast<const unsigned char*>(p.key), 8, i, live, at, key);
+    // the first column rides with the keys (the key column itself: no reload)
+    if ((const void*)p.c.in[0] == (const void*)p.key && p.c.rb[0] == 8) {
+#pragma unroll
+      for (int k = 0; k < FI; ++k) v[k] = key[k];
+    } else {
+      few_column<MODE, ALL>(p, p.c.in[0], p.c.rb[0], i, live, at, v);
+    }
+    few_buckets<EVERY>(p.logB, key, live, bk, rank, count);
+  }
+  // each bucket's rows in the lanes before, a byte a bucket (248 at most)
+  const unsigned c0 = nibbles_to_bytes(count & 0xffff), c1 = nibbles_to_bytes(count >> 16);
+  unsigned e0 = __shfl_up_sync(FULL, c0, 1), e1 = __shfl_up_sync(FULL, c1, 1);
+  if (lane == 0) e0 = e1 = 0;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned y0 = __shfl_up_sync(FULL, e0, o), y1 = __shfl_up_sync(FULL, e1, o);
+    if (lane >= o) {
+      e0 += y0;
+      e1 += y1;
+    }
+  }
+  // lane b < 8: bucket b's rows in the warp, and its first staged row
+  const unsigned t0 = __shfl_sync(FULL, e0, 31), t1 = __shfl_sync(FULL, e1, 31);
+  const unsigned l0 = __shfl_sync(FULL, c0, 31), l1 = __shfl_sync(FULL, c1, 31);
+  const int sh = 8 * (lane & 3);
+  const int cnt = lane < FB ? (int)(((lane < 4 ? t0 : t1) >> sh & 0xff) +
+                                    ((lane < 4 ? l0 : l1) >> sh & 0xff))
+                            : 0;
+  int incl = cnt;
+#pragma unroll
+  for (int o = 1; o < FB; o <<= 1) {
+    const int y = __shfl_up_sync(FULL, incl, o);
+    if (lane >= o) incl += y;
+  }
+  const int first = incl - cnt, n = __shfl_sync(FULL, incl, FB - 1);
+  if (lane < FB) {
+    wh[w][lane] = cnt;
+    S.first[lane] = (unsigned char)first;
+  }
+  __syncthreads();
+  // the rows' places in the stage, a byte each (byte sums wrap: the place does not)
+  unsigned s0 = 0, s1 = 0;
+  {
+    const unsigned f0 = __vadd4(e0, *reinterpret_cast<const unsigned*>(S.first));
+    const unsigned f1 = __vadd4(e1, *reinterpret_cast<const unsigned*>(S.first + 4));
+#pragma unroll
+    for (int k = 0; k < FI; ++k) {
+      const unsigned b = bk >> 4 * k & 15;
+      const unsigned s = (__byte_perm(f0, f1, b) + (rank >> 4 * k & 15)) & 0xff;
+      (k < 4 ? s0 : s1) |= s << 8 * (k & 3);
+      if (EVERY || (live >> k & 1)) S.meta[s] = (unsigned short)(b << 8 | (lane * FI + k));
+    }
+  }
+  if (lane < p.B) {
+    unsigned d = (unsigned)p.hist[(long long)blockIdx.x * p.B + lane] - (unsigned)first;
+    for (int q = 0; q < w; ++q) d += (unsigned)wh[q][lane];
+    for (int cl = 0; cl < p.ncls; ++cl)
+      S.dst[cl][lane] = d + (unsigned)p.bases[(long long)cl * p.B + lane];
+  }
+  __syncwarp();
+  unsigned meta[FI];
+#pragma unroll
+  for (int t = 0; t < FI; ++t) meta[t] = EVERY || t * 32 + lane < n ? S.meta[t * 32 + lane] : 0;
+  for (int c = 0; c < p.c.ncols; ++c) {
+    const int rb = p.c.rb[c];
+    const unsigned* dst = S.dst[p.c.cls[c]];
+    unsigned char* out = p.c.out[c];
+    switch (rb) {
+      case 8: few_stage<EVERY, unsigned long long>(S, s0, s1, live, v); break;
+      case 4: few_stage<EVERY, unsigned>(S, s0, s1, live, v); break;
+      case 2: few_stage<EVERY, unsigned short>(S, s0, s1, live, v); break;
+      default: few_stage<EVERY, unsigned char>(S, s0, s1, live, v); break;
+    }
+    __syncwarp();
+    if (c + 1 < p.c.ncols)
+      few_column<MODE, ALL>(p, p.c.in[c + 1], p.c.rb[c + 1], i, live, at, v);
+    switch (rb) {
+      case 8: few_write<EVERY, unsigned long long>(S, out, dst, n, meta); break;
+      case 4: few_write<EVERY, unsigned>(S, out, dst, n, meta); break;
+      case 2: few_write<EVERY, unsigned short>(S, out, dst, n, meta); break;
+      default: few_write<EVERY, unsigned char>(S, out, dst, n, meta); break;
+    }
+    __syncwarp();
+  }
+  const unsigned* dst = S.dst[p.gcls];
+#pragma unroll
+  for (int t = 0; t < FI; ++t) {
+    const int e = t * 32 + lane;
+    if (!EVERY && e >= n) continue;
+    const long long r = r0 + (meta[t] & 255);
+    p.gout[dst[meta[t] >> 8] + (unsigned)e] = p.goff + (MODE == 2 ? (long long)p.src[r] : r);
+  }
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(FT, 4) k_scatter_few(Params p) {
+  if (failed(p)) return;
+  __shared__ __align__(16) FewWarp warps[FW];
+  __shared__ int wh[FW][FB];
+  FewWarp& S = warps[threadIdx.x >> 5];
+  if ((long long)(blockIdx.x + 1) * SUB <= p.ndom) few_scatter<MODE, true>(p, S, wh);
+  else few_scatter<MODE, false>(p, S, wh);
 }
 
 __global__ void __launch_bounds__(PT) k_scatter(Params p) {
@@ -1139,25 +1450,30 @@ extern "C" int pf_partition_sort(const void* const* cols_in, void* const* cols_o
   p.hist = l.hist;
   p.bases = l.bases;
 
-  // the plain case: no mask, one sub-tile a chunk, one word a row
-  bool plain = !p.mask && !p.src && !p.needs_j && p.chunk == SUB && !p.key_comp &&
-               getenv("PF_PART_GENERAL") == nullptr;
+  // no compacted column, one sub-tile a chunk, one word a row: few buckets, or
+  // no mask
+  bool words = !p.needs_j && p.chunk == SUB && !p.key_comp && getenv("PF_PART_GENERAL") == nullptr;
   for (int c = 0; c < p.c.ncols; ++c)
-    plain = plain && !p.c.comp[c] && p.c.word[c] == p.c.rb[c] &&
+    words = words && !p.c.comp[c] && p.c.word[c] == p.c.rb[c] &&
             (p.c.rb[c] == 1 || p.c.rb[c] == 2 || p.c.rb[c] == 4 || p.c.rb[c] == 8);
+  bool few = words && B <= FB && (use_sel || ((uintptr_t)mask & 7) == 0);
+  for (int c = 0; c < p.c.ncols && !use_sel; ++c)  // eight rows a load, 32 bytes at most
+    few = few && ((uintptr_t)p.c.in[c] & (std::min(32, 8 * p.c.rb[c]) - 1)) == 0;
+  const bool plain = words && !few && !p.mask && !p.src;
   {
     PF_KERNEL("k_hist", st);
-    if (plain) k_hist_plain<<<p.nchunks, PT, 0, st>>>(p);
+    if (few && p.src) k_hist_few<2><<<p.nchunks, FT, 0, st>>>(p);
+    else if (few && p.mask) k_hist_few<1><<<p.nchunks, FT, 0, st>>>(p);
+    else if (few) k_hist_few<0><<<p.nchunks, FT, 0, st>>>(p);
+    else if (plain) k_hist_plain<<<p.nchunks, PT, 0, st>>>(p);
     else k_hist<<<p.nchunks, PT, 0, st>>>(p);
   }
   PF_LAUNCH("k_hist");
+  const int cg = (p.nchunks + SCAN_G - 1) / SCAN_G;
+  const dim3 scan_grid((B + 31) / 32, SCAN_G);
   {
-    const int cg = (p.nchunks + SCAN_G - 1) / SCAN_G;
-    const dim3 grid((B + 31) / 32, SCAN_G);
     PF_KERNEL("k_scan", st);
-    k_scan_sum<<<grid, PT, 0, st>>>(l.hist, p.nchunks, B, cg, l.gsum, l.flags);
-    k_scan_groups<<<(B + 255) / 256, 256, 0, st>>>(l.gsum, B, l.counts, l.flags);
-    k_scan_write<<<grid, PT, 0, st>>>(l.hist, p.nchunks, B, cg, l.gsum, l.flags);
+    k_scan_sum<<<scan_grid, PT, 0, st>>>(l.hist, p.nchunks, B, cg, l.gsum, l.flags);
   }
   PF_LAUNCH("k_scan");
   Rpu rpu;
@@ -1165,13 +1481,30 @@ extern "C" int pf_partition_sort(const void* const* cols_in, void* const* cols_o
   for (int c = 0; c < ncls; ++c) rpu.v[c] = pf_rows_per_unit(rb_cls[c]);
   {
     PF_KERNEL("k_bases", st);
-    k_bases<<<1, 1024, 0, st>>>(l.counts, B, rpu, ncls, l.bases, host_dev, l.flags, n_valid,
+    k_bases<<<1, 1024, 0, st>>>(l.gsum, l.counts, B, rpu, ncls, l.bases, host_dev, l.flags, n_valid,
                                 prologue ? l.ptotal : nullptr);
   }
   PF_LAUNCH("k_bases");
   cudaEvent_t ev;
   if (int rc = record_event(st, &ev)) return rc;
+  {
+    PF_KERNEL("k_scan", st);
+    k_scan_write<<<scan_grid, PT, 0, st>>>(l.hist, p.nchunks, B, cg, l.gsum, l.flags);
+  }
+  PF_LAUNCH("k_scan");
 
+  if (few) {
+    {
+      PF_KERNEL("k_scatter", st);
+      if (p.src) k_scatter_few<2><<<p.nchunks, FT, 0, st>>>(p);
+      else if (p.mask) k_scatter_few<1><<<p.nchunks, FT, 0, st>>>(p);
+      else k_scatter_few<0><<<p.nchunks, FT, 0, st>>>(p);
+    }
+    PF_LAUNCH("k_scatter");
+    // the call's one host wait: the counts, while the scatter runs
+    if (int rc = wait_event(ev)) return rc;
+    return ok();
+  }
   if (plain) {
     const size_t smem = sizeof(PlainSmem);
     if (int rc = opt_in_smem((const void*)k_scatter_plain, smem)) return rc;
