@@ -13,6 +13,7 @@
 // one such step, a thread takes several rows with all their loads issued
 // before the first store.
 #include <algorithm>
+#include <climits>
 #include <vector>
 
 #include "common.cuh"
@@ -98,94 +99,63 @@ __global__ void __launch_bounds__(GT) k_gather(GatherArgs a) {
   if ((threadIdx.x & 31) == 0 && bad) atomicAdd(a.bad, bad);
 }
 
-#ifndef PF_GATHER_LDG
-#define PF_GATHER_LDG 1
-#endif
-#ifndef PF_GATHER_R
-#define PF_GATHER_R 4
-#endif
-constexpr int GR = PF_GATHER_R;  // rows a thread takes together
+constexpr int GR = 4;  // rows a thread takes together (8: no faster)
+// Columns of at most this many bytes in all, which L2 holds, are gathered in one
+// launch: their random reads do not reach HBM, and the indexes are read once
+// (5.4M random rows of 8 + 4 bytes from 72 MB 74 us, a launch a column 91; 30M of
+// 8 + 8 from 48 MB 349 and 431, from 96 MB 473 and 432, from 160 MB 732 and 461).
+constexpr long long GATHER_TOGETHER = 80LL << 20;
 
+// A column's words at GR indexes, all loaded before the first store.  ok: the
+// rows that have one, live: those there are (the others of them are null rows).
 template <typename W>
-__device__ __forceinline__ W load_word(const unsigned char* base, long long j) {
-  const W* p = reinterpret_cast<const W*>(base) + j;
-  return PF_GATHER_LDG ? ldg_word(p) : *p;
+__device__ __forceinline__ void gather_column(const GatherArgs& a, int c, long long i,
+                                              const long long (&j)[GR], unsigned ok,
+                                              unsigned live) {
+  const W* in = reinterpret_cast<const W*>(a.in[c]);
+  W* out = reinterpret_cast<W*>(a.out[c]) + i;
+  W v[GR];
+#pragma unroll
+  for (int r = 0; r < GR; ++r)
+    if (ok >> r & 1) v[r] = ldg_word(in + j[r]);
+#pragma unroll
+  for (int r = 0; r < GR; ++r)
+    if (ok >> r & 1) out[r * GT] = v[r];
+  if (ok == live) return;
+  for (int r = 0; r < GR; ++r)
+    if ((live & ~ok) >> r & 1) copy_row<unsigned char>(a, c, i + r * GT, 0, true);
 }
 
-// One word a row in every column (row_bytes == wsize): GR rows a thread, the
-// indexes and then every column's words loaded before the first store.
-template <int NC>
+// One word a row in every column (row_bytes == wsize): GR rows a thread, their
+// indexes read once, the columns in turn, each with its own loop for its word
+// (a choice of word a row left 5.4M rows of 8 + 4 bytes at 86 us, now 68).
 __global__ void __launch_bounds__(GT) k_gather_words(GatherArgs a) {
+  const long long i = (long long)blockIdx.x * GT * GR + threadIdx.x;
+  long long j[GR];
+  unsigned ok = 0, live = 0;
+#pragma unroll
+  for (int r = 0; r < GR; ++r) j[r] = i + r * GT < a.n ? __ldcs(a.idx + i + r * GT) : 0;
   unsigned long long bad = 0;
-  for (long long b = (long long)blockIdx.x * GT * GR; b < a.n;
-       b += (long long)gridDim.x * GT * GR) {
-    long long j[GR];
-    bool null_row[GR];
 #pragma unroll
-    for (int r = 0; r < GR; ++r) {
-      const long long i = b + r * GT + threadIdx.x;
-      j[r] = i < a.n ? a.idx[i] : 0;
-    }
-#pragma unroll
-    for (int r = 0; r < GR; ++r) {
-      const bool live = b + r * GT + threadIdx.x < a.n;
-      null_row[r] = false;
-      if (live && a.allow_null && j[r] == a.null_idx) {
-        null_row[r] = true;
-      } else if (live && (j[r] < 0 || j[r] >= a.n_src)) {
-        null_row[r] = true;
-        ++bad;
-      }
-      if (!live) null_row[r] = true;
-    }
-    uint4 v[NC][GR];
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-#pragma unroll
-      for (int r = 0; r < GR; ++r) {
-        if (null_row[r]) continue;
-        switch (a.wsize[c]) {
-          case 16: v[c][r] = load_word<uint4>(a.in[c], j[r]); break;
-          case 8: {
-            const unsigned long long x = load_word<unsigned long long>(a.in[c], j[r]);
-            v[c][r].x = (unsigned)x;
-            v[c][r].y = (unsigned)(x >> 32);
-            break;
-          }
-          case 4: v[c][r].x = load_word<unsigned>(a.in[c], j[r]); break;
-          case 2: v[c][r].x = load_word<unsigned short>(a.in[c], j[r]); break;
-          default: v[c][r].x = load_word<unsigned char>(a.in[c], j[r]); break;
-        }
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-#pragma unroll
-      for (int r = 0; r < GR; ++r) {
-        const long long i = b + r * GT + threadIdx.x;
-        if (i >= a.n) continue;
-        if (null_row[r]) {
-          copy_row<unsigned char>(a, c, i, 0, true);
-          continue;
-        }
-        unsigned char* out = a.out[c];
-        switch (a.wsize[c]) {
-          case 16: reinterpret_cast<uint4*>(out)[i] = v[c][r]; break;
-          case 8:
-            reinterpret_cast<unsigned long long*>(out)[i] =
-                ((unsigned long long)v[c][r].y << 32) | v[c][r].x;
-            break;
-          case 4: reinterpret_cast<unsigned*>(out)[i] = v[c][r].x; break;
-          case 2: reinterpret_cast<unsigned short*>(out)[i] = (unsigned short)v[c][r].x; break;
-          default: out[i] = (unsigned char)v[c][r].x; break;
-        }
-      }
+  for (int r = 0; r < GR; ++r) {
+    if (i + r * GT >= a.n) continue;
+    live |= 1u << r;
+    if (a.allow_null && j[r] == a.null_idx) continue;
+    if (j[r] < 0 || j[r] >= a.n_src) ++bad;
+    else ok |= 1u << r;
+  }
+  for (int c = 0; c < a.ncols; ++c) {
+    switch (a.wsize[c]) {
+      case 16: gather_column<uint4>(a, c, i, j, ok, live); break;
+      case 8: gather_column<unsigned long long>(a, c, i, j, ok, live); break;
+      case 4: gather_column<unsigned>(a, c, i, j, ok, live); break;
+      case 2: gather_column<unsigned short>(a, c, i, j, ok, live); break;
+      default: gather_column<unsigned char>(a, c, i, j, ok, live); break;
     }
   }
   for (int o = 16; o; o >>= 1) bad += __shfl_xor_sync(FULL, bad, o);
   if ((threadIdx.x & 31) == 0 && bad && a.bad) atomicAdd(a.bad, bad);
 }
-
 
 // ---- zero copy: rows read in place from pinned host segments ----------------
 //
@@ -299,18 +269,16 @@ extern "C" int pf_gather(const void* const* cols_in, void* const* cols_out, cons
   a.bad = (unsigned long long*)bad;
   const unsigned gx = (unsigned)std::max<long long>(
       1, std::min<long long>((n + GT - 1) / GT, (long long)sm_count() * 8));
-  bool words = ncols <= 4;
+  bool words = (n + GT * GR - 1) / (GT * GR) <= INT_MAX;
   for (int c = 0; c < ncols; ++c) words = words && a.row_bytes[c] == a.wsize[c];
   if (words) {
-    const unsigned gw = (unsigned)std::max<long long>(
-        1, std::min<long long>((n + GT * GR - 1) / (GT * GR), (long long)sm_count() * 8));
-#ifndef PF_GATHER_SPLIT
-#define PF_GATHER_SPLIT 1
-#endif
-    if (PF_GATHER_SPLIT) {
-      // a pass a column: one column's random reads at a time (2 int64
-      // columns at 100M random rows: 4.70 ms, both columns in one pass with
-      // 2 rows a thread 4.76, with 4 rows a thread 5.14)
+    const unsigned gw = (unsigned)((n + GT * GR - 1) / (GT * GR));
+    long long bytes = 0;
+    for (int c = 0; c < ncols; ++c) bytes += n_src * a.row_bytes[c];
+    PF_KERNEL("k_gather_words", st);
+    if (bytes <= GATHER_TOGETHER) {
+      k_gather_words<<<gw, GT, 0, st>>>(a);
+    } else {
       for (int c = 0; c < ncols; ++c) {
         GatherArgs one = a;
         one.ncols = 1;
@@ -321,18 +289,8 @@ extern "C" int pf_gather(const void* const* cols_in, void* const* cols_out, cons
         one.esize[0] = a.esize[c];
         one.wsize[0] = a.wsize[c];
         if (c > 0) one.bad = nullptr;
-        PF_KERNEL("k_gather_words", st);
-        k_gather_words<1><<<gw, GT, 0, st>>>(one);
+        k_gather_words<<<gw, GT, 0, st>>>(one);
       }
-      PF_LAUNCH("k_gather_words");
-      return ok();
-    }
-    PF_KERNEL("k_gather_words", st);
-    switch (ncols) {
-      case 1: k_gather_words<1><<<gw, GT, 0, st>>>(a); break;
-      case 2: k_gather_words<2><<<gw, GT, 0, st>>>(a); break;
-      case 3: k_gather_words<3><<<gw, GT, 0, st>>>(a); break;
-      default: k_gather_words<4><<<gw, GT, 0, st>>>(a); break;
     }
     PF_LAUNCH("k_gather_words");
     return ok();
