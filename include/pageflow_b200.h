@@ -115,8 +115,9 @@ int64_t pf_rows_per_unit(int64_t row_bytes);
 /*
  * Inner join on a unique build tuple of 1 or 2 int64 keys.  build_idx and
  * probe_idx have n_probe rows each; the first host_out[0] hold the matches in
- * probe-row order.  host_out: pinned int64[2] ([1] is set to 0).  Waits once.
- * 1 <= n_build, n_probe <= PF_JOIN_MAX_ROWS.
+ * probe-row order; what the others hold is unspecified (probe_idx serves as
+ * scratch until it is written).  host_out: pinned int64[2] ([1] is set to 0).
+ * Waits once.  1 <= n_build, n_probe <= PF_JOIN_MAX_ROWS.
  */
 size_t pf_join_unique_hash_workspace(int64_t n_build, int64_t n_probe);
 int pf_join_unique_hash(const int64_t* build0, const int64_t* build1, int64_t n_build,

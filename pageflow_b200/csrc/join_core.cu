@@ -3,9 +3,9 @@
 // wrapper operators/join_core.py):
 //
 //   unique hash  inner join on a build tuple (1-2 int64 keys) proven unique:
-//                a table of 2*n_build 4-byte slots (the build row in the low
-//                r bits, r the bit width of n_build; the tuple hash's bits
-//                above them as a fingerprint), linear probing; each probe
+//                a table of 4-byte slots (the build row in the low r bits, r
+//                the bit width of n_build; the tuple hash's bits above them as
+//                a fingerprint) in buckets of one 32-byte sector; each probe
 //                row's partner; the matched probe rows compacted in order
 //   semi / anti  a set of the build keys (INT64_MIN marks an empty slot), with
 //                an optional per-key min / max of one build column answering
@@ -45,26 +45,33 @@ __device__ __forceinline__ uint64_t first_slot(uint64_t h, int logcap) {
 //
 // A slot holds (hash << r) | row, rmask = 2^r - 1 with n_build <= rmask: a
 // row never fills its r bits, so no entry is all ones (EMPTY_SLOT).  The home
-// slot is the multiply-shift of the hash's bits below its top nine onto
-// [0, cap) (reference operators/kernels/join_core.cu:55 slot_of), which
-// leans on the high bits; the fingerprint takes the low ones.
+// bucket is the multiply-shift of the hash's bits below its top nine onto
+// [0, buckets), which leans on the high bits; the fingerprint takes the low
+// ones.  A row leaves a bucket only when its eight slots are taken, so a bucket
+// with a free one ends a lookup.
+//
+// A random read costs about the same whatever its size up to a sector: with
+// linear probing a lookup read two slots and a build key (6M against 1.5M rows:
+// 98 us), now a bucket and a build key (61 us).
 
 struct UhTable {
-  unsigned* slot;
-  unsigned long long cap;
+  unsigned* slot;              // [8 * buckets]
+  unsigned long long buckets;
   unsigned rmask;
   int rbits;
 };
 
-__device__ __forceinline__ unsigned long long uh_home(uint64_t h, unsigned long long cap) {
-  return __umul64hi(h << 9, cap);
+__device__ __forceinline__ unsigned long long uh_home(uint64_t h, unsigned long long buckets) {
+  return __umul64hi(h << 9, buckets);
 }
 
-__device__ __forceinline__ unsigned long long uh_next(unsigned long long s,
-                                                      unsigned long long cap) {
-  return s + 1 == cap ? 0 : s + 1;
+__device__ __forceinline__ unsigned long long uh_next(unsigned long long b,
+                                                      unsigned long long buckets) {
+  return b + 1 == buckets ? 0 : b + 1;
 }
 
+// Claims a slot without reading it first, from one that the fingerprint picks
+// on (1.2 claims a row at 0.3 full; 1.5M rows 33 -> 24 us).
 template <bool TWO>
 __global__ void __launch_bounds__(T) k_uh_build(const long long* __restrict__ b0,
                                                 const long long* __restrict__ b1, long long n,
@@ -73,22 +80,46 @@ __global__ void __launch_bounds__(T) k_uh_build(const long long* __restrict__ b0
   if (i >= n) return;
   const uint64_t h = tuple_hash(b0[i], TWO ? b1[i] : 0, TWO);
   const unsigned entry = ((unsigned)h << t.rbits) | (unsigned)i;
-  unsigned long long s = uh_home(h, t.cap);
-  for (unsigned long long probes = 0; probes < t.cap; ++probes) {
-    if (atomicCAS(&t.slot[s], EMPTY_SLOT, entry) == EMPTY_SLOT) return;
-    s = uh_next(s, t.cap);
+  unsigned long long b = uh_home(h, t.buckets);
+  for (unsigned long long probes = 0; probes < t.buckets; ++probes) {
+    for (unsigned k = 0; k < 8; ++k)
+      if (atomicCAS(&t.slot[8 * b + (((unsigned)h + k) & 7)], EMPTY_SLOT, entry) == EMPTY_SLOT)
+        return;
+    b = uh_next(b, t.buckets);
   }
 }
 
-#ifndef PF_UH_U
-#define PF_UH_U 2
-#endif
-constexpr int UH_U = PF_UH_U;  // probe rows a thread resolves together
+struct UhBucket {
+  unsigned e[8];
+};
+__device__ __forceinline__ UhBucket uh_load(const unsigned* p) {
+  UhBucket b;
+  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(b.e[0]), "=r"(b.e[1]), "=r"(b.e[2]), "=r"(b.e[3]), "=r"(b.e[4]),
+                 "=r"(b.e[5]), "=r"(b.e[6]), "=r"(b.e[7])
+               : "l"(p));
+  return b;
+}
+
+// The slots of a bucket that hold the fingerprint, and whether one is free.
+__device__ __forceinline__ unsigned uh_match(const UhBucket& b, unsigned fp, unsigned fmask,
+                                             bool* open) {
+  unsigned m = 0;
+  *open = false;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    if (b.e[k] == EMPTY_SLOT) *open = true;
+    else if ((b.e[k] & fmask) == fp) m |= 1u << k;
+  }
+  return m;
+}
+
+constexpr int UH_U = 2;  // probe rows a thread resolves together (6M: 61 us; 1 or 4: 70)
 static_assert(CITEMS % UH_U == 0, "probe batches tile a thread's rows");
 
 // Probe CB rows a block: partner[i] (build row or -1), the block's matches.
-// UH_U rows at a time: their home and next slots loaded together, then their
-// candidates' keys; a row that those two slots do not settle walks on.
+// UH_U rows at a time: their home buckets loaded together, then their first
+// candidates' keys; a row that those do not settle walks from its home bucket.
 template <bool TWO>
 __global__ void __launch_bounds__(CT) k_uh_probe(const long long* __restrict__ b0,
                                                  const long long* __restrict__ b1,
@@ -96,41 +127,43 @@ __global__ void __launch_bounds__(CT) k_uh_probe(const long long* __restrict__ b
                                                  const long long* __restrict__ p1, long long n,
                                                  UhTable t, int* __restrict__ partner,
                                                  long long* __restrict__ bcnt) {
-  const unsigned* __restrict__ tab = t.slot;
   const unsigned fmask = ~t.rmask;
   const long long base = (long long)blockIdx.x * CB;
   int c = 0;
   for (int kk = 0; kk < CITEMS; kk += UH_U) {
     long long k0[UH_U], k1[UH_U];
-    unsigned fp[UH_U], e0[UH_U], e1[UH_U];
-    unsigned long long s0[UH_U];
-    int cand[UH_U], r[UH_U];
+    unsigned fp[UH_U];
+    unsigned long long home[UH_U];
+    UhBucket bu[UH_U];
+    int cand[UH_U];
+    bool settled[UH_U];
 #pragma unroll
     for (int u = 0; u < UH_U; ++u) {
       const long long i = base + (kk + u) * CT + threadIdx.x;
-      k0[u] = i < n ? p0[i] : 0;
-      k1[u] = TWO && i < n ? p1[i] : 0;
+      k0[u] = i < n ? __ldcs(p0 + i) : 0;
+      k1[u] = TWO && i < n ? __ldcs(p1 + i) : 0;
     }
 #pragma unroll
     for (int u = 0; u < UH_U; ++u) {
       const uint64_t h = tuple_hash(k0[u], k1[u], TWO);
       fp[u] = (unsigned)h << t.rbits;
-      s0[u] = uh_home(h, t.cap);
+      home[u] = uh_home(h, t.buckets);
+      if (base + (kk + u) * CT + threadIdx.x < n) bu[u] = uh_load(t.slot + 8 * home[u]);
     }
+    // the first candidate (-1: none), and whether a miss of it settles the row
 #pragma unroll
     for (int u = 0; u < UH_U; ++u) {
-      const bool in = base + (kk + u) * CT + threadIdx.x < n;
-      e0[u] = in ? tab[s0[u]] : EMPTY_SLOT;
-      e1[u] = in ? tab[uh_next(s0[u], t.cap)] : EMPTY_SLOT;
-    }
-    // the candidate among the two slots: -1 settled as no match, -2 walk on
+      cand[u] = -1;
+      settled[u] = true;
+      if (base + (kk + u) * CT + threadIdx.x >= n) continue;
+      bool open;
+      const unsigned m = uh_match(bu[u], fp[u], fmask, &open);
+      unsigned e = 0;
 #pragma unroll
-    for (int u = 0; u < UH_U; ++u) {
-      if (e0[u] == EMPTY_SLOT) cand[u] = -1;
-      else if ((e0[u] & fmask) == fp[u]) cand[u] = (int)(e0[u] & t.rmask);
-      else if (e1[u] == EMPTY_SLOT) cand[u] = -1;
-      else if ((e1[u] & fmask) == fp[u]) cand[u] = (int)(e1[u] & t.rmask);
-      else cand[u] = -2;
+      for (int k = 7; k >= 0; --k)
+        if (m >> k & 1) e = bu[u].e[k];
+      if (m) cand[u] = (int)(e & t.rmask);
+      settled[u] = open && (m & (m - 1)) == 0;
     }
     long long c0[UH_U], c1[UH_U];
 #pragma unroll
@@ -140,32 +173,30 @@ __global__ void __launch_bounds__(CT) k_uh_probe(const long long* __restrict__ b
     }
 #pragma unroll
     for (int u = 0; u < UH_U; ++u) {
-      r[u] = -1;
-      if (cand[u] >= 0 && c0[u] == k0[u] && (!TWO || c1[u] == k1[u])) r[u] = cand[u];
-      else if (cand[u] != -1) {
-        // a fingerprint that matched another key, or two full slots: walk
-        // the chain from its home slot
-        unsigned long long s = s0[u];
-        for (unsigned long long probes = 0; probes < t.cap; ++probes) {
-          const unsigned e = tab[s];
-          if (e == EMPTY_SLOT) break;
-          if ((e & fmask) == fp[u]) {
-            const int row = (int)(e & t.rmask);
-            if (b0[row] == k0[u] && (!TWO || b1[row] == k1[u])) {
-              r[u] = row;
-              break;
+      const long long i = base + (kk + u) * CT + threadIdx.x;
+      int r = cand[u] >= 0 && c0[u] == k0[u] && (!TWO || c1[u] == k1[u]) ? cand[u] : -1;
+      if (r < 0 && !settled[u]) {
+        // another slot of its fingerprint, or a full bucket
+        unsigned long long b = home[u];
+        for (unsigned long long probes = 0; probes < t.buckets && r < 0; ++probes) {
+          bool open = false;
+          for (int k = 0; k < 8 && r < 0; ++k) {
+            const unsigned e = t.slot[8 * b + k];
+            if (e == EMPTY_SLOT) {
+              open = true;
+              continue;
             }
+            if ((e & fmask) != fp[u]) continue;
+            const int row = (int)(e & t.rmask);
+            if (b0[row] == k0[u] && (!TWO || b1[row] == k1[u])) r = row;
           }
-          s = uh_next(s, t.cap);
+          if (open) break;
+          b = uh_next(b, t.buckets);
         }
       }
-    }
-#pragma unroll
-    for (int u = 0; u < UH_U; ++u) {
-      const long long i = base + (kk + u) * CT + threadIdx.x;
       if (i < n) {
-        partner[i] = r[u];
-        c += r[u] >= 0;
+        partner[i] = r;
+        c += r >= 0;
       }
     }
   }
@@ -382,16 +413,35 @@ struct UhLayout {
 
 UhLayout uh_layout(Arena& a, long long nb, long long np) {
   UhLayout l{};
-  l.table.cap = (unsigned long long)std::max<long long>(2 * nb, 2);
+  l.table.buckets = (unsigned long long)std::max<long long>(2 * nb / 8, 1);
   int r = 1;
   while (r < 31 && (1LL << r) - 1 < nb) ++r;  // nb <= 2^r - 1 (nb < 2^31)
   l.table.rbits = r;
   l.table.rmask = (1u << r) - 1;
-  l.table.slot = a.take<unsigned>(l.table.cap);
+  l.table.slot = a.take<unsigned>(8 * l.table.buckets);
   l.partner = a.take<int>(std::max<long long>(np, 1));
   l.bcnt = a.take<long long>((np + CB - 1) / CB + 1);
   l.total = a.take<long long>(1);
   return l;
+}
+
+// The scratch holds a table half full.  One 0.3 full is faster while L2 holds it
+// (a lookup that leaves its bucket holds up its warp; 1.5M x 6M rows: build and
+// probe 24 + 61 us, half full 35 + 85); it lies in the probe row output, which
+// nothing writes before the last lookup is done, where that is large enough,
+// aligned and none of the inputs.
+constexpr long long UH_ROOMY = (64LL << 20) / 32;  // buckets
+
+void uh_roomy(UhLayout& l, const int64_t* b0, const int64_t* b1, long long nb,
+              const int64_t* p0, const int64_t* p1, long long np, int64_t* probe_idx) {
+  const long long room = (nb * 10 / 3 + 7) / 8;
+  if (room > UH_ROOMY || room * 32 > np * 8 || ((uintptr_t)probe_idx & 31)) return;
+  auto apart = [&](const int64_t* x, long long n) {
+    return !x || x + n <= probe_idx || probe_idx + np <= x;
+  };
+  if (!apart(b0, nb) || !apart(b1, nb) || !apart(p0, np) || !apart(p1, np)) return;
+  l.table.slot = (unsigned*)probe_idx;
+  l.table.buckets = (unsigned long long)std::max<long long>(room, 1);
 }
 
 // Queues the table's reset, build and probe, and the scan of the probe
@@ -399,7 +449,7 @@ UhLayout uh_layout(Arena& a, long long nb, long long np) {
 int uh_queue(const UhLayout& l, const int64_t* build0, const int64_t* build1, int64_t nb,
              const int64_t* probe0, const int64_t* probe1, int64_t np, int nkeys,
              long long* count, cudaStream_t st) {
-  PF_CUDA(cudaMemsetAsync(l.table.slot, 0xff, l.table.cap * sizeof(unsigned), st));
+  PF_CUDA(cudaMemsetAsync(l.table.slot, 0xff, 8 * l.table.buckets * sizeof(unsigned), st));
   const unsigned nblk = blocks_for(np, CB);
   const long long* b0 = (const long long*)build0;
   const long long* b1 = (const long long*)(nkeys == 2 ? build1 : build0);
@@ -497,6 +547,8 @@ extern "C" int pf_join_unique_hash(const int64_t* build0, const int64_t* build1,
   if (!workspace || !a.fits())
     return fail(PF_ENOSPACE, "join_unique_hash: workspace of %zu bytes, %zu needed",
                 workspace_bytes, a.used);
+  uh_roomy(l, build0, nkeys == 2 ? build1 : nullptr, n_build, probe0,
+           nkeys == 2 ? probe1 : nullptr, n_probe, probe_idx);
   long long* host_dev = nullptr;
   if (int rc = host_alias(host_out, (void**)&host_dev)) return rc;
   host_out[1] = 0;
