@@ -36,9 +36,10 @@ __device__ __forceinline__ uint64_t tuple_hash(long long k0, long long k1, bool 
   return h;
 }
 
-// The first slot of a hash among 2^logcap: the bits right below its top nine.
-__device__ __forceinline__ uint64_t first_slot(uint64_t h, int logcap) {
-  return (h << 9) >> (64 - logcap);
+// The home slot of a key in the semi / anti set: the multiply-shift of the bits
+// right below its hash's top nine.
+__device__ __forceinline__ unsigned long long set_home(uint64_t key, unsigned long long slots) {
+  return __umul64hi(mix64(key) << 9, slots);
 }
 
 // ---- unique hash -------------------------------------------------------------
@@ -256,10 +257,39 @@ __global__ void __launch_bounds__(CT) k_uh_emit(const int* __restrict__ partner,
 
 // ---- semi / anti ----------------------------------------------------------------
 
+// A slot is W words: the key, the minimum or maximum (W 2) or both and one
+// unused (W 4, a 32-byte sector), so that one random read answers a probe row
+// (a != residual with the three in arrays of their own: 20M rows against 6M 1180
+// us, so 895; build and reset for 400K rows 33 us, so 23).
+
+template <int W>
+__device__ __forceinline__ void set_load(const long long* slot, long long (&x)[4]) {
+  if (W == 4)
+    asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];"
+                 : "=l"(x[0]), "=l"(x[1]), "=l"(x[2]), "=l"(x[3])
+                 : "l"(slot));
+  else if (W == 2)
+    asm volatile("ld.global.v2.b64 {%0, %1}, [%2];" : "=l"(x[0]), "=l"(x[1]) : "l"(slot));
+  else
+    asm volatile("ld.global.b64 %0, [%1];" : "=l"(x[0]) : "l"(slot));
+}
+
+// The empty set, 16 bytes at a time.  least: word 1 is a maximum (W 2), else a
+// minimum.
+template <int W>
+__global__ void __launch_bounds__(T) k_set_reset(longlong2* table, long long pairs, bool least) {
+  for (long long i = (long long)blockIdx.x * T + threadIdx.x; i < pairs;
+       i += (long long)gridDim.x * T)
+    table[i] = W == 4 && (i & 1) ? make_longlong2(LLONG_MIN, 0)
+               : W == 1          ? make_longlong2(EMPTY_KEY, EMPTY_KEY)
+                                 : make_longlong2(EMPTY_KEY, least ? LLONG_MIN : LLONG_MAX);
+}
+
+template <int W>
 __global__ void __launch_bounds__(T) k_set_build(const long long* __restrict__ key,
                                                  const long long* __restrict__ val, long long n,
-                                                 long long* table, long long* mn, long long* mx,
-                                                 int logcap, long long* bad) {
+                                                 long long* table, unsigned long long slots,
+                                                 bool least, long long* bad) {
   const long long i = (long long)blockIdx.x * T + threadIdx.x;
   if (i >= n) return;
   const long long k = key[i];
@@ -267,71 +297,83 @@ __global__ void __launch_bounds__(T) k_set_build(const long long* __restrict__ k
     *bad = 1;
     return;
   }
-  const uint64_t mask = (1ULL << logcap) - 1;
-  uint64_t s = first_slot(mix64((uint64_t)k), logcap);
+  unsigned long long s = set_home((uint64_t)k, slots);
+  long long x[4];
   bool in = false;
-  for (uint64_t probes = 0; probes <= mask; ++probes) {
-    long long cur = table[s];
-    if (cur == EMPTY_KEY)
-      cur = (long long)atomicCAS((unsigned long long*)&table[s], (unsigned long long)EMPTY_KEY,
-                                 (unsigned long long)k);
-    if (cur == EMPTY_KEY || cur == k) {
+  for (unsigned long long probes = 0; probes < slots; ++probes) {
+    set_load<W>(table + W * s, x);
+    if (x[0] == EMPTY_KEY)
+      x[0] = (long long)atomicCAS((unsigned long long*)&table[W * s],
+                                  (unsigned long long)EMPTY_KEY, (unsigned long long)k);
+    if (x[0] == EMPTY_KEY || x[0] == k) {
       in = true;
       break;
     }
-    s = (s + 1) & mask;
+    s = s + 1 == slots ? 0 : s + 1;
   }
   if (!in) {
-    *bad = 2;  // the set is full: cannot happen at half load
+    *bad = 2;  // the set is full: there are more slots than rows
     return;
   }
-  if (mn || mx) {
-    const long long v = val[i];
-    if (mn && v < mn[s]) atomicMin(&mn[s], v);
-    if (mx && v > mx[s]) atomicMax(&mx[s], v);
-  }
+  if (W == 1) return;
+  const long long v = val[i];
+  if ((W == 4 || !least) && v < x[1]) atomicMin(&table[W * s + 1], v);
+  if (W == 2 && least && v > x[1]) atomicMax(&table[W * s + 1], v);
+  if (W == 4 && v > x[2]) atomicMax(&table[W * s + 2], v);
 }
 
+constexpr int SA_U = 2;
+static_assert(CITEMS % SA_U == 0, "probe batches tile a thread's rows");
+
+// SA_U rows a thread at a time, their slots loaded together (2.5M rows: 29.8
+// us; 1 row 32.4, 4 rows 42.4, blocks of 512 or 1024 31.7 and 30.4).
+template <int W>
 __global__ void __launch_bounds__(CT) k_set_probe(const long long* __restrict__ key,
                                                   const long long* __restrict__ val, long long n,
                                                   const long long* __restrict__ table,
-                                                  const long long* __restrict__ mn,
-                                                  const long long* __restrict__ mx, int logcap,
-                                                  int op, bool anti, unsigned char* __restrict__ keep,
+                                                  unsigned long long slots, int op, bool anti,
+                                                  unsigned char* __restrict__ keep,
                                                   long long* __restrict__ bcnt) {
-  const uint64_t mask = (1ULL << logcap) - 1;
   const long long base = (long long)blockIdx.x * CB;
   int c = 0;
-  for (int k = 0; k < CITEMS; ++k) {
-    const long long i = base + k * CT + threadIdx.x;
-    if (i >= n) break;
-    const long long kk = key[i];
-    bool hit = false;
-    uint64_t s = first_slot(mix64((uint64_t)kk), logcap);
-    if (kk != EMPTY_KEY) {
-      for (uint64_t probes = 0; probes <= mask; ++probes) {
-        const long long t = table[s];
-        if (t == kk) {
-          hit = true;
-          break;
+  for (int kk = 0; kk < CITEMS; kk += SA_U) {
+    long long k[SA_U], v[SA_U], x[SA_U][4];
+    unsigned long long s[SA_U];
+#pragma unroll
+    for (int u = 0; u < SA_U; ++u) {
+      const long long i = base + (kk + u) * CT + threadIdx.x;
+      k[u] = i < n ? __ldcs(key + i) : EMPTY_KEY;
+      v[u] = W > 1 && i < n ? __ldcs(val + i) : 0;
+    }
+#pragma unroll
+    for (int u = 0; u < SA_U; ++u) {
+      s[u] = set_home((uint64_t)k[u], slots);
+      set_load<W>(table + W * s[u], x[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < SA_U; ++u) {
+      // the key's slot, or an empty one
+      for (unsigned long long probes = 1;
+           probes < slots && x[u][0] != k[u] && x[u][0] != EMPTY_KEY; ++probes) {
+        s[u] = s[u] + 1 == slots ? 0 : s[u] + 1;
+        set_load<W>(table + W * s[u], x[u]);
+      }
+      const long long i = base + (kk + u) * CT + threadIdx.x;
+      if (i >= n) continue;
+      bool hit = x[u][0] == k[u] && k[u] != EMPTY_KEY;
+      if (W > 1 && hit) {
+        switch (op) {
+          case PF_OP_NE: hit = x[u][1] != v[u] || x[u][W == 4 ? 2 : 1] != v[u]; break;
+          case PF_OP_LT: hit = x[u][1] < v[u]; break;
+          case PF_OP_LE: hit = x[u][1] <= v[u]; break;
+          case PF_OP_GT: hit = x[u][1] > v[u]; break;
+          default: hit = x[u][1] >= v[u]; break;
         }
-        if (t == EMPTY_KEY) break;
-        s = (s + 1) & mask;
       }
+      const bool kp = hit != anti;
+      keep[i] = kp;
+      c += kp;
     }
-    if (hit && op != PF_OP_NONE) {
-      const long long v = val[i];
-      switch (op) {
-        case PF_OP_NE: hit = mn[s] != v || mx[s] != v; break;
-        case PF_OP_LT: hit = mn[s] < v; break;
-        case PF_OP_LE: hit = mn[s] <= v; break;
-        case PF_OP_GT: hit = mx[s] > v; break;
-        default: hit = mx[s] >= v; break;
-      }
-    }
-    const bool kp = hit != anti;
-    keep[i] = kp;
-    c += kp;
   }
   __shared__ int red[CT / 32];
   for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(FULL, c, o);
@@ -364,12 +406,6 @@ __global__ void __launch_bounds__(CT) k_keep_emit(const unsigned char* __restric
   const int tot = block_compact(kp, rank, rows, wsum);
   const long long o = boff[blockIdx.x], b0 = (long long)blockIdx.x * CB;
   for (int e = threadIdx.x; e < tot; e += CT) out[o + e] = b0 + rows[e];
-}
-
-__global__ void k_fill_i64(long long* p, long long v, long long n) {
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x)
-    p[i] = v;
 }
 
 // ---- expand ---------------------------------------------------------------------
@@ -494,27 +530,57 @@ int uh_emit(const UhLayout& l, int64_t np, int64_t* build_idx, int64_t* probe_id
   return PF_OK;
 }
 
+constexpr unsigned long long SA_SLOTS = 1ULL << 26;  // 2 GiB
+
 struct SaLayout {
   long long* table;
-  long long* mn;
-  long long* mx;
+  int words;                 // a slot's (1, 2, 4)
+  unsigned long long slots;
   unsigned char* keep;
   long long* bcnt;
-  long long* dev;  // [0] kept rows, [1] bad
+  long long* total;
 };
 
 SaLayout sa_layout(Arena& a, long long nb, long long np, int op) {
   SaLayout l{};
-  const uint64_t cap = pow2_at_least((uint64_t)std::max<long long>(2 * nb, 2));
-  l.table = a.take<long long>(cap);
-  const bool need_mn = op == PF_OP_NE || op == PF_OP_LT || op == PF_OP_LE;
-  const bool need_mx = op == PF_OP_NE || op == PF_OP_GT || op == PF_OP_GE;
-  l.mn = need_mn ? a.take<long long>(cap) : nullptr;
-  l.mx = need_mx ? a.take<long long>(cap) : nullptr;
+  l.slots = pow2_at_least((uint64_t)std::max<long long>(2 * nb, 2));
+  l.words = op == PF_OP_NONE ? 1 : op == PF_OP_NE ? 4 : 2;
+  // a slot of a sector where three words would do: at most two thirds full in
+  // the same bytes once those matter
+  if (l.words == 4 && l.slots > SA_SLOTS) l.slots = l.slots / 4 * 3;
+  l.table = a.take<long long>(l.words * l.slots);
   l.keep = a.take<unsigned char>(std::max<long long>(np, 1));
   l.bcnt = a.take<long long>((np + CB - 1) / CB + 1);
-  l.dev = a.take<long long>(2);
+  l.total = a.take<long long>(1);
   return l;
+}
+
+template <int W>
+int sa_queue(const SaLayout& l, const int64_t* bk, long long nb, const int64_t* pk, long long np,
+             const int64_t* bv, const int64_t* pv, int op, bool anti, long long* bad,
+             cudaStream_t st) {
+  const bool least = op == PF_OP_GT || op == PF_OP_GE;
+  {
+    PF_KERNEL("k_set_reset", st);
+    const uint64_t pairs = W * l.slots / 2;  // an even number of slots
+    k_set_reset<W><<<(unsigned)std::min<uint64_t>((pairs + T - 1) / T, 8192), T, 0, st>>>(
+        (longlong2*)l.table, (long long)pairs, least);
+  }
+  PF_LAUNCH("k_set_reset");
+  {
+    PF_KERNEL("k_set_build", st);
+    k_set_build<W><<<blocks_for(nb, T), T, 0, st>>>((const long long*)bk, (const long long*)bv,
+                                                    nb, l.table, l.slots, least, bad);
+  }
+  PF_LAUNCH("k_set_build");
+  {
+    PF_KERNEL("k_set_probe", st);
+    k_set_probe<W><<<blocks_for(np, CB), CT, 0, st>>>((const long long*)pk, (const long long*)pv,
+                                                      np, l.table, l.slots, op, anti, l.keep,
+                                                      l.bcnt);
+  }
+  PF_LAUNCH("k_set_probe");
+  return PF_OK;
 }
 
 }  // namespace
@@ -588,35 +654,16 @@ extern "C" int pf_join_semi_anti(const int64_t* build_key, int64_t n_build,
                 a.used);
   long long* host_dev = nullptr;
   if (int rc = host_alias(host_out, (void**)&host_dev)) return rc;
-  const uint64_t cap = pow2_at_least((uint64_t)std::max<long long>(2 * n_build, 2));
-  const int logcap = log2_exact(cap);
-  const unsigned fill_blocks = (unsigned)std::min<uint64_t>((cap + 255) / 256, 4096);
-  {
-    PF_KERNEL("k_fill_i64", st);
-    k_fill_i64<<<fill_blocks, 256, 0, st>>>(l.table, EMPTY_KEY, (long long)cap);
-  }
-  if (l.mn) k_fill_i64<<<fill_blocks, 256, 0, st>>>(l.mn, LLONG_MAX, (long long)cap);
-  if (l.mx) k_fill_i64<<<fill_blocks, 256, 0, st>>>(l.mx, LLONG_MIN, (long long)cap);
   host_out[0] = 0;
-  host_out[1] = 0;  // the build below sets it through the alias
-  {
-    PF_KERNEL("k_set_build", st);
-    k_set_build<<<blocks_for(n_build, T), T, 0, st>>>((const long long*)build_key,
-                                                      (const long long*)build_val, n_build, l.table,
-                                                      l.mn, l.mx, logcap, host_dev + 1);
-  }
-  PF_LAUNCH("k_set_build");
+  host_out[1] = 0;  // the build sets it through the alias
+  auto queue = l.words == 1 ? sa_queue<1> : l.words == 2 ? sa_queue<2> : sa_queue<4>;
+  if (int rc = queue(l, build_key, n_build, probe_key, n_probe, build_val, probe_val, op,
+                     anti != 0, host_dev + 1, st))
+    return rc;
   const unsigned nblk = blocks_for(n_probe, CB);
   {
-    PF_KERNEL("k_set_probe", st);
-    k_set_probe<<<nblk, CT, 0, st>>>((const long long*)probe_key, (const long long*)probe_val,
-                                     n_probe, l.table, l.mn, l.mx, logcap, op, anti != 0, l.keep,
-                                     l.bcnt);
-  }
-  PF_LAUNCH("k_set_probe");
-  {
     PF_KERNEL("k_scan_counts", st);
-    k_scan_counts<<<1, 1024, 0, st>>>(l.bcnt, nblk, l.dev, host_dev);
+    k_scan_counts<<<1, 1024, 0, st>>>(l.bcnt, nblk, l.total, host_dev);
   }
   PF_LAUNCH("k_scan_counts");
   cudaEvent_t ev;
