@@ -7,7 +7,7 @@
 // by row group (every column's page of rows [g*rpp, (g+1)*rpp), in column
 // order).  Batches of row groups are copied to the device on a copy stream,
 // up to NSTAGE batches ahead, while the compute stream runs per batch:
-//   k_paged_hist     decode the filter and key columns of a quarter row group
+//   k_paged_hist     decode the filter and key columns of a part of a row group
 //                    per CTA, count the passing rows per bucket
 //   k_fscan-like     per bucket, each CTA's offset; bucket totals
 //   k_paged_place    the batch's place in the output (a device cursor) and
@@ -32,7 +32,12 @@ namespace {
 constexpr int QT = 512;              // threads of a decode CTA
 constexpr int QV = 8;                // rows a thread per sub-tile (blocked)
 constexpr int QSUB = QT * QV;        // 4096 rows: four PFC blocks
-constexpr int QPARTS = 4;            // CTAs per row group
+// CTAs a row group is cut into, at most: a CTA decodes its sub-tiles one after
+// the other behind barriers, two CTAs a SM, so short ones even out (61 groups of
+// 131072 rows: 4 a group 62 + 227 us, 8 51 + 150, 16 54 + 144 and twice the
+// offsets to scan).
+constexpr int QPARTS = 8;
+constexpr int QPAGE = 4 * QSUB;      // a page has a multiple of so many rows
 constexpr int MAXPC = 8;             // columns
 constexpr int NSTAGE = 3;
 
@@ -42,6 +47,7 @@ struct PagedArgs {
   long long batch_start;       // host byte offset of the batch
   long long g0, g1;            // the batch's row groups
   int ncols, rpp;
+  int parts;                   // CTAs a row group
   long long n_rows;
   int filter_col, key_col;
   long long lo, hi;            // filter: lo <= value < hi
@@ -182,11 +188,11 @@ __global__ void __launch_bounds__(QT) k_paged(PagedArgs a) {
   extern __shared__ __align__(16) unsigned char qsm[];
   QSmem& S = *reinterpret_cast<QSmem*>(qsm);
   if (SCATTER && *a.skip) return;
-  const long long g = a.g0 + blockIdx.x / QPARTS;
-  const int part = blockIdx.x % QPARTS;
+  const long long g = a.g0 + blockIdx.x / a.parts;
+  const int part = blockIdx.x % a.parts;
   const long long grow0 = g * a.rpp;
   const int rows_g = (int)min((long long)a.rpp, a.n_rows - grow0);
-  const int per = (a.rpp / QPARTS + QSUB - 1) / QSUB * QSUB;
+  const int per = (a.rpp / a.parts + QSUB - 1) / QSUB * QSUB;
   const int r_lo = part * per, r_hi = min(rows_g, r_lo + per);
   const int* hrow = a.hist + (long long)blockIdx.x * a.B;
   for (int b = threadIdx.x; b < a.B; b += QT) S.cnt[b] = 0;
@@ -197,7 +203,7 @@ __global__ void __launch_bounds__(QT) k_paged(PagedArgs a) {
   }
   __syncthreads();
   if (S.flag) {
-    if (threadIdx.x == 0 && !SCATTER) atomicAdd(&a.stats[2], 1ULL);
+    if (threadIdx.x == 0 && !SCATTER && part < QPAGE / QSUB) atomicAdd(&a.stats[2], 1ULL);
     if (!SCATTER)
       for (int b = threadIdx.x; b < a.B; b += QT) a.hist[(long long)blockIdx.x * a.B + b] = 0;
     return;
@@ -408,8 +414,8 @@ extern "C" int pf_paged_scan(const uint8_t* host_pages, const int64_t* directory
       key_col >= ncols || key_col == filter_col)
     return fail(PF_EINVAL, "paged_scan: bad columns");
   if (B < 1 || B > 4096 || (B & (B - 1))) return fail(PF_EINVAL, "paged_scan: B must be a power of two <= 4096");
-  if (rows_per_page < QSUB || rows_per_page % (QSUB * QPARTS))
-    return fail(PF_EINVAL, "paged_scan: rows_per_page must be a multiple of %d", QSUB * QPARTS);
+  if (rows_per_page < QSUB || rows_per_page % QPAGE)
+    return fail(PF_EINVAL, "paged_scan: rows_per_page must be a multiple of %d", QPAGE);
   if (groups_per_batch < 1 || n_groups < 1 || n_rows > n_groups * (int64_t)rows_per_page)
     return fail(PF_EINVAL, "paged_scan: bad sizes");
   if (esizes[key_col] != 8) return fail(PF_EINVAL, "paged_scan: the key column must be int64");
@@ -456,6 +462,7 @@ extern "C" int pf_paged_scan(const uint8_t* host_pages, const int64_t* directory
   a.dir = l.dir;
   a.ncols = ncols;
   a.rpp = rows_per_page;
+  a.parts = std::min(QPARTS, (int)(rows_per_page / QSUB));
   a.n_rows = n_rows;
   a.filter_col = filter_col;
   a.key_col = key_col;
@@ -488,7 +495,7 @@ extern "C" int pf_paged_scan(const uint8_t* host_pages, const int64_t* directory
     a.g0 = g0;
     a.g1 = g1;
     a.skip = l.skip + s;
-    const int ctas = (int)(g1 - g0) * QPARTS;
+    const int ctas = (int)(g1 - g0) * a.parts;
     {
       PF_KERNEL("k_paged_hist", st);
       k_paged<false><<<ctas, QT, smem, st>>>(a);
