@@ -780,10 +780,11 @@ __global__ void __launch_bounds__(PT, PF_PART_PLAIN_MINB) k_scatter_plain(Params
 // rows together takes 16.  A lane has eight rows in a row, loaded as one or two
 // vectors, and their buckets' counts as eight fields of a word, which the warp
 // adds up as such: the kernel is bound by its instructions as much as by its
-// bytes.  (16.8M rows of 8 + 8 + 4 + 1 bytes and the gidx into 8 buckets: 178
-// us, 4.7 TB/s; staged by the block 265, a row a lane with a ballot a bit of the
-// bucket 228; three or five blocks a SM 177 and 196.  The whole call 348 -> 247
-// us, under a mask of half the rows 644 -> 246.)
+// bytes.  (16.8M rows of 8 + 8 + 4 + 1 bytes and the gidx into 8 buckets: 168
+// us, 5.0 TB/s; staged by the block 265, a row a lane with a ballot a bit of the
+// bucket 228; with the flags, the offsets and the bases asked for where they are
+// used 178, then with three or five blocks a SM 177 and 196.  The whole call 348
+// -> 238 us, under a mask of half the rows 644 -> 243.)
 // MODE 0: every row, 1: those of a mask, 2: those of src (their numbers).
 constexpr int FB = 8;
 constexpr int FT = 256, FW = FT / 32, FI = SUB / FT, FSEG = 32 * FI;
@@ -928,7 +929,7 @@ __device__ __forceinline__ void few_hist(const Params& p, int (&h)[FW][FB]) {
 
 template <int MODE>
 __global__ void __launch_bounds__(FT) k_hist_few(Params p) {
-  if (failed(p)) return;
+  if (MODE == 2 && failed(p)) return;  // without a prologue nothing has failed yet
   __shared__ int h[FW][FB];
   if ((long long)(blockIdx.x + 1) * SUB <= p.ndom) few_hist<MODE, true>(p, h);
   else few_hist<MODE, false>(p, h);
@@ -970,6 +971,15 @@ __device__ __forceinline__ void few_scatter(const Params& p, FewWarp& S, int (&w
   const long long r0 = (long long)blockIdx.x * SUB + w * FSEG, i = r0 + lane * FI;
   int at[FI];
   unsigned long long v[FI] = {};
+  // the tile's place in the buckets' runs, in the lanes of the buckets: asked
+  // for first, as a warp lives for little more than its loads' latencies
+  unsigned place = 0, start[MAXCLS] = {};
+  if (lane < p.B) {
+    place = (unsigned)p.hist[(long long)blockIdx.x * p.B + lane];
+#pragma unroll
+    for (int cl = 0; cl < MAXCLS; ++cl)
+      if (cl < p.ncls) start[cl] = (unsigned)p.bases[(long long)cl * p.B + lane];
+  }
   const unsigned live = few_live<MODE, ALL>(p, i, at);
   unsigned bk, rank, count;
   {
@@ -982,6 +992,7 @@ __device__ __forceinline__ void few_scatter(const Params& p, FewWarp& S, int (&w
     } else {
       few_column<MODE, ALL>(p, p.c.in[0], p.c.rb[0], i, live, at, v);
     }
+    if (MODE != 2 && failed(p)) return;
     few_buckets<EVERY>(p.logB, key, live, bk, rank, count);
   }
   // each bucket's rows in the lanes before, a byte a bucket (248 at most)
@@ -1029,10 +1040,11 @@ __device__ __forceinline__ void few_scatter(const Params& p, FewWarp& S, int (&w
     }
   }
   if (lane < p.B) {
-    unsigned d = (unsigned)p.hist[(long long)blockIdx.x * p.B + lane] - (unsigned)first;
+    unsigned d = place - (unsigned)first;
     for (int q = 0; q < w; ++q) d += (unsigned)wh[q][lane];
-    for (int cl = 0; cl < p.ncls; ++cl)
-      S.dst[cl][lane] = d + (unsigned)p.bases[(long long)cl * p.B + lane];
+#pragma unroll
+    for (int cl = 0; cl < MAXCLS; ++cl)
+      if (cl < p.ncls) S.dst[cl][lane] = d + start[cl];
   }
   __syncwarp();
   unsigned meta[FI];
@@ -1071,7 +1083,7 @@ __device__ __forceinline__ void few_scatter(const Params& p, FewWarp& S, int (&w
 
 template <int MODE>
 __global__ void __launch_bounds__(FT, 4) k_scatter_few(Params p) {
-  if (failed(p)) return;
+  if (MODE == 2 && failed(p)) return;  // else few_scatter looks, its loads on the way
   __shared__ __align__(16) FewWarp warps[FW];
   __shared__ int wh[FW][FB];
   FewWarp& S = warps[threadIdx.x >> 5];
