@@ -145,8 +145,8 @@ struct Own {
         S.lo[c] = S.hi[c] = S.cnt[c] = 0;
       }
       if (!n) continue;
-      atomicAdd(&slab[2 * g], sum);
-      atomicAdd(&slab[2 * g + 1], n);
+      red_add(&slab[2 * g], sum);
+      red_add(&slab[2 * g + 1], n);
     }
     __syncthreads();
   }

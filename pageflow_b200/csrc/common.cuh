@@ -31,6 +31,27 @@ __host__ __device__ __forceinline__ int bucket_of_hash(uint64_t h, int logB) {
   return logB ? (int)(h >> (64 - logB)) : 0;
 }
 
+// Adds to global memory without an answer.  An atomicAdd on a pointer that came
+// out of a descriptor, which the compiler takes for any kind of memory, becomes
+// one that fetches the old value (about 100 G/s into L2, these 140): the serving
+// kernel's 487M rows 3260 -> 2850 us, 48 batch instances 5380 -> 5200, a keyed
+// tick of 4M rows 203 -> 182.
+__device__ __forceinline__ void red_add(unsigned long long* p, unsigned long long v) {
+  asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(__cvta_generic_to_global(p)),
+               "l"(v)
+               : "memory");
+}
+__device__ __forceinline__ void red_max(long long* p, long long v) {
+  asm volatile("red.relaxed.gpu.global.max.s64 [%0], %1;" ::"l"(__cvta_generic_to_global(p)),
+               "l"(v)
+               : "memory");
+}
+__device__ __forceinline__ void red_add(double* p, double v) {
+  asm volatile("red.relaxed.gpu.global.add.f64 [%0], %1;" ::"l"(__cvta_generic_to_global(p)),
+               "d"(v)
+               : "memory");
+}
+
 __device__ __forceinline__ unsigned lanemask_lt() {
   unsigned r;
   asm("mov.u32 %0, %%lanemask_lt;" : "=r"(r));

@@ -1,6 +1,6 @@
 // A hash table of 8-byte entries over unique int64 keys with a small group
 // number each, shared by the joins that keep one in L2 or HBM (join_direct.cu,
-// batch.cu).
+// batch.cu, serve.cu).
 //
 // 2^q buckets of four entries, a bucket one 32-byte sector.  A key's hash is a
 // bijection of it, so its top q bits (the home bucket) and the 64 - q others
