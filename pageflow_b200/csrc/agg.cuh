@@ -22,7 +22,7 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
 // a RED every 14 clocks, while groups met once an item would fill the cells),
 // OWN_COPIES copies of each.  The cells are flushed into the (sum, count) slab
 // at an item's end; the hot groups' places stay for the block's next item of
-// the same source.  (48 batch instances: 5.6 ms; 256 groups of 4 copies 5.8,
+// the same source.  (48 batch instances: 512 groups of 2 copies 5.6 ms, 256 of 4 5.8,
 // and twice the time with 54 KB of cells, whose blocks leave no L1.  Serving:
 // 2048 cells no faster, 4096 a tenth slower.)
 constexpr int OWN_CELLS = 1024;
