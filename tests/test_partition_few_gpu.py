@@ -2,8 +2,10 @@
 does not, every word width, masks and both prologues, sizes around a warp's
 segment and a tile, against the oracle, bit for bit."""
 import pytest
+import torch
 
-from tests.test_partition_gpu import _check, _mask, _table
+from tests.dropin import partition
+from tests.test_partition_gpu import _check, _contradicted, _mask, _table
 
 pytestmark = pytest.mark.gpu
 
@@ -38,3 +40,16 @@ def test_columns_off_their_words(offset):
     kernel's copies."""
     cols = [c[offset:] for c in _table(30_000, ["i32", "i16", "u8x8", "u8x3"], seed=9)]
     _check(cols, 0, None, 0, 8)
+
+
+@pytest.mark.parametrize("select_first", [False, True])
+@pytest.mark.parametrize("off", [-37, 41])
+def test_a_contradicted_count_writes_nothing_past_it(select_first, off):
+    n = 60_003
+    cols = _table(n, ["i64", "i8"], seed=91)
+    mask = _mask(n, 0.2, seed=92)
+    wrong = int(mask.sum()) + off
+    call = partition(list(cols), 0, mask, 0, 8, n_valid=wrong, select_first=select_first)
+    torch.cuda.synchronize()
+    assert _contradicted(call, wrong)
+    _check(cols, 0, mask, 0, 8, compact=[False] * 3, count=True, select_first=select_first)
