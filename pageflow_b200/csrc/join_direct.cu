@@ -23,8 +23,9 @@
 // groups: count and sum in one 64-bit word {count, sum}, one RED a row instead
 // of two.  That is exact or known not to be: with every value in [0, 2^s) (s
 // the sum's bits; any other raises a word) group g's word gives the count
-// C_g + floor(S_g / 2^s) modulo 2^(64 - s), so the counts add up to the matched
-// rows, counted by themselves, only if no sum left its field; a wrapped count
+// C_g + floor(S_g / 2^s) modulo 2^(64 - s), so the counts add up to the rows put
+// into the words, counted by themselves (a matched row whose build row has no
+// group in the range is in none), only if no sum left its field; a wrapped count
 // would need sums of 2^64 in all, which a bound on them (added up by
 // themselves too) excludes.  Where the check fails the call runs again with
 // two words a group.  Groups that a block meets often (skewed keys) go through
@@ -65,8 +66,8 @@ struct DjHead {
   unsigned gave_up;             // k_dj_finish: a wait on another tile ran out
   unsigned ticket, done;        // its tiles taken and done
   unsigned pad;
-  unsigned long long matched;
-  unsigned long long high;      // sum of value >> 20 over the matched rows
+  unsigned long long rows;      // rows put into packed words
+  unsigned long long high;      // sum of their values >> 20
   unsigned long long counts;    // the groups' counts added up
   long long groups;             // occupied groups
 };
@@ -149,7 +150,7 @@ __global__ void __launch_bounds__(DT, PF_DJ_MINB) k_dj_probe(DjArgs a) {
                                  : a.slab + (unsigned long long)(blockIdx.x % a.reps) *
                                                 (unsigned long long)a.G *
                                                 (MODE == SUM_PACKED ? 1 : 2);
-  unsigned matched = 0;
+  unsigned matched = 0, rows = 0;
   unsigned long long high = 0;
   bool outside = false, cached = false;
   const long long tile = (long long)DT * DR, first = (long long)blockIdx.x * tile;
@@ -205,6 +206,7 @@ __global__ void __launch_bounds__(DT, PF_DJ_MINB) k_dj_probe(DjArgs a) {
       if (MODE == SUM_PACKED) {
         outside |= (unsigned long long)v[r] >> a.sbits != 0;
         high += (unsigned long long)v[r] >> 20;
+        ++rows;
       }
       const unsigned s = (g * 0x9E3779B1u) >> 22;  // of DJ_CACHE = 1024
       if (cached) {
@@ -264,26 +266,31 @@ __global__ void __launch_bounds__(DT, PF_DJ_MINB) k_dj_probe(DjArgs a) {
     }
   }
   // the block's counts, one atomic each
-  __shared__ unsigned long long red[2][DT / 32];
-  unsigned long long m = matched;
+  __shared__ unsigned long long red[3][DT / 32];
+  unsigned long long m = matched, in = rows;
   for (int o = 16; o; o >>= 1) {
     m += __shfl_xor_sync(FULL, m, o);
-    if (MODE == SUM_PACKED) high += __shfl_xor_sync(FULL, high, o);
+    if (MODE == SUM_PACKED) {
+      in += __shfl_xor_sync(FULL, in, o);
+      high += __shfl_xor_sync(FULL, high, o);
+    }
   }
   if (lane == 0) {
     red[0][tid >> 5] = m;
-    red[1][tid >> 5] = high;
+    red[1][tid >> 5] = in;
+    red[2][tid >> 5] = high;
   }
   if (MODE == SUM_PACKED && outside) a.head->bad_value = 1;
   __syncthreads();
   if (tid == 0) {
     for (int w = 1; w < DT / 32; ++w) {
       m += red[0][w];
-      high += red[1][w];
+      in += red[1][w];
+      high += red[2][w];
     }
     if (m) atomicAdd(&a.stats[0], m);
     if (MODE == SUM_PACKED) {
-      if (m) atomicAdd(&a.head->matched, m);
+      if (in) atomicAdd(&a.head->rows, in);
       if (high) atomicAdd(&a.head->high, high);
     }
   }
@@ -494,7 +501,7 @@ __global__ void __launch_bounds__(DT) k_dj_finish(DjArgs a, DjOut o) {
     o.host->overflow = h->overflow;
     o.host->bad_value = h->bad_value;
     o.host->gave_up = h->gave_up;
-    o.host->matched = h->matched;
+    o.host->rows = h->rows;
     o.host->high = h->high;
     o.host->counts = h->counts;
     o.host->groups = h->groups;
@@ -669,8 +676,8 @@ extern "C" int pf_join_direct(const int64_t* build_key, const int32_t* build_gro
     if (int rc = wait_stream(st)) return rc;
     if (host->gave_up) return fail(PF_EDEVICE, "join_direct: a device wait gave up");
     if (host->overflow) return ok();  // *done = 0
-    if (!packed || (!host->bad_value && host->counts == host->matched &&
-                    host->high + host->matched < 1ULL << 43)) {
+    if (!packed || (!host->bad_value && host->counts == host->rows &&
+                    host->high + host->rows < 1ULL << 43)) {
       *done = 1;
       if (n_out) *n_out = host->groups;
       return ok();
