@@ -324,9 +324,10 @@ int pf_join_aggregate_ex(const int64_t* build_key, const int32_t* build_group, i
  * the largest table, half a million groups at most; 0 else): one table over all
  * build rows, each probe row looked up in it.  Outputs as
  * pf_join_aggregate's and, with keys_out, the occupied groups as
- * pf_groups_finish's (*n_out of them, host).  Waits once.  *done (host) is 0
- * when the build keys' hashes crowd its table: nothing was joined, take
- * pf_join_aggregate.
+ * pf_groups_finish's (*n_out of them, host).  Waits once, and once more where
+ * the one-word sums of more than 2048 groups left their fields, after which it
+ * runs again with two words a group.  *done (host) is 0 when the build keys'
+ * hashes crowd its table: nothing was joined, take pf_join_aggregate.
  */
 int pf_join_direct_fits(int64_t n_build, int64_t n_probe, int64_t n_groups);
 size_t pf_join_direct_workspace(int64_t n_build, int64_t n_groups);

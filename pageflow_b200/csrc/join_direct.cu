@@ -21,17 +21,18 @@
 // copies of a group as fit, a lane its own, so a warp's lanes meet on no
 // address), flushed once into one of DJ_REPS copies in global memory.  More
 // groups: count and sum in one 64-bit word {count, sum}, one RED a row instead
-// of two.  That is exact or known not to be: with every value in [0, 2^s) (s
-// the sum's bits; any other raises a word) group g's word gives the count
-// C_g + floor(S_g / 2^s) modulo 2^(64 - s), so the counts add up to the rows put
-// into the words, counted by themselves (a matched row whose build row has no
-// group in the range is in none), only if no sum left its field; a wrapped count
-// would need sums of 2^64 in all, which a bound on them (added up by
-// themselves too) excludes.  Where the check fails the call runs again with
-// two words a group.  Groups that a block meets often (skewed keys) go through
-// a cache in shared memory, so that they do not queue up on one address;
-// up to 64K groups have several copies of their sums, so that four groups'
-// words of a sector do not queue up (18M rows into 5000 groups: 488 -> 354 us).
+// of two, s bits of sum.  That is exact or known not to be: group g's word gives
+// the count C_g + floor(S_g / 2^s) modulo 2^(64 - s).  Values of [0, 2^v) alone go
+// into words, v chosen so that all of them add up to less than 2^63: what the
+// sums carry into the counts is then less than a wrapped count takes away, and the
+// counts add up to the rows put into the words, counted by themselves, only if no
+// field was left.  (A matched row whose build row has no group in the range is in
+// none.)  Where they do not, the call runs again with two words a group.
+// Other values go into a pair {sum, count} of the group, and so do the groups that a
+// block meets often (skewed keys or groups), collected in shared memory, so that
+// they neither queue up on one address nor fill a count's field.  Up to 64K groups
+// have several copies of their words, so that four groups' words of a sector do not
+// queue up (18M rows into 5000 groups: 488 -> 354 us).
 #include <algorithm>
 #include <climits>
 
@@ -57,17 +58,26 @@ constexpr int DJ_SMALL = 2048;         // groups summed in shared memory
 constexpr int DJ_REPS = 8;             // global copies of their sums
 constexpr int DJ_SPREAD = 1 << 17;     // words that a few groups' sums are spread over
 constexpr int DJ_MAX_REPS = 32;
-constexpr int DJ_CACHE = 1024;         // cached groups a block
-constexpr int DJ_REPEATS = 16;         // of a block's first rows, for the cache
+// A block's cache of its hot groups.  In the block's first DJ_LOOK steps (4096
+// rows) a group that comes again before another one of its `seen` entry gets a
+// cell, which one of a share of 0.1% or more soon does and one of 100K equal ones
+// hardly ever; the cells stay in use where DJ_HITS threads found theirs by then (a
+// share of 0.2% in all), else the other steps do without.  3M x 20M rows into 100K
+// groups, the radix path's time after it: equal ones 350 us (600), one of 1% 358
+// (614), one of 10% 385 (917), Zipf 1.0 594 (1379); with a cache taken into use by
+// the first 512 rows alone and emptied into the packed words, whose counts it then
+// overfilled, so that the call ran twice: 350, 1065, 798 and 1251.
+constexpr int DJ_CACHE = 1024;
+constexpr int DJ_LOOK = 8;
+constexpr int DJ_HITS = 8;
 
 struct DjHead {
   unsigned overflow;            // a build row found no entry
-  unsigned bad_value;           // packed sums: a value outside [0, 2^s)
+  unsigned pairs;               // packed sums: some are in the groups' pairs
   unsigned gave_up;             // k_dj_finish: a wait on another tile ran out
   unsigned ticket, done;        // its tiles taken and done
   unsigned pad;
   unsigned long long rows;      // rows put into packed words
-  unsigned long long high;      // sum of their values >> 20
   unsigned long long counts;    // the groups' counts added up
   long long groups;             // occupied groups
 };
@@ -82,9 +92,10 @@ struct DjArgs {
   long long scale, np;
   CompactTable table;
   long long gmin, G;
-  unsigned long long* slab;     // pairs (small, wide) or packed words
-  int sbits;                    // packed: bits of the sum
-  int reps;                     // copies of the sums, a block's own by its number
+  unsigned long long* slab;     // the groups' pairs [preps][2 * G]
+  unsigned long long* packed;   // and packed words [reps][G]
+  int sbits, vbits;             // packed: bits of the sum, of a value
+  int reps, preps;              // copies, a block's own by its number
   int copies;                   // small: copies of a group in shared memory, log2
   unsigned long long* stats;
   DjHead* head;
@@ -139,22 +150,27 @@ __global__ void __launch_bounds__(DT, PF_DJ_MINB) k_dj_probe(DjArgs a) {
   unsigned* hi = lo + cells;
   unsigned* cnt = hi + cells;
   int* tag = reinterpret_cast<int*>(cnt + cells);  // the cache's groups
+  unsigned short* seen = reinterpret_cast<unsigned short*>(tag + cells);
   for (int i = tid; i < cells; i += DT) {
     lo[i] = hi[i] = cnt[i] = 0;
-    if (MODE != SUM_SMALL) tag[i] = -1;
+    if (MODE != SUM_SMALL) {
+      tag[i] = -1;
+      seen[i] = 0;
+    }
   }
   __syncthreads();
   const unsigned copy = lane & ((1u << a.copies) - 1);
-  unsigned long long* slab = MODE == SUM_SMALL
-                                 ? nullptr
-                                 : a.slab + (unsigned long long)(blockIdx.x % a.reps) *
-                                                (unsigned long long)a.G *
-                                                (MODE == SUM_PACKED ? 1 : 2);
+  const unsigned long long G = (unsigned long long)a.G;
+  unsigned long long* pairs = a.slab + 2 * G * (unsigned)(blockIdx.x % a.preps);
+  unsigned long long* packed = a.packed + G * (unsigned)(blockIdx.x % a.reps);
   unsigned matched = 0, rows = 0;
-  unsigned long long high = 0;
-  bool outside = false, cached = false;
-  const long long tile = (long long)DT * DR, first = (long long)blockIdx.x * tile;
-  for (long long t0 = first; t0 < a.np; t0 += (long long)gridDim.x * tile) {
+  int hits = 0, steps = 0;
+  bool paired = false, look = MODE != SUM_SMALL, cached = false;
+  const long long tile = (long long)DT * DR;
+  // a block's first step, before its hot groups have cells, would overfill a hot
+  // group's count: its rows go into pairs where they are an eighth at most
+  int vbits = a.np >= DJ_LOOK * (long long)gridDim.x * tile ? 0 : a.vbits;
+  for (long long t0 = (long long)blockIdx.x * tile; t0 < a.np; t0 += (long long)gridDim.x * tile) {
     unsigned long long h[DR], want[DR];
     long long v[DR];
     CtBucket k[DR];
@@ -187,7 +203,6 @@ __global__ void __launch_bounds__(DT, PF_DJ_MINB) k_dj_probe(DjArgs a) {
       want[r] = ct_want(a.table, h[r]);
       k[r] = ct_load(ct_home(a.table, h[r]));
     }
-    int repeats = 0;
 #pragma unroll
     for (int r = 0; r < DR; ++r) {
       if (!live[r]) continue;
@@ -203,43 +218,38 @@ __global__ void __launch_bounds__(DT, PF_DJ_MINB) k_dj_probe(DjArgs a) {
         add_shared(lo, hi, cnt, g << a.copies | copy, v[r]);
         continue;
       }
-      if (MODE == SUM_PACKED) {
-        outside |= (unsigned long long)v[r] >> a.sbits != 0;
-        high += (unsigned long long)v[r] >> 20;
-        ++rows;
-      }
-      const unsigned s = (g * 0x9E3779B1u) >> 22;  // of DJ_CACHE = 1024
-      if (cached) {
-        int t = *(volatile int*)&tag[s];
-        if (t == -1) {
-          t = atomicCAS(&tag[s], -1, (int)g);
-          if (t == -1) t = (int)g;
-        }
+      if (look || cached) {
+        const unsigned mixed = g * 0x9E3779B1u, c = mixed >> 22;  // of DJ_CACHE = 1024
+        const int t = *(volatile int*)&tag[c];
         if (t == (int)g) {
-          add_shared(lo, hi, cnt, s, v[r]);
+          add_shared(lo, hi, cnt, c, v[r]);
+          ++hits;
           continue;
         }
-      } else if (t0 == first) {
-        // the block's first rows: how often a group comes again
-        repeats += *(volatile int*)&tag[s] == (int)g;
-        *(volatile int*)&tag[s] = (int)g;
+        if (look) {
+          volatile unsigned short* last = &seen[c];
+          const unsigned short me = (unsigned short)(mixed >> 6);
+          if (*last != me) *last = me;
+          else if (t == -1) atomicCAS(&tag[c], -1, (int)g);
+        }
       }
-      if (MODE == SUM_PACKED) {
-        atomicAdd(&slab[g], (1ULL << a.sbits) + (unsigned long long)v[r]);
+      if (MODE == SUM_PACKED && (unsigned long long)v[r] >> vbits == 0) {
+        ++rows;
+        red_add(&packed[g], (1ULL << a.sbits) + (unsigned long long)v[r]);
       } else {
-        atomicAdd(&slab[2 * (unsigned long long)g], (unsigned long long)v[r]);
-        atomicAdd(&slab[2 * (unsigned long long)g + 1], 1ULL);
+        paired = true;
+        red_add(&pairs[2 * (unsigned long long)g], (unsigned long long)v[r]);
+        red_add(&pairs[2 * (unsigned long long)g + 1], 1ULL);
       }
     }
-    if (MODE != SUM_SMALL && t0 == first) {
-      cached = __syncthreads_count(repeats > 0) >= DJ_REPEATS;
-      for (int i = tid; i < cells; i += DT) tag[i] = -1;
-      __syncthreads();
+    vbits = a.vbits;
+    if (MODE != SUM_SMALL && ++steps == DJ_LOOK) {
+      look = false;
+      cached = __syncthreads_count(hits > 0) >= DJ_HITS;
     }
   }
   __syncthreads();
   if (MODE == SUM_SMALL) {
-    unsigned long long* rep = a.slab + 2ULL * (blockIdx.x % DJ_REPS) * (unsigned long long)a.G;
     for (int g = tid; g < (int)a.G; g += DT) {
       unsigned long long s = 0, c = 0;
       for (int j = 0; j < 1 << a.copies; ++j) {
@@ -248,51 +258,41 @@ __global__ void __launch_bounds__(DT, PF_DJ_MINB) k_dj_probe(DjArgs a) {
         c += cnt[x];
       }
       if (c) {
-        atomicAdd(&rep[2 * g], s);
-        atomicAdd(&rep[2 * g + 1], c);
+        atomicAdd(&pairs[2 * g], s);
+        atomicAdd(&pairs[2 * g + 1], c);
       }
     }
-  } else if (cached) {
+  } else {
     for (int i = tid; i < cells; i += DT) {
       const int g = tag[i];
       if (g < 0) continue;
       const unsigned long long s = (unsigned long long)hi[i] << 32 | lo[i], c = cnt[i];
-      if (MODE == SUM_PACKED) {
-        atomicAdd(&slab[g], (c << a.sbits) + s);
-      } else {
-        atomicAdd(&slab[2 * (unsigned long long)g], s);
-        atomicAdd(&slab[2 * (unsigned long long)g + 1], c);
-      }
+      if (!c) continue;
+      paired = true;
+      red_add(&pairs[2 * (unsigned long long)g], s);
+      red_add(&pairs[2 * (unsigned long long)g + 1], c);
     }
   }
   // the block's counts, one atomic each
-  __shared__ unsigned long long red[3][DT / 32];
+  __shared__ unsigned long long red[2][DT / 32];
   unsigned long long m = matched, in = rows;
   for (int o = 16; o; o >>= 1) {
     m += __shfl_xor_sync(FULL, m, o);
-    if (MODE == SUM_PACKED) {
-      in += __shfl_xor_sync(FULL, in, o);
-      high += __shfl_xor_sync(FULL, high, o);
-    }
+    if (MODE == SUM_PACKED) in += __shfl_xor_sync(FULL, in, o);
   }
   if (lane == 0) {
     red[0][tid >> 5] = m;
     red[1][tid >> 5] = in;
-    red[2][tid >> 5] = high;
   }
-  if (MODE == SUM_PACKED && outside) a.head->bad_value = 1;
+  if (MODE == SUM_PACKED && paired) a.head->pairs = 1;
   __syncthreads();
   if (tid == 0) {
     for (int w = 1; w < DT / 32; ++w) {
       m += red[0][w];
       in += red[1][w];
-      high += red[2][w];
     }
     if (m) atomicAdd(&a.stats[0], m);
-    if (MODE == SUM_PACKED) {
-      if (in) atomicAdd(&a.head->rows, in);
-      if (high) atomicAdd(&a.head->high, high);
-    }
+    if (MODE == SUM_PACKED && in) atomicAdd(&a.head->rows, in);
   }
 }
 
@@ -395,26 +395,27 @@ __global__ void __launch_bounds__(DT) k_dj_finish(DjArgs a, DjOut o) {
   unsigned long long s[FG], c[FG], total = 0;
   int mine = 0;
 #pragma unroll
-  for (int k = 0; k < FG; ++k) {
-    s[k] = c[k] = 0;
-    if (g0 + k >= a.G) continue;
-    if (PACKED) {
-      s[k] = a.slab[g0 + k];
-    } else {
-      const ulonglong2 x = reinterpret_cast<const ulonglong2*>(a.slab)[g0 + k];
-      s[k] = x.x;
-      c[k] = x.y;
+  for (int k = 0; k < FG; ++k) s[k] = c[k] = 0;
+  if (PACKED) {
+    for (int r = 0; r < a.reps; ++r) {
+#pragma unroll
+      for (int k = 0; k < FG; ++k)
+        if (g0 + k < a.G) s[k] += a.packed[(long long)r * a.G + g0 + k];
     }
-  }
-  for (int r = 1; r < a.reps; ++r) {
 #pragma unroll
     for (int k = 0; k < FG; ++k) {
-      if (g0 + k >= a.G) continue;
-      const long long at = (long long)r * a.G + g0 + k;
-      if (PACKED) {
-        s[k] += a.slab[at];
-      } else {
-        const ulonglong2 x = reinterpret_cast<const ulonglong2*>(a.slab)[at];
+      c[k] = s[k] >> a.sbits;
+      s[k] &= smask;
+      total += c[k];
+    }
+  }
+  if (!PACKED || a.head->pairs) {
+    for (int r = 0; r < a.preps; ++r) {
+#pragma unroll
+      for (int k = 0; k < FG; ++k) {
+        if (g0 + k >= a.G) continue;
+        const ulonglong2 x =
+            reinterpret_cast<const ulonglong2*>(a.slab)[(long long)r * a.G + g0 + k];
         s[k] += x.x;
         c[k] += x.y;
       }
@@ -422,14 +423,7 @@ __global__ void __launch_bounds__(DT) k_dj_finish(DjArgs a, DjOut o) {
   }
 #pragma unroll
   for (int k = 0; k < FG; ++k) {
-    if (!PACKED) break;
-    c[k] = s[k] >> a.sbits;
-    s[k] &= smask;
-  }
-#pragma unroll
-  for (int k = 0; k < FG; ++k) {
     if (g0 + k >= a.G) continue;
-    total += c[k];
     mine += c[k] > 0;
     o.sum[g0 + k] = (long long)s[k];
     o.count[g0 + k] = (long long)c[k];
@@ -499,10 +493,8 @@ __global__ void __launch_bounds__(DT) k_dj_finish(DjArgs a, DjOut o) {
     __threadfence();
     volatile DjHead* h = a.head;
     o.host->overflow = h->overflow;
-    o.host->bad_value = h->bad_value;
     o.host->gave_up = h->gave_up;
     o.host->rows = h->rows;
-    o.host->high = h->high;
     o.host->counts = h->counts;
     o.host->groups = h->groups;
   }
@@ -513,7 +505,7 @@ struct DjLayout {
   unsigned long long* table;
   unsigned long long* slab;
   unsigned long long* tiles;
-  int q, gbits, dbits, ntiles, reps;
+  int q, gbits, dbits, ntiles, reps, preps;
 };
 
 // The table's bits for nb build rows and groups of g bits, or q = 0.
@@ -537,7 +529,9 @@ DjLayout dj_layout(Arena& a, long long nb, long long G) {
   l.table = a.take<unsigned long long>(l.q ? (size_t)4 << l.q : 1);
   l.reps = G <= DJ_SMALL ? DJ_REPS
                          : (int)std::max<long long>(1, std::min<long long>(DJ_MAX_REPS, DJ_SPREAD / G));
-  const long long words = 2LL * l.reps * G;
+  // the packed form's copies of the words, and half as many of the pairs
+  l.preps = std::max(1, l.reps / 2);
+  const long long words = std::max(2LL * l.reps, 2LL * l.preps + l.reps) * G;
   l.slab = a.take<unsigned long long>((size_t)std::max<long long>(words, 1));
   l.ntiles = G <= DJ_SMALL ? 0 : (int)((G + FTILE - 1) / FTILE);
   l.tiles = a.take<unsigned long long>((size_t)l.ntiles + 1);
@@ -556,7 +550,7 @@ DjHead* pinned_dj_head() {
 
 template <int MODE>
 int dj_probe(const DjArgs& a, cudaStream_t st) {
-  const size_t smem = MODE == SUM_SMALL ? (size_t)3 * 4 * (a.G << a.copies) : 4 * 4 * DJ_CACHE;
+  const size_t smem = MODE == SUM_SMALL ? (size_t)3 * 4 * (a.G << a.copies) : 18 * DJ_CACHE;
   auto kern = a.disc ? k_dj_probe<MODE, true> : k_dj_probe<MODE, false>;
   if (int rc = opt_in_smem((const void*)kern, smem)) return rc;
   int per_sm = 0;
@@ -632,14 +626,16 @@ extern "C" int pf_join_direct(const int64_t* build_key, const int32_t* build_gro
   a.head = l.head;
   a.tiles = l.tiles;
   a.ntiles = l.ntiles;
-  a.reps = l.reps;
   const bool small = n_groups <= DJ_SMALL;
-  // packed: the count's field for 16 times the mean rows a group (or for all
-  // rows), where that leaves a mean group's sum 31 bits a value: else the check
-  // would fail on ordinary values, and the call run twice
+  // packed: the count's field for a 256th of the rows (a larger group is hot), for
+  // 2^17 and for 16 times the mean of a group (or for all rows), where that leaves a
+  // mean group's sum 31 bits a value: else the check would fail on ordinary values,
+  // and the call run twice
+  const int all = bits_of((unsigned long long)n_probe);
   const int mean = bits_of((unsigned long long)(n_probe / n_groups));
-  a.sbits = 64 - std::min(bits_of((unsigned long long)n_probe), mean + 4);
+  a.sbits = 64 - std::min(all, std::max(mean + 4, std::min(std::max(17, all - 8), 33 - mean)));
   const bool pack = a.sbits - mean >= 31;
+  a.vbits = std::min(a.sbits - mean - 2, 63 - all);
   while (a.copies < 5 && (n_groups << (a.copies + 1)) <= DJ_SMALL) ++a.copies;
   DjOut o{(long long*)sum_out, (long long*)count_out, (long long*)keys_out, (long long*)sums_out,
           (long long*)counts_out, host_dev};
@@ -647,7 +643,10 @@ extern "C" int pf_join_direct(const int64_t* build_key, const int32_t* build_gro
   *done = 0;
   for (int attempt = small || pack ? 0 : 1; attempt < 2; ++attempt) {
     const bool packed = !small && attempt == 0;
-    const long long words = (packed ? 1LL : 2LL) * l.reps * n_groups;
+    a.reps = packed ? l.reps : 1;
+    a.preps = packed ? l.preps : l.reps;
+    a.packed = l.slab + 2LL * a.preps * n_groups;
+    const long long words = (2LL * a.preps + (packed ? l.reps : 0)) * n_groups;
     {
       const long long work = (4LL << a.table.q) / 2 + words;
       PF_KERNEL("k_dj_init", st);
@@ -676,8 +675,7 @@ extern "C" int pf_join_direct(const int64_t* build_key, const int32_t* build_gro
     if (int rc = wait_stream(st)) return rc;
     if (host->gave_up) return fail(PF_EDEVICE, "join_direct: a device wait gave up");
     if (host->overflow) return ok();  // *done = 0
-    if (!packed || (!host->bad_value && host->counts == host->rows &&
-                    host->high + host->rows < 1ULL << 43)) {
+    if (!packed || host->counts == host->rows) {
       *done = 1;
       if (n_out) *n_out = host->groups;
       return ok();

@@ -67,3 +67,45 @@ def test_rows_without_a_group_cost_no_second_run():
     bgrp[1] = -1
     fk = rng.integers(0, 22_000, 200_000)
     assert _run(bkey, bgrp, fk, rng.integers(0, 1 << 24, 200_000), 4000) == ATTEMPT
+
+
+def _groups(kind, n, G, rng):
+    g = rng.integers(0, G, n)
+    if kind == "zipf":
+        w = 1.0 / np.arange(1, G + 1)
+        g = np.searchsorted(np.cumsum(w) / w.sum(), rng.random(n)).clip(max=G - 1)
+    elif kind != "equal":
+        g[rng.random(n) < float(kind)] = 7
+    return g.astype(np.int32)
+
+
+@pytest.mark.parametrize("kind", ["equal", "zipf", "0.002", "0.01", "0.1", "0.6"])
+@pytest.mark.parametrize("np_", [60_000, 900_001, 4_000_000])
+def test_skewed_groups_cost_no_second_run(kind, np_):
+    rng = np.random.default_rng(np_)
+    nb, G = 150_001, 5000
+    fk = rng.integers(0, nb + nb // 10, np_)
+    assert _run(rng.permutation(nb).astype(np.int64), _groups(kind, nb, G, rng), fk,
+                rng.integers(0, 1 << 24, np_), G) == ATTEMPT
+
+
+@pytest.mark.parametrize("np_", [900_001, 4_000_000])
+def test_skewed_keys_cost_no_second_run(np_):
+    rng = np.random.default_rng(np_)
+    nb, G = 150_001, 5000
+    fk = (rng.random(np_) ** 40 * nb).astype(np.int64)
+    assert _run(rng.permutation(nb).astype(np.int64), _groups("equal", nb, G, rng), fk,
+                rng.integers(0, 1 << 24, np_), G) == ATTEMPT
+
+
+@pytest.mark.parametrize("lo,hi", [(-1000, 1000), (-5, 0), (-(1 << 63), (1 << 63) - 1),
+                                   (1 << 55, 1 << 60)])
+@pytest.mark.parametrize("every", [1, 1000])
+@pytest.mark.parametrize("np_", [200_000, 4_000_000])
+def test_values_outside_a_packed_words_cost_no_second_run(lo, hi, every, np_):
+    rng = np.random.default_rng(5)
+    nb, G = 20_001, 3000
+    price = rng.integers(0, 1 << 24, np_)
+    price[::every] = rng.integers(lo, hi, len(price[::every]), endpoint=True)
+    assert _run(rng.permutation(nb).astype(np.int64), _groups("equal", nb, G, rng),
+                rng.integers(0, nb, np_), price, G) == ATTEMPT
