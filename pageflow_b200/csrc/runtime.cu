@@ -169,7 +169,7 @@ int wait_event(cudaEvent_t ev) {
     const int64_t us = std::chrono::duration_cast<std::chrono::microseconds>(
                            std::chrono::steady_clock::now() - t0)
                            .count();
-    if (us > limit * 1000)
+    if (us / 1000 > limit)  // any limit in milliseconds, the largest too
       return fail(PF_ETIMEOUT, "the stream did not reach the call's event within %lld ms",
                   (long long)limit);
     if (us > SPIN_US) std::this_thread::sleep_for(std::chrono::microseconds(50));
