@@ -211,6 +211,16 @@ class KeyedPass1:
         return (bytes((_native.KeyedAcc * max(1, len(accs)))(*accs)), source,
                 bytes((_native.KeyedOut * max(1, len(outs)))(*outs)), dest, results)
 
+    def _layout_of(self, keys, cols):
+        """_layout's answer, kept for the last types and widths (it depends on
+        nothing else); another thread may keep its own meanwhile."""
+        sig = (tuple((k.dtype, k.shape[1]) for k in keys),
+               tuple(v.dtype for v in cols.values()))
+        laid = self._laid
+        if laid is None or laid[0] != sig:
+            laid = self._laid = (sig, self._layout(dict(zip(self.key_ids, keys)), cols))
+        return laid[1]
+
     def _one_read(self, columns, keys, B=1):
         """pass1 by pf_keyed_pass1_read, or None when a column's type or shape or
         the number of groups is not its."""
@@ -224,12 +234,7 @@ class KeyedPass1:
         if any(v.dim() != 1 or v.shape[0] != n or v.device != dev or v.dtype not in _KK
                for v in cols.values()):
             return None
-        # the layout depends on types and widths alone
-        sig = (tuple((k.dtype, k.shape[1]) for k in keys),
-               tuple(v.dtype for v in cols.values()))
-        if self._laid is None or self._laid[0] != sig:
-            self._laid = (sig, self._layout(dict(zip(self.key_ids, keys)), cols))
-        lay = self._laid[1]
+        lay = self._layout_of(keys, cols)
         if lay is None:
             return None
         acc_bytes, source, out_bytes, dest, results = lay
