@@ -140,7 +140,12 @@ class KeyedPass1:
         keys = [_as_2d(columns[k]) for k in self.key_ids]
         if self._coeffs is None:
             self._coeffs = make_key_coeffs(keys, keys[0].device)
-        out = self._one_read(columns, keys, B)
+        try:
+            out = self._one_read(columns, keys, B)
+        except torch.OutOfMemoryError:
+            # no room for its table (3 GB for 16M groups of eight accumulators):
+            # the general route works a column at a time
+            out = None
         if out is not None:
             return out
         out = self._hash_and_sort(columns, keys)
@@ -291,6 +296,7 @@ class KeyedPass1:
                 if expect or -g > 2 * n // 3 or -g > _MAX_EXPECT:
                     return None
                 expect = -g
+                ws = res = outs = h = bucket = counts = None   # before the larger ones
         buckets = (bucket[:g], list(host_counts), counts) if B > 1 and g > 0 else None
         return [h[:g]] + [t[:g] for t in res], buckets
 
