@@ -435,6 +435,9 @@ int pf_hash_buckets(const int64_t* hash, int64_t n, int B, int32_t* bucket_out,
  *   PF_KA_SUM_I  the int64 sum of an integer column (wraps)
  *   PF_KA_SUM_F  the float64 sum of a float column, in no fixed order
  *   PF_KA_MIN, PF_KA_MAX  of an integer column
+ *   PF_KA_SUM_ERR  what the adds of accumulator `word`, the PF_KA_SUM_F of a
+ *                float64 column, round away (no column); the sum's outputs
+ *                have it added
  * Outputs (nouts <= 40), with room for pf_keyed_pass1_groups(n, naccs, expect)
  * rows
  * as hash_out and bucket_out, from accumulators acc, acc2 and acc3:
@@ -457,6 +460,7 @@ int pf_hash_buckets(const int64_t* hash, int64_t n, int B, int32_t* bucket_out,
 #define PF_KA_SUM_F 4
 #define PF_KA_MIN 5
 #define PF_KA_MAX 6
+#define PF_KA_SUM_ERR 7
 #define PF_KK_I64 0
 #define PF_KK_I32 1
 #define PF_KK_F64 2

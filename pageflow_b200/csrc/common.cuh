@@ -52,6 +52,16 @@ __device__ __forceinline__ void red_add(double* p, double v) {
                : "memory");
 }
 
+// With the old value.
+__device__ __forceinline__ double fetch_add(double* p, double v) {
+  double old;
+  asm volatile("atom.relaxed.gpu.global.add.f64 %0, [%1], %2;"
+               : "=d"(old)
+               : "l"(__cvta_generic_to_global(p)), "d"(v)
+               : "memory");
+  return old;
+}
+
 __device__ __forceinline__ unsigned lanemask_lt() {
   unsigned r;
   asm("mov.u32 %0, %%lanemask_lt;" : "=r"(r));

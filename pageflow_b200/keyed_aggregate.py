@@ -109,7 +109,7 @@ def _unpack_words(words: torch.Tensor, like: torch.Tensor) -> torch.Tensor:
 
 
 # accumulators, column kinds and outputs of pf_keyed_pass1_read and _emit
-_KA_WORD, _KA_COUNT, _KA_NULLS, _KA_SUM_I, _KA_SUM_F, _KA_MIN, _KA_MAX = range(7)
+(_KA_WORD, _KA_COUNT, _KA_NULLS, _KA_SUM_I, _KA_SUM_F, _KA_MIN, _KA_MAX, _KA_SUM_ERR) = range(8)
 _KK = {torch.int64: 0, torch.int32: 1, torch.float64: 2, torch.float32: 3}
 (_KO_WORD, _KO_I64, _KO_I32, _KO_F64, _KO_F32, _KO_I64_MAX0, _KO_I32_MAX0, _KO_COUNT, _KO_AVG_I,
  _KO_AVG_F) = range(10)
@@ -169,6 +169,12 @@ class KeyedPass1:
                 source.append(None if cid is None else (op == _KA_WORD, cid))
             return at
 
+        def summed(cid, kind, fp):
+            s = acc(_KA_SUM_F if fp else _KA_SUM_I, cid, kind)
+            if cols[cid].dtype == torch.float64:
+                acc(_KA_SUM_ERR, None, kind, 0, s)   # its rounding errors
+            return s
+
         outs, dest, results = [], [], []
 
         def out(*fields):
@@ -193,12 +199,12 @@ class KeyedPass1:
                     out(_KO_COUNT, c, acc(_KA_NULLS, cid, kind), 0, 0, 0)
                 results.append((torch.int64, 1))
             elif op == 'avg':
-                s = acc(_KA_SUM_F if fp else _KA_SUM_I, cid, kind)
+                s = summed(cid, kind, fp)
                 out(_KO_AVG_F if fp else _KO_AVG_I, s, acc(_KA_COUNT), acc(_KA_NULLS, cid, kind),
                     0, 0)
                 results.append((torch.float64, 2))
             elif op == 'sum':
-                s = acc(_KA_SUM_F if fp else _KA_SUM_I, cid, kind)
+                s = summed(cid, kind, fp)
                 out({torch.float64: _KO_F64, torch.float32: _KO_F32}.get(v.dtype, _KO_I64), s, 0,
                     0, 0, 0)
                 results.append((v.dtype if fp else torch.int64, 1))
