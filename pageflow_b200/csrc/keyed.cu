@@ -60,7 +60,11 @@ constexpr int KP_MAX_KEYS = 8;
 constexpr int KP_MAX_ACC = 15;
 constexpr int KP_MAX_OUT = 40;
 constexpr long long KP_EMPTY = LLONG_MIN;  // a group of this hash has the slot after the last
-constexpr int KP_WALK = 16;        // sectors of keys a probe looks at
+// Sectors of keys a probe looks at: in a table two thirds full, the fullest one made, a
+// place that far from home is as good as never needed (16 sectors, three quarters
+// full, gave up tables that fitted: 20,000 rows of as many groups took 670 us, by
+// the general route after all, now 159; 300,000 in one run of two 690, now 211).
+constexpr int KP_WALK = 64;
 constexpr size_t KP_TABLE_BYTES = (size_t)64 << 20;
 constexpr size_t KP_CACHE_BYTES = 36 << 10;
 constexpr int KP_CACHE_WALK = 12;
@@ -342,7 +346,7 @@ __device__ __forceinline__ int own_place(long long* own_key, int slots, long lon
 // After a block's first step its last warp adds the block's rows and claims
 // to the launch's and looks whether the groups will fit: rows drawn alike from
 // U groups claim (1 - exp(-z)) / z of the first P, z = P / U.  Past the share
-// that a U of four fifths of the table would give, the launch stops, and what
+// that a U of two thirds of the table would give, the launch stops, and what
 // it met tells the caller how many groups to expect (4M rows of 2M groups: the
 // attempt took 0.6 ms until the table was full).
 struct FirstStep {
@@ -364,7 +368,7 @@ __device__ __forceinline__ void first_step(const KpArgs& a, FirstStep& f, unsign
   const unsigned long long all = atomicAdd((unsigned long long*)&a.head->seen, mine) + mine;
   const unsigned long long P = all >> 32, C = all & 0xffffffffu;
   if (P < 16384) return;
-  const float z = 1.25f * (float)P / (float)a.cap;
+  const float z = 1.5f * (float)P / (float)a.cap;
   if ((float)C > (float)P * ((1.0f - expf(-z)) / z + 0.005f)) a.head->full = 1;
 }
 
@@ -546,7 +550,7 @@ __global__ void __launch_bounds__(KT, PF_KP_MINB) k_kp_insert(KpArgs a) {
   if (own) {
     kp_rows<true>(a, own_key, own_acc, from, a.n, lo, hi, placed, claims);
   } else {
-    const bool look = a.cap < (unsigned long long)a.n;
+    const bool look = a.cap < (unsigned long long)(a.n + a.n / 2 + 1);
 #pragma unroll 1
     for (int part = look ? 0 : 1; part < 2; ++part) {
       const long long f = part && look ? from + step : from;
@@ -833,17 +837,17 @@ struct KpLayout {
   int W, log_buckets;
 };
 
-// Places for n rows of naccs accumulators: a power of two of at least 4 n / 3, the
+// Places for n rows of naccs accumulators: a power of two of at least 3 n / 2, the
 // table of at most KP_TABLE_BYTES; with an expected number of groups, at
-// least a third more than them.
+// least half more than them.
 unsigned long long kp_places(long long n, int naccs, long long expect) {
   const int W = (std::max(naccs, 1) + 3) / 4 * 4;
   if (expect > 0)
-    return pow2_at_least((uint64_t)std::max<long long>(1024, expect + expect / 3 + 1));
+    return pow2_at_least((uint64_t)std::max<long long>(1024, expect + expect / 2 + 1));
   unsigned long long most = 1024;
   while (most * 2 * (W + 1) * 8 <= KP_TABLE_BYTES) most *= 2;
   return std::min<unsigned long long>(
-      most, std::max<unsigned long long>(1024, pow2_at_least((uint64_t)(n + n / 3 + 1))));
+      most, std::max<unsigned long long>(1024, pow2_at_least((uint64_t)(n + n / 2 + 1))));
 }
 
 // The groups U of n rows of which the first `placed` held `claimed` of them:
