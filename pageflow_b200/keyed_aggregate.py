@@ -115,6 +115,10 @@ _KK = {torch.int64: 0, torch.int32: 1, torch.float64: 2, torch.float32: 3}
  _KO_AVG_F) = range(10)
 _MAX_ACCS, _MAX_OUTS, _MAX_KEYS, _MAX_B = 15, 40, 8, 4096
 _MAX_EXPECT = 1 << 24
+# chunks that go straight to the general route after one whose groups were too many
+# for the one-read route's table: the attempt costs 4M rows of as many groups 210 of
+# 1440 us, which a table's other chunks, mostly alike, need not pay
+_GENERAL_CHUNKS = 7
 
 
 class KeyedPass1:
@@ -132,6 +136,7 @@ class KeyedPass1:
                 raise NotImplementedError(f"KeyedPass1: aggregate {op!r}")
         self._coeffs = None
         self._laid = None   # (column types and widths, _layout's answer for them)
+        self._general = 0   # chunks left that take the general route unasked
 
     def pass1(self, columns: Dict[int, torch.Tensor], B: int = 1):
         """``[hash] + keys + values`` of one chunk (hash ascending, unique),
@@ -140,12 +145,16 @@ class KeyedPass1:
         keys = [_as_2d(columns[k]) for k in self.key_ids]
         if self._coeffs is None:
             self._coeffs = make_key_coeffs(keys, keys[0].device)
-        try:
-            out = self._one_read(columns, keys, B)
-        except torch.OutOfMemoryError:
-            # no room for its table (3 GB for 16M groups of eight accumulators):
-            # the general route works a column at a time
-            out = None
+        out, general = None, self._general
+        if general > 0:
+            self._general = general - 1
+        else:
+            try:
+                out = self._one_read(columns, keys, B)
+            except torch.OutOfMemoryError:
+                # no room for its table (3 GB for 16M groups of eight accumulators):
+                # the general route works a column at a time
+                pass
         if out is not None:
             return out
         out = self._hash_and_sort(columns, keys)
@@ -300,6 +309,10 @@ class KeyedPass1:
                 # one for them, unless most rows are a group of their own (the
                 # general route is as fast then, at a smaller workspace)
                 if expect or -g > 2 * n // 3 or -g > _MAX_EXPECT:
+                    # (float sums are rounded otherwise there: a chunk's own groups
+                    # decide, not those of another)
+                    if not any(v.dtype.is_floating_point for v in cols.values()):
+                        self._general = _GENERAL_CHUNKS
                     return None
                 expect = -g
                 ws = res = outs = h = bucket = counts = None   # before the larger ones
