@@ -319,7 +319,7 @@ __global__ void __launch_bounds__(PT) k_hist_plain(Params p) {
 // chunks.  k_scan_sum: each group's rows a bucket; k_bases: per bucket, each
 // group's first row (exclusive over the groups) and the bucket's rows;
 // k_scan_write: every chunk's exclusive offset into hist.
-constexpr int SCAN_G = 64;  // a multiple of 16 (k_bases)
+constexpr int SCAN_G = 64;  // two a lane in k_bases
 
 __device__ __forceinline__ void scan_range(int nchunks, int cg, int& c0, int& c1) {
   const int g0 = blockIdx.y * cg, g1 = min(nchunks, g0 + cg);
@@ -390,12 +390,13 @@ struct Rpu {
   long long v[MAXCLS];
 };
 
-// One block of 1024.  The groups' first rows, a thread a bucket with sixteen loads
-// on their way (a load at a time, in a launch of its own, took 10 us; a warp a
-// bucket, whose loads are a row of buckets apart, 40 us more at 512 buckets: 16.8M
-// rows 614 us, now 576; 100K rows 132 and 93); then host[b] = count b;
-// host[B + cls] = the class's padded total; host[B + MAXCLS] = the prologue's kept
-// rows or -1.  Flag 1 when the counts total more than n_valid.
+// One block of 1024.  The groups' first rows: up to 32 buckets a warp a bucket, one
+// round of loads; more of them a thread a bucket, coalesced, with sixteen loads on
+// their way (a load at a time, in a launch of its own, took 10 us).  By a warp and by
+// a thread: 16.8M rows into 8 buckets 217 and 220 us, 32 405 and 408, 64 429 and 429,
+// 128 456 and 449, 512 616 and 578; 100K rows into 512 133 and 98.  Then
+// host[b] = count b; host[B + cls] = the class's padded total; host[B + MAXCLS] =
+// the prologue's kept rows or -1.  Flag 1 when the counts total more than n_valid.
 __global__ void __launch_bounds__(1024) k_bases(long long* gsum, long long* counts, int B,
                                                 Rpu rpu, int ncls, long long* __restrict__ bases,
                                                 long long* host, int* flags, long long n_valid,
@@ -406,7 +407,22 @@ __global__ void __launch_bounds__(1024) k_bases(long long* gsum, long long* coun
   const int per = (B + 1023) / 1024;
   const int st = tid * per;
   const bool bad = flags[0] != 0;
-  for (int b = tid; b < B && !bad; b += 1024) {
+  if (B <= 32 && w < B && !bad) {
+    const long long x0 = gsum[(long long)lane * B + w], x1 = gsum[(long long)(32 + lane) * B + w];
+    long long i0 = x0, i1 = x1;
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long y0 = __shfl_up_sync(FULL, i0, o), y1 = __shfl_up_sync(FULL, i1, o);
+      if (lane >= o) {
+        i0 += y0;
+        i1 += y1;
+      }
+    }
+    i1 += __shfl_sync(FULL, i0, 31);
+    gsum[(long long)lane * B + w] = i0 - x0;
+    gsum[(long long)(32 + lane) * B + w] = i1 - x1;
+    if (lane == 31) counts[w] = i1;
+  }
+  for (int b = tid; B > 32 && b < B && !bad; b += 1024) {
     long long run = 0;
     for (int g0 = 0; g0 < SCAN_G; g0 += 16) {
       long long x[16];
