@@ -304,7 +304,7 @@ __device__ __forceinline__ void probe_rows(const Desc& D, const BatchArgs& a, un
   __builtin_assume(__isGlobal(pval));
   const int vbits = D.vbits;
   const unsigned long long one = 1ULL << D.sbits;
-  const long long bias = 1LL << (vbits - 1);
+  const unsigned long long bias = 1ULL << (vbits - 1);
   unsigned long long next[BV];
 #pragma unroll
   for (int k = 0; k < BV; ++k) {
@@ -362,7 +362,7 @@ __device__ __forceinline__ void probe_rows(const Desc& D, const BatchArgs& a, un
       matched += g[k] >= -1;
       if (g[k] < 0 || own.add((unsigned)g[k], value[k], i0 == lo)) continue;
       if (PACK) {
-        const unsigned long long v = (unsigned long long)(value[k] + bias);
+        const unsigned long long v = (unsigned long long)value[k] + bias;
         outside |= v >> vbits != 0;
         high += v >> 20;
         ++rows;
