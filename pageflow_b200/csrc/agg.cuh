@@ -13,6 +13,24 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
   return v;
 }
 
+// Where a warp has a group in four lanes or more: the words x of the lanes of the same
+// group (every lane of the warp; g < 0: none) added up into the group's first lane; how
+// many they are, 0 in the others.  Else each lane's own.
+__device__ __forceinline__ unsigned warp_group_sum(int g, unsigned long long& x) {
+  const int lane = threadIdx.x & 31;
+  const unsigned all = __match_any_sync(FULL, g);
+  if (!__any_sync(FULL, g >= 0 && __popc(all) >= 4)) return g >= 0;
+  unsigned rank = __popc(all & lanemask_lt()), above = g < 0 ? 0u : all & ~1u << lane;
+  const unsigned n = g < 0 || rank ? 0u : (unsigned)__popc(all);
+  while (__any_sync(FULL, above)) {
+    const unsigned long long y = __shfl_sync(FULL, x, above ? __ffs(above) - 1 : lane);
+    if (above) x += y;
+    above &= __ballot_sync(FULL, (rank & 1) == 0);  // every other one has been taken
+    rank >>= 1;
+  }
+  return n;
+}
+
 // The block's own sums: lo, hi and count of OWN_CELLS cells.  A source of few
 // groups has all of them there, as many copies of each as fit, a lane its own
 // (a warp's lanes then meet on no address).  Else, where the source's first
