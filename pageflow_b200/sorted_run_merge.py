@@ -85,17 +85,17 @@ def reduce_tick_slice(keys: torch.Tensor, vals: Sequence[torch.Tensor],
 
 
 def _copy_rows(dst: Sequence[torch.Tensor], src: Sequence[torch.Tensor], n: int) -> None:
-    """``d[:n] = s[:n]`` for every pair, the plain ones in one launch."""
+    """``d[:n] = s`` for every pair, the plain ones (of n rows each) in one launch."""
     plain = []
     for d, s in zip(dst, src):
         if (d.is_cuda and s.is_cuda and d.device == s.device and d.dtype == s.dtype
-                and d.shape[1:] == s.shape[1:] and d.shape[0] >= n and s.shape[0] >= n
+                and s.shape == (n,) + d.shape[1:] and d.shape[0] >= n
                 and d.is_contiguous() and s.is_contiguous() and d[:1].numel() > 0
                 and not d.requires_grad and not s.requires_grad
                 and d.untyped_storage().data_ptr() != s.untyped_storage().data_ptr()):
             plain.append((d, s))
         else:
-            d[:n] = s[:n]
+            d[:n] = s
     for i in range(0, len(plain), 16):
         part = plain[i:i + 16]
         rb = [d.element_size() * (d.numel() // d.shape[0]) for d, _ in part]
@@ -156,7 +156,7 @@ def merge_sorted_unique_runs_inplace(key_buf: torch.Tensor, val_bufs: Sequence[t
     assert M <= key_buf.shape[0], (
         f"merge capacity exhausted: M={M} > buf={key_buf.shape[0]} — the buffers must be "
         f"sized to the pass2 total input rows")
-    _copy_rows([key_buf] + list(val_bufs), [out_k] + outs, M)
+    _copy_rows([key_buf] + list(val_bufs), [t[:M] for t in [out_k] + outs], M)
     return M
 
 
