@@ -539,8 +539,9 @@ int pf_merge_sorted_runs(const int64_t* run_keys, const void* const* run_vals, i
  * The merge in place where it moves nothing: *n_new (host) gets the tick keys
  * that the run does not hold, and when there is none every tick row is
  * combined into its run row, op(run value, tick value), and the run is the
- * merged one.  Else nothing is written (take pf_merge_sorted_runs).  The
- * workspace is pf_merge_sorted_runs_workspace's; waits once.
+ * merged one.  Else nothing is written (take pf_merge_sorted_runs), nor where a
+ * run column shares memory with another column or with keys (*n_new is -1).
+ * The workspace is pf_merge_sorted_runs_workspace's; waits once.
  */
 int pf_fold_sorted_run(const int64_t* run_keys, void* const* run_vals, int64_t n_run,
                        const int64_t* tick_keys, const void* const* tick_vals, int64_t n_tick,

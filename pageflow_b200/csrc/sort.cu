@@ -813,6 +813,29 @@ extern "C" int pf_merge_sorted_runs(const int64_t* run_keys, const void* const* 
   return ok();
 }
 
+namespace {
+// Whether a run column to be combined in place shares memory with another column or
+// the keys: a row's values could then change before they are read.
+bool columns_overlap(const VCols& c, const void* run_keys, int64_t n_run, const void* tick_keys,
+                     int64_t n_tick) {
+  struct Span {
+    const char* at;
+    int64_t bytes;
+  };
+  Span s[2 * MAXV + 2];
+  int n = 0;
+  auto add = [&](const void* p, int64_t bytes) { s[n++] = Span{(const char*)p, bytes}; };
+  for (int q = 0; q < c.n; ++q) add(c.out[q], n_run * c.esize[q] * c.width[q]);
+  for (int q = 0; q < c.n; ++q) add(c.b[q], n_tick * c.esize[q] * c.width[q]);
+  add(run_keys, 8 * n_run);
+  add(tick_keys, 8 * n_tick);
+  for (int w = 0; w < c.n; ++w)
+    for (int k = w + 1; k < n; ++k)
+      if (s[w].at < s[k].at + s[k].bytes && s[k].at < s[w].at + s[w].bytes) return true;
+  return false;
+}
+}  // namespace
+
 extern "C" int pf_fold_sorted_run(const int64_t* run_keys, void* const* run_vals, int64_t n_run,
                                   const int64_t* tick_keys, const void* const* tick_vals,
                                   int64_t n_tick, int ncols, const int* kinds, const int* esizes,
@@ -843,6 +866,10 @@ extern "C" int pf_fold_sorted_run(const int64_t* run_keys, void* const* run_vals
   if (!workspace || !a.fits())
     return fail(PF_ENOSPACE, "fold_sorted_run: workspace of %zu bytes, %zu needed",
                 workspace_bytes, a.used);
+  if (columns_overlap(c, run_keys, n_run, tick_keys, n_tick)) {
+    *n_new = -1;
+    return ok();
+  }
   PF_CUDA(cudaMemsetAsync(l.total, 0, sizeof(long long), st));
   {
     PF_KERNEL("k_merge_tick", st);

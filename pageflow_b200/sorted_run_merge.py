@@ -84,18 +84,20 @@ def reduce_tick_slice(keys: torch.Tensor, vals: Sequence[torch.Tensor],
     return out_k[:u], [o[:u] for o in outs]
 
 
-def _copy_rows(dst: Sequence[torch.Tensor], src: Sequence[torch.Tensor], n: int) -> None:
-    """``d[:n] = s`` for every pair, the plain ones (of n rows each) in one launch."""
+def _copy_rows(dst: Sequence[torch.Tensor], src: Sequence[torch.Tensor], n: int,
+               room: int) -> None:
+    """``d[:n] = s`` for every pair, s of n rows, the first of ``room``; the plain ones in
+    one launch."""
     plain = []
     for d, s in zip(dst, src):
         if (d.is_cuda and s.is_cuda and d.device == s.device and d.dtype == s.dtype
-                and s.shape == (n,) + d.shape[1:] and d.shape[0] >= n
+                and s.shape == (room,) + d.shape[1:] and d.shape[0] >= n
                 and d.is_contiguous() and s.is_contiguous() and d[:1].numel() > 0
                 and not d.requires_grad and not s.requires_grad
                 and d.untyped_storage().data_ptr() != s.untyped_storage().data_ptr()):
             plain.append((d, s))
         else:
-            d[:n] = s
+            d[:n] = s if room == n else s[:n]
     for i in range(0, len(plain), 16):
         part = plain[i:i + 16]
         rb = [d.element_size() * (d.numel() // d.shape[0]) for d, _ in part]
@@ -117,7 +119,7 @@ def merge_sorted_unique_runs_inplace(key_buf: torch.Tensor, val_bufs: Sequence[t
     if T == 0:
         return run_len
     if run_len == 0:
-        _copy_rows([key_buf] + list(val_bufs), [tick_keys] + list(tick_vals), T)
+        _copy_rows([key_buf] + list(val_bufs), [tick_keys] + list(tick_vals), T, T)
         return T
     R = run_len
     dev = key_buf.device
@@ -156,7 +158,7 @@ def merge_sorted_unique_runs_inplace(key_buf: torch.Tensor, val_bufs: Sequence[t
     assert M <= key_buf.shape[0], (
         f"merge capacity exhausted: M={M} > buf={key_buf.shape[0]} — the buffers must be "
         f"sized to the pass2 total input rows")
-    _copy_rows([key_buf] + list(val_bufs), [t[:M] for t in [out_k] + outs], M)
+    _copy_rows([key_buf] + list(val_bufs), [out_k] + outs, M, cap)
     return M
 
 
