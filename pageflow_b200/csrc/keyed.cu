@@ -610,13 +610,12 @@ __global__ void __launch_bounds__(KT, PF_KP_MINB) k_kp_insert(KpArgs a) {
   }
 }
 
-// The bucket of a hash: the top log2(buckets) bits of its place in the
-// hashes' range, the range taken up to a power of two.
+// The bucket of a hash: the top log2(buckets) bits (three at least) of its place in
+// the hashes' range, the range taken up to a power of two.
 __device__ __forceinline__ unsigned kp_bucket(long long h, long long lo, long long hi,
                                               int log_buckets) {
   const unsigned long long r = (unsigned long long)hi - (unsigned long long)lo;
   const int up = r ? __clzll((long long)r) : 63;
-  if (!log_buckets) return 0;
   return (unsigned)((((unsigned long long)h - (unsigned long long)lo) << up) >>
                     (64 - log_buckets));
 }
