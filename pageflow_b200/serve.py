@@ -347,7 +347,17 @@ class Server:
     def run(self, requests: list[Request], keep_results: bool = True,
             timeout_s: float = 600.0) -> ServeRun:
         """Serves the requests at their arrival times (seconds after the
-        call starts); returns when every request is complete."""
+        call starts); returns when every request is complete.  A call that
+        raises does so when its launches have ended: they write results into
+        the pinned pool, which its owner may then give up."""
+        try:
+            return self._run(requests, keep_results, timeout_s)
+        except BaseException:
+            self.stream.synchronize()
+            self.copy_stream.synchronize()
+            raise
+
+    def _run(self, requests, keep_results, timeout_s) -> ServeRun:
         L = lib()
         spec_keys = self.dims.spec.dim_keys
         spec_groups = self.dims.spec.dim_groups
