@@ -250,6 +250,7 @@ __global__ void __launch_bounds__(DT, PF_DJ_MINB) k_dj_probe(DjArgs a) {
   }
   __syncthreads();
   if (MODE == SUM_SMALL) {
+    unsigned long long* rep = a.slab + 2ULL * (blockIdx.x % DJ_REPS) * (unsigned long long)a.G;
     for (int g = tid; g < (int)a.G; g += DT) {
       unsigned long long s = 0, c = 0;
       for (int j = 0; j < 1 << a.copies; ++j) {
@@ -258,8 +259,8 @@ __global__ void __launch_bounds__(DT, PF_DJ_MINB) k_dj_probe(DjArgs a) {
         c += cnt[x];
       }
       if (c) {
-        atomicAdd(&pairs[2 * g], s);
-        atomicAdd(&pairs[2 * g + 1], c);
+        atomicAdd(&rep[2 * g], s);
+        atomicAdd(&rep[2 * g + 1], c);
       }
     }
   } else {

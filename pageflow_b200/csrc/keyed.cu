@@ -375,7 +375,7 @@ __device__ __forceinline__ void first_step(const KpArgs& a, FirstStep& f, unsign
 // The block's rows folded in, KR a thread a step.  OWN: through the block's
 // own table, by a warp while one row in eight finds its group there (looked
 // at every eight steps).
-template <bool OWN>
+template <bool OWN, bool ERRS>
 __device__ __forceinline__ void kp_rows(const KpArgs& a, long long* own_key, long long* own_acc,
                                         long long from, long long to, long long& lo,
                                         long long& hi, unsigned& placed, unsigned& claims) {
@@ -474,7 +474,7 @@ __device__ __forceinline__ void kp_rows(const KpArgs& a, long long* own_key, lon
         }
       }
     }
-    for (int k = ncmp; k < a.acc.nplain; ++k) {
+    for (int k = ncmp; k < (ERRS ? a.acc.nplain : na); ++k) {
       long long v[KR];
       acc_values(a.acc, k, i0, at, v);
       const int is_float = a.acc.is_float[k];
@@ -485,7 +485,7 @@ __device__ __forceinline__ void kp_rows(const KpArgs& a, long long* own_key, lon
         else add_to(a.accs + (long long)at[r] * W + k, is_float, v[r]);
       }
     }
-    for (int k = a.acc.nplain; k < a.acc.nplain + a.acc.nerr; ++k) {
+    for (int k = a.acc.nplain; ERRS && k < a.acc.nplain + a.acc.nerr; ++k) {
       const double* src = reinterpret_cast<const double*>(a.acc.src[k]);
       double v[KR];
 #pragma unroll
@@ -505,6 +505,8 @@ __device__ __forceinline__ void kp_rows(const KpArgs& a, long long* own_key, lon
   }
 }
 
+// ERRS: there are float64 sums whose errors are kept (3% of the others' time).
+template <bool ERRS>
 __global__ void __launch_bounds__(KT, PF_KP_MINB) k_kp_insert(KpArgs a) {
   extern __shared__ __align__(16) long long own_smem[];
   __shared__ long long red[2][KT / 32];
@@ -548,13 +550,13 @@ __global__ void __launch_bounds__(KT, PF_KP_MINB) k_kp_insert(KpArgs a) {
   unsigned placed = 0, claims = 0;  // a thread's, below 2^32 (at most 2^40 rows)
   const long long from = (long long)blockIdx.x * tile, step = (long long)gridDim.x * tile;
   if (own) {
-    kp_rows<true>(a, own_key, own_acc, from, a.n, lo, hi, placed, claims);
+    kp_rows<true, ERRS>(a, own_key, own_acc, from, a.n, lo, hi, placed, claims);
   } else {
     const bool look = a.cap < (unsigned long long)(a.n + a.n / 2 + 1);
 #pragma unroll 1
     for (int part = look ? 0 : 1; part < 2; ++part) {
       const long long f = part && look ? from + step : from;
-      kp_rows<false>(a, own_key, own_acc, f, part ? a.n : min(a.n, from + step), lo, hi, placed,
+      kp_rows<false, ERRS>(a, own_key, own_acc, f, part ? a.n : min(a.n, from + step), lo, hi, placed,
                      claims);
       if (part == 0) {
         first_step(a, first, placed, claims);
@@ -573,11 +575,11 @@ __global__ void __launch_bounds__(KT, PF_KP_MINB) k_kp_insert(KpArgs a) {
       continue;
     }
     long long* p = a.accs + (long long)g * W;
-    const int nplain = a.acc.nplain, nerr = a.acc.nerr;
+    const int nplain = ERRS ? a.acc.nplain : na, nerr = ERRS ? a.acc.nerr : 0;
     for (int k = 0; k < nplain + nerr; ++k) {
       const long long v = own_acc[s * na + k];
       if (k < ncmp) red_max(p + k, v);
-      else if (k < nplain) add_to(p + k, a.acc.is_float[k], v);
+      else if (!ERRS || k < nplain) add_to(p + k, a.acc.is_float[k], v);
       else add_with_error(p + k, nerr, __longlong_as_double(v),
                           __longlong_as_double(own_acc[s * na + k + nerr]));
     }
@@ -1075,10 +1077,11 @@ extern "C" int pf_keyed_pass1_read(const void* const* key_cols, const int* row_b
     k_kp_init<<<(unsigned)(sm_count() * 2 * 3), KT, 0, st>>>(x, l.hist, nbuckets);
   }
   PF_LAUNCH("k_kp_init");
-  if (int rc = opt_in_smem((const void*)k_kp_insert, smem)) return rc;
+  auto insert = x.acc.nerr ? k_kp_insert<true> : k_kp_insert<false>;
+  if (int rc = opt_in_smem((const void*)insert, smem)) return rc;
   {
     PF_KERNEL("k_kp_insert", st);
-    k_kp_insert<<<kp_grid(n, KT * KR, PF_KP_MINB), KT, smem, st>>>(x);
+    insert<<<kp_grid(n, KT * KR, PF_KP_MINB), KT, smem, st>>>(x);
   }
   PF_LAUNCH("k_kp_insert");
   {
