@@ -27,7 +27,7 @@
 // What bounds it: L2's rate of requests.  A probe row costs one table sector and
 // one RED, where 16-byte slots half full took two or three dependent reads and a
 // group's (sum, count) pair two REDs: 48 instances (29M build, 290M probe rows,
-// FKs of Zipf 0, 0.8 and 1.2) 8.7 -> 5.4 ms, 8 of up to 50K rows 285 -> 90 us.
+// FKs of Zipf 0, 0.8 and 1.2) 8.7 -> 5.2 ms, 8 of up to 50K rows 285 -> 90 us.
 // One instance of 2M x 20M rows and 20 groups 548 -> 260 us.  Its value and 1 go into the
 // group's packed word, or, for the groups a block meets often (skewed keys),
 // through a cache in shared memory flushed into the slab at the item's end.

@@ -36,7 +36,8 @@
 // group of their own.  4M rows, two key columns, five aggregates, the pass
 // through KeyedPass1 against the general route: 4 groups 0.30 against 1.38 ms,
 // 1000 0.37 against 0.94, 100K 0.34 against 1.05, 900K (a second table) 0.63
-// against 1.10, 4M 1.43 both.  k_kp_insert takes 0.18 ms of it at 250K groups.
+// against 1.10; 4M, by the general route after a failed attempt, 1.43 against
+// 1.23.  k_kp_insert takes 0.18 ms of it at 250K groups.
 #include <algorithm>
 #include <climits>
 #include <cmath>
@@ -248,7 +249,8 @@ __device__ __forceinline__ void add_to_shared(long long* p, int is_float, long l
 
 // A float64 sum's rows with their errors (every lane of the warp; at < 0: none): the
 // lanes of a group add theirs up as a tree, so that a group of many lanes does
-// not queue up on the loop of its add (the pass over 4M rows of 4 groups: 272 us; a lane each 423).
+// not queue up on the loop of its add (the pass over 4M rows of 4 groups: 272 us; a
+// lane each 423).
 __device__ __forceinline__ void add_group_to_shared(long long* own, int na, int k, int nerr,
                                                     int at, double x) {
   const int lane = threadIdx.x & 31;

@@ -18,7 +18,10 @@ A chunk whose rows share groups (two a group or more) takes hash and groups
 in one read of its rows (pf_keyed_pass1_read, _emit: a place of a hash table
 holds every accumulator of its group); one of mostly single rows, or of
 columns that the table does not hold (floats' min and max, two-dimensional or
-narrow values), the steps above.
+narrow values), the steps above.  After a chunk of integer columns whose groups
+were too many for the table, the object's next seven take the steps without the
+attempt.  A float64 SUM is exact to its own rounding in the one read, and added
+as a segmented tree by the steps.
 
 Aggregates: ``('sum', col)``, ``('count', None)`` (every row) or
 ``('count', col)`` (the rows whose value is not the null -64), ``('min',
